@@ -816,13 +816,16 @@ static int pair_setup(fedg_ctx* c, MixedState* m) {
   OpsP& x = m->opp;
   std::memset(&x, 0, sizeof(x));
   for (int k = 0; k < FEDG_MAXN1 * FEDG_MAXN1; ++k) {
-    x.D[k] = split_host(o.D[k]); x.T[k] = split_host(o.T[k]);
+    x.Dx[k] = split_host(o.E11 * o.D[k]); x.Dy[k] = split_host(o.E22 * o.D[k]); x.Dz[k] = split_host(o.E33 * o.D[k]);
+    x.Tg[k] = split_host(o.grav * o.T[k]);
     x.F[k] = split_host(o.F[k]); x.Fv[k] = split_host(o.Fv[k]);
   }
-  for (int k = 0; k < FEDG_MAXN1; ++k) { x.Lb[k] = split_host(o.Lb[k]); x.Lt[k] = split_host(o.Lt[k]); }
-  x.E11 = split_host(o.E11); x.E22 = split_host(o.E22); x.E33 = split_host(o.E33);
-  x.FSx = split_host(o.FSx); x.FSy = split_host(o.FSy); x.FSz = split_host(o.FSz);
-  x.grav = split_host(o.grav); x.kap = split_host(o.kap); x.cor = split_host(o.coriolis_f);
+  for (int k = 0; k < FEDG_MAXN1; ++k) {
+    x.Lxb[k] = split_host(0.5 * o.FSx * o.Lb[k]); x.Lxt[k] = split_host(0.5 * o.FSx * o.Lt[k]);
+    x.Lyb[k] = split_host(0.5 * o.FSy * o.Lb[k]); x.Lyt[k] = split_host(0.5 * o.FSy * o.Lt[k]);
+    x.Lzb[k] = split_host(0.5 * o.FSz * o.Lb[k]); x.Lzt[k] = split_host(0.5 * o.FSz * o.Lt[k]);
+  }
+  x.kap = split_host(o.kap); x.cor = split_host(o.coriolis_f);
   x.kap64 = o.kap;
   x.rmax = m->opx.rmax;
   for (int n = 0; n < 12; ++n) x.cb[n] = m->opx.cb[n];
@@ -993,7 +996,7 @@ static int pair_update_heve(fedg_ctx* c, double* const q[5], int nsteps, const f
       if (slab(c) && (r = halo_exchange_pair(c, BP.qs, s))) return r;
       for (int v = 0; v < 5; ++v) BP.qh[v] = (hout && s == 3 && step == nsteps - 1) ? hout[v] : nullptr;
       r = tracked(c, FEDG_K_MTEND, [&] {
-        return launch_stage_pair_heve(c->N1, s, m->opp, pfp, c->d_prof, BP, pc, c->Ne, filt, c->stream);
+        return launch_stage_pair_heve(c->N1, s, m->opp, pfp, BP, pc, c->Ne, filt, c->stream);
       });
       if (r) return api_cuda_fail((cudaError_t)r, "fedg_update(pair, HEVE): stage");
       if (tf[0]) {  // save_massflux of the stage state (driver_nonhydro3d.F90:900-917)
@@ -1103,8 +1106,12 @@ int mixed_update(fedg_ctx* c, double* const q[5], int nsteps, const fedg_update_
   const double impl_fac = gam * o->dt;
   MixViArgs va{impl_fac, 1.0 / impl_fac, o->tol, 340.0, split_host(impl_fac), split_host(1.0 / impl_fac), o->max_iter, 1,
                c->vi_neumann};
-  const PairCoef pc{split_host(o->dt), split_host(2.0 * gam), split_host(gam), split_host(1.0 - alp), split_host(del),
-                    split_host(alp), split_host(del), split_host(del), split_host(del), split_host(gam)};
+  PairCoef pc;
+  std::memset(&pc, 0, sizeof(pc));
+  pc.q1e = split_host(o->dt * (2.0 * gam)); pc.q1i = split_host(o->dt * gam);
+  pc.s3e = split_host(o->dt * (1.0 - alp)); pc.s3i = split_host(o->dt * del);
+  pc.q2e = split_host(o->dt * alp); pc.q2i = split_host(o->dt * del);
+  pc.sf1 = pc.sf2 = split_host(o->dt * del); pc.sf3 = split_host(o->dt * gam);
   ProfP pfp{m->prof5, m->prof5 + c->L, m->prof5 + 2 * c->L, m->prof5 + 3 * c->L, m->prof5 + 4 * c->L,
             m->prof + c->L};
   if ((r = set_sponge_prof(c, m, &pff, &pfp))) return r;
@@ -1145,7 +1152,7 @@ int mixed_update(fedg_ctx* c, double* const q[5], int nsteps, const fedg_update_
   const int filt = c->d.mf_on;
   auto stage = [&](int s) -> int {
     return tracked(c, FEDG_K_MTEND, [&] {
-      if (pair) return launch_stage_pair(c->N1, s, m->opp, pfp, c->d_prof, BP, pc, c->Ne, filt, c->stream);
+      if (pair) return launch_stage_pair(c->N1, s, m->opp, pfp, BP, pc, c->Ne, filt, c->stream);
       switch (c->N1) {
         case 4: return launch_stage_m<4>(s, m->opf, pff, c->d_prof, B, cf, c->Ne, filt, c->stream);
         case 8: return launch_stage_m<8>(s, m->opf, pff, c->d_prof, B, cf, c->Ne, filt, c->stream);
@@ -1203,7 +1210,7 @@ int mixed_update(fedg_ctx* c, double* const q[5], int nsteps, const fedg_update_
     if (step == 0 && hin) {
       if ((r = pipelined_first_stage(c, m, q, hin, [&](int ke0, int ke1) {
              return tracked(c, FEDG_K_MTEND, [&] {
-               return launch_stage_pair(c->N1, 1, m->opp, pfp, c->d_prof, BP, pc, ke1, filt, c->stream, ke0);
+               return launch_stage_pair(c->N1, 1, m->opp, pfp, BP, pc, ke1, filt, c->stream, ke0);
              });
            })))
         return r;

@@ -73,10 +73,11 @@ struct MixViArgs {
 
 // ---- float-pair precision mode (FEDG_PREC_PAIR, fedg_pair.cu) ----
 struct OpsP {
-  float2 D[FEDG_MAXN1 * FEDG_MAXN1], T[FEDG_MAXN1 * FEDG_MAXN1];
-  float2 F[FEDG_MAXN1 * FEDG_MAXN1], Fv[FEDG_MAXN1 * FEDG_MAXN1];
-  float2 Lb[FEDG_MAXN1], Lt[FEDG_MAXN1];
-  float2 E11, E22, E33, FSx, FSy, FSz, grav, kap, cor, Uref, Vref;
+  // metric factors multiplied in: Dx = E11 D and so on, Tg = grav T, Lxb = FSx/2 Lb and so on
+  float2 Dx[FEDG_MAXN1 * FEDG_MAXN1], Dy[FEDG_MAXN1 * FEDG_MAXN1], Dz[FEDG_MAXN1 * FEDG_MAXN1];
+  float2 Tg[FEDG_MAXN1 * FEDG_MAXN1], F[FEDG_MAXN1 * FEDG_MAXN1], Fv[FEDG_MAXN1 * FEDG_MAXN1];
+  float2 Lxb[FEDG_MAXN1], Lxt[FEDG_MAXN1], Lyb[FEDG_MAXN1], Lyt[FEDG_MAXN1], Lzb[FEDG_MAXN1], Lzt[FEDG_MAXN1];
+  float2 kap, cor, Uref, Vref;
   float cb[12];
   float rmax;
   double kap64;
@@ -92,9 +93,12 @@ struct ProfP {
   const float2* sl = nullptr;               // sponge-layer coefficient per level (NULL: no sponge)
   float sl_h = 0.f;                         // 1: the sponge also damps MOMX/MOMY
 };
+// Stage coefficients.  HEVI (IMEX ARK232), the time step multiplied in: q*_2 = q^n + q1e t_ex + q1i t_im,
+// S3 = s3e t_ex + s3i t_im, SF = sf1 (t_ex + t_im); q*_3 = q^n + S3 + q2e t_ex + q2i t_im, SF += sf2 (...);
+// q^{n+1} = q^n + SF + sf3 (...).  HEVE: dt and ERK_SSP_3s3o's 3/4, 1/4, 1/3, 2/3.
 struct PairCoef {
-  float2 dt, a21e, a21i, a31e, a31i, a32e, a32i, b1, b2, b3;
-  float2 ssp[4];  // ERK_SSP_3s3o: 3/4, 1/4, 1/3, 2/3 (HEVE)
+  float2 q1e, q1i, s3e, s3i, sf1, q2e, q2i, sf2, sf3;
+  float2 dt, ssp[4];
 };
 struct StagePairBufs {
   const float2* qs[5];  // deviation state of the explicit tendency (q^n at stage 1, Q_s after)
@@ -111,11 +115,11 @@ struct StagePairBufs {
   float2* a0[3];        // stage 1 (HEVI): A(q^n) of DENS, MOMZ, RHOT for the column solves' first residual
   double* qh[5];        // stage 3: also store q^{n+1} here (mapped page-locked host memory; NULL: none)
 };
-int launch_stage_pair_heve(int N1, int stage, const OpsP& op, const ProfP& pf, const double* dens64,
-                           const StagePairBufs& B, const PairCoef& cf, int Ne, int filt, cudaStream_t s);
+int launch_stage_pair_heve(int N1, int stage, const OpsP& op, const ProfP& pf, const StagePairBufs& B,
+                           const PairCoef& cf, int Ne, int filt, cudaStream_t s);
 // elements [ke0, Ne) (ke0 > 0: one z-range of the mesh, for the pipelined first stage)
-int launch_stage_pair(int N1, int stage, const OpsP& op, const ProfP& pf, const double* dens64,
-                      const StagePairBufs& B, const PairCoef& cf, int Ne, int filt, cudaStream_t s, int ke0 = 0);
+int launch_stage_pair(int N1, int stage, const OpsP& op, const ProfP& pf, const StagePairBufs& B,
+                      const PairCoef& cf, int Ne, int filt, cudaStream_t s, int ke0 = 0);
 
 // Mixed-precision column solve (fedg_vicol.cu).  qin: stage input q* (float pairs); z: var0
 // (FP64; alph and the plain initial iterate); guess: FP32 increments of (DENS, MOMZ, RHOT) over

@@ -15,6 +15,22 @@
 // flows (a -15 K density current at p = 7) that drifts from FP64 by ~4e-8 of the state per step.
 // Pairs bring the same amplification down to ~1e-14.
 //
+// Layout: one thread owns the two nodes (i, j, k) and (i, j, k + N1/2) of an element and carries both
+// in the packed pair arithmetic of fedg_p2.cuh, so an element takes Np/2 threads and two blocks of
+// 256 threads share an SM at p = 7.  Shared memory holds each field as 16-byte entries (hi of both
+// nodes, lo of both nodes).  The x and y contractions read one entry per term; along z an entry holds
+// two terms of the same line.  All three directions and the Lift accumulate into one compensated sum
+// per variable, with the metric factors multiplied into the operator tables on the host.  A face node
+// takes its own side's normal flux from the volume fluxes and computes the neighbour's side only in
+// the face's direction (one warp per face at p = 7).
+//
+// What bounds it: the FP32 pipe (62 % of its cycles at p = 7, 24x24x12 elements; issue slots 49 %), then
+// the barriers between the volume fluxes, the faces and the Lift.  With one node per thread, scalar
+// pairs and one 512-thread block per SM the same pipe was 44 % busy.  HEVE step (three launches) at
+// p = 7, 45x37x13 elements: 7.25 -> 4.95 ms.  The derivative loops stay rolled (unrolled, the code
+// misses the instruction caches: 5.5 ms), and an L2 prefetch of the following block's fields, which the
+// one-block form needed, costs 2-3 % here: the SM's second block already covers a block's first loads.
+//
 // FElib counterparts: cal_tend for HEVI (FElib/src/atmosphere/dynamics/
 // scale_atm_dyn_dgm_nonhydro3d_rhot_hevi.F90:289-482), the HEVI numerical flux
 // (scale_atm_dyn_dgm_nonhydro3d_rhot_hevi_numflux.F90:232-418), the implicit operator at var0
@@ -25,503 +41,611 @@
 // The sponge layer (…_dgm_spongelayer.F90:134-219) is added to the explicit tendency when a
 // profile is given.
 #include "fedg_ctx.cuh"
-#include "fedg_f2.cuh"
 #include "fedg_mixed.cuh"
+#include "fedg_p2.cuh"
 
 namespace fedg {
 namespace {
 
-__device__ __forceinline__ f2 operator+(f2 a, f2 b) { return f2_add(a, b); }
-__device__ __forceinline__ f2 operator-(f2 a, f2 b) { return f2_sub(a, b); }
-__device__ __forceinline__ f2 operator*(f2 a, f2 b) { return f2_mul(a, b); }
-__device__ __forceinline__ f2 operator*(f2 a, float b) { return f2_mul_f(a, b); }
-__device__ __forceinline__ f2 operator-(f2 a) { return f2_neg(a); }
-__device__ __forceinline__ f2 ld2(const float2* p) { return f2_of(__ldg(p)); }
-constexpr f2 Z2{0.f, 0.f};
+__device__ __forceinline__ p2 ld2(const float2* p, size_t a, size_t b) { return p2_of(__ldg(p + a), __ldg(p + b)); }
+__device__ __forceinline__ void st2(float2* p, size_t a, size_t b, p2 v) {
+  const float2 h = unpk(v.h), l = unpk(v.l);
+  p[a] = make_float2(h.x, l.x);
+  p[b] = make_float2(h.y, l.y);
+}
+__device__ __forceinline__ double to64(f2 v) { return (double)v.h + (double)v.l; }
 
 // pressure deviation PRES_hyd ((1 + DRHOT/THERM_hyd)^kappa - 1): leading term in pairs, the rest
 // of the binomial series in FP32 (relative size |r|), pow() in FP64 beyond rmax
-__device__ __forceinline__ f2 dpres2(const OpsP& o, f2 dr, f2 rth, f2 ph) {
-  const f2 r = dr * rth;
-  f2 S;
-  if (fabsf(r.h) <= o.rmax) {
-    float tl = o.cb[11];
+__device__ __noinline__ f2 dpres_pow(float rh, float rl, double kap64) {
+  return f2_split(pow(1.0 + ((double)rh + (double)rl), kap64) - 1.0);
+}
+__device__ __forceinline__ p2 dpres2(const OpsP& o, p2 dr, p2 rth, p2 ph) {
+  const p2 r = dr * rth;
+  u64x tl = pk1(o.cb[11]);
 #pragma unroll
-    for (int m = 10; m >= 1; --m) tl = fmaf(tl, r.h, o.cb[m]);
-    S = f2_add_f(f2_of(o.kap) * r, __fmul_rn(__fmul_rn(r.h, r.h), tl));
-  } else {
-    S = f2_split(pow(1.0 + ((double)r.h + (double)r.l), o.kap64) - 1.0);
+  for (int m = 10; m >= 1; --m) tl = xfma(tl, r.h, pk1(o.cb[m]));
+  p2 S = p2_add_x(p2_dup(o.kap) * r, xmul(xmul(r.h, r.h), tl));
+  const float2 rh = unpk(r.h);
+  if (!(fabsf(rh.x) <= o.rmax && fabsf(rh.y) <= o.rmax)) {
+    const float2 rl = unpk(r.l);
+    f2 a = p2_a(S), b = p2_b(S);
+    if (!(fabsf(rh.x) <= o.rmax)) a = dpres_pow(rh.x, rl.x, o.kap64);
+    if (!(fabsf(rh.y) <= o.rmax)) b = dpres_pow(rh.y, rl.y, o.kap64);
+    S = p2_of(a, b);
   }
   return ph * S;
 }
 
+// operator tables of one block in shared memory, built from OpsP: entries for the lane's row of D
+// along x and y with both halves equal, and for the rows k and k + H along z
 template <int N1>
-__device__ __forceinline__ void face_nb(const OpsP& op, int f, int ke, int ex, int ey, int ez, int nxy, long& kn,
-                                        int& levP, int kM) {
-  constexpr int N = N1 - 1;
-  levP = ez * N1 + kM;
-  switch (f) {
-    case 0: kn = (long)ke + (ey > 0 ? -op.NeX : (op.NeY - 1) * op.NeX); break;
-    case 1: kn = (long)ke + (ex < op.NeX - 1 ? 1 : -(op.NeX - 1)); break;
-    case 2: kn = (long)ke + (ey < op.NeY - 1 ? op.NeX : -(op.NeY - 1) * op.NeX); break;
-    case 3: kn = (long)ke + (ex > 0 ? -1 : op.NeX - 1); break;
-    case 4: kn = ez > 0 ? (long)ke - nxy : -1; levP = (ez - 1) * N1 + N; break;
-    default: kn = ez < op.NeZ - 1 ? (long)ke + nxy : -1; levP = (ez + 1) * N1; break;
+struct Tab {
+  static constexpr int H = N1 / 2;
+  p2m dx[N1 * N1], dy[N1 * N1];              // [l][i]: metric times D(i, l)
+  p2m dz[N1 * H], tg[N1 * H];                // [l][k]: rows k, k + H; tg: grav times VPOrdM1
+  p2m lxb[N1], lxt[N1], lyb[N1], lyt[N1];    // Fscale/2 times the Lift of the -1 and +1 faces
+  p2m lzb[H], lzt[H];
+};
+template <int N1>
+struct TabF {  // modal filter, stage 3
+  static constexpr int H = N1 / 2;
+  p2m f[N1 * N1], fz[N1 * H];
+};
+
+template <int N1, bool LAST>
+__device__ __forceinline__ void fill_tables(const OpsP& op, Tab<N1>& T, TabF<N1>* F) {
+  constexpr int H = N1 / 2;
+  for (int e = threadIdx.x; e < N1 * N1; e += blockDim.x) {
+    const int l = e / N1, r = e % N1;
+    st(T.dx[e], p2_dup(op.Dx[r * N1 + l]));
+    st(T.dy[e], p2_dup(op.Dy[r * N1 + l]));
+    if (LAST) st(F->f[e], p2_dup(op.F[r * N1 + l]));
+    if (r < H) {
+      st(T.dz[l * H + r], p2_of(op.Dz[r * N1 + l], op.Dz[(r + H) * N1 + l]));
+      st(T.tg[l * H + r], p2_of(op.Tg[r * N1 + l], op.Tg[(r + H) * N1 + l]));
+      if (LAST) st(F->fz[l * H + r], p2_of(op.Fv[r * N1 + l], op.Fv[(r + H) * N1 + l]));
+    }
+  }
+  for (int e = threadIdx.x; e < N1; e += blockDim.x) {
+    st(T.lxb[e], p2_dup(op.Lxb[e]));
+    st(T.lxt[e], p2_dup(op.Lxt[e]));
+    st(T.lyb[e], p2_dup(op.Lyb[e]));
+    st(T.lyt[e], p2_dup(op.Lyt[e]));
+    if (e < H) {
+      st(T.lzb[e], p2_of(op.Lzb[e], op.Lzb[e + H]));
+      st(T.lzt[e], p2_of(op.Lzt[e], op.Lzt[e + H]));
+    }
   }
 }
 
-// stage-3 output: modal filter (tensorprod3D_kernel.F90:2555-2618) of the five deviation fields,
-// all five per pass (three barriers), then q^{n+1} = ref + F(dev) in FP64 and its deviation pair.
-// fa, fb: [5][Np] float2 of this element (free shared memory at this point).
+// shared memory of one element
+template <int N1, bool IMP>
+struct ElemSm {
+  static constexpr int NH = N1 * N1 * N1 / 2, NF = N1 * N1;
+  p2m st[6 * NH];             // deviation state and pressure deviation
+  p2m fl[15 * NH];            // volume fluxes [direction * 5 + variable]
+  p2m df[5 * 4 * (NF / 2)];   // lateral face fluxes [variable][face][a + N1 b], nodes b and b + H
+  float2 dz[5 * 2 * NF];      // bottom and top face fluxes
+  float2 di[IMP ? 5 * 2 * NF : 1];  // vertical faces of the implicit operator
+};
+
+// one variable's filtered output in the three passes of the modal filter; q^{n+1} = ref + F(dev)
 template <int N1>
-__device__ __forceinline__ void filter_store(const OpsP& op, float2* fa, float2* fb, const f2 (&dev)[5],
-                                             const f2 (&ref)[5], const StagePairBufs& B, size_t g, bool valid,
-                                             int i, int j, int k, int p) {
-  constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
-#pragma unroll
-  for (int v = 0; v < 5; ++v) fa[v * Np + p] = f2_pack(dev[v]);
+__device__ __forceinline__ void filter_store(const TabF<N1>& F, p2m* fa, p2m* fb, const p2 (&ref)[5],
+                                             const StagePairBufs& B, size_t gA, size_t gB, bool valid, int i, int j,
+                                             int k, int t) {
+  constexpr int NF = N1 * N1, H = N1 / 2, NH = NF * H;
   __syncthreads();
+  p2acc s[5];
+#pragma unroll 1
+  for (int l = 0; l < N1; ++l) {
+    const p2 f = ld(F.f[l * N1 + i]);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) s[v].add(f, ld(fa[v * NH + l + N1 * j + NF * k]));
+  }
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
-    f2acc s1;
-#pragma unroll
-    for (int l = 0; l < N1; ++l) s1.add(f2_of(op.F[i * N1 + l]), f2_of(fa[v * Np + l + N1 * j + NF * k]));
-    fb[v * Np + p] = f2_pack(s1.get());
+    st(fb[v * NH + t], s[v].get());
+    s[v] = p2acc{};
   }
   __syncthreads();
+#pragma unroll 1
+  for (int l = 0; l < N1; ++l) {
+    const p2 f = ld(F.f[l * N1 + j]);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) s[v].add(f, ld(fb[v * NH + i + N1 * l + NF * k]));
+  }
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
-    f2acc s2;
-#pragma unroll
-    for (int l = 0; l < N1; ++l) s2.add(f2_of(op.F[j * N1 + l]), f2_of(fb[v * Np + i + N1 * l + NF * k]));
-    fa[v * Np + p] = f2_pack(s2.get());
+    st(fa[v * NH + t], s[v].get());
+    s[v] = p2acc{};
   }
   __syncthreads();
+#pragma unroll 1
+  for (int l = 0; l < H; ++l) {
+    const p2 f0 = ld(F.fz[l * H + k]), f1 = ld(F.fz[(l + H) * H + k]);
 #pragma unroll
-  for (int v = 0; v < 5; ++v) {
-    f2acc s3;
-#pragma unroll
-    for (int l = 0; l < N1; ++l) s3.add(f2_of(op.Fv[k * N1 + l]), f2_of(fa[v * Np + i + N1 * j + NF * l]));
-    if (valid) {
-      const f2 fil = s3.get();
-      const f2 out = ref[v] + fil;
-      const double o64 = (double)out.h + (double)out.l;
-      B.qn[v][g] = o64;
-      if (B.qh[0]) B.qh[v][g] = o64;
-      B.qnf[v][g] = f2_pack(fil);
+    for (int v = 0; v < 5; ++v) {
+      const p2 x = ld(fa[v * NH + i + N1 * j + NF * l]);
+      s[v].add(f0, p2_dup(p2_a(x)));
+      s[v].add(f1, p2_dup(p2_b(x)));
     }
+  }
+  if (!valid) return;
+#pragma unroll
+  for (int v = 0; v < 5; ++v) {
+    const p2 fil = s[v].get();
+    const p2 out = v == VMX || v == VMY ? ref[v] + fil : fil;
+    const double a = to64(p2_a(out)), b = to64(p2_b(out));
+    B.qn[v][gA] = a;
+    B.qn[v][gB] = b;
+    if (B.qh[0]) {
+      B.qh[v][gA] = a;
+      B.qh[v][gB] = b;
+    }
+    st2(B.qnf[v], gA, gB, fil);
   }
 }
 
 // HEVE: the explicit HEVE operator (heve.F90:292-489, heve_numflux.F90:946-1139: vertical DENS/RHOT
 // fluxes, the vertical pressure gradient and -g VFilterPM1(DDENS) explicit, unmasked wave speed) with
 // the SSP-RK3 low-storage update (timeint_rk.F90:1182-1278) in place of the IMEX ARK232 stages
-template <int N1, int EPB, int STAGE, bool HEVE = false>
-__global__ void __launch_bounds__(EPB* N1* N1* N1)
-    k_stage_pair(const OpsP op, const ProfP pf, const double* __restrict__ dens64, const StagePairBufs B,
-                 const PairCoef cf, int Ne, int filter_on, int ke0, int pf_next) {
-  constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
-  extern __shared__ float2 smp[];
-  // One block per SM leaves the latency of an element's loads uncovered when the block starts: ask
-  // L2 now for the fields of the block that will follow this one on the SM (pf_next elements on,
-  // the grid's resident width), one bulk prefetch per field and element range.
-  if (pf_next > 0 && threadIdx.x < 25) {
-    const int kn0 = ke0 + blockIdx.x * EPB + pf_next;
-    if (kn0 < Ne) {
-      const size_t off = (size_t)kn0 * Np;
-      const unsigned bytes = (unsigned)((Ne - kn0 < EPB ? Ne - kn0 : EPB) * Np * 8);
-      const int t = threadIdx.x, f = t % 5;
-      const void* src = nullptr;
-      if (t < 5) src = B.qs[f] + off;
-      else if (t < 10) src = B.qn[f] + off;
-      else if (t < 15 && !HEVE && STAGE >= 2) src = B.TI[f] + off;
-      else if (t < 20 && !HEVE && STAGE == 2) src = B.S3[f] + off;
-      else if (t < 25 && !HEVE && STAGE >= 2) src = B.SF[f] + off;
-      if (src) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-    }
-  }
-  float2* s_st = smp;                       // [EPB][6][Np]
-  float2* s_fl = s_st + EPB * 6 * Np;       // [EPB][15][Np]
-  float2* s_df = s_fl + EPB * 15 * Np;      // [EPB][5][6NF]
-  float2* s_di = s_df + EPB * 5 * 6 * NF;   // [EPB][5][2NF]
-  const int tid = threadIdx.x;
-  const int le = tid / Np, p = tid - le * Np;
+template <int N1, int EPB, int MINB, int STAGE, bool HEVE = false>
+__global__ void __launch_bounds__(EPB* N1* N1* N1 / 2, MINB)
+    k_stage_pair(const __grid_constant__ OpsP op, const ProfP pf, const __grid_constant__ StagePairBufs B,
+                 const PairCoef cf, int Ne, int filter_on, int ke0) {
+  constexpr int Np = N1 * N1 * N1, NF = N1 * N1, H = N1 / 2, NH = NF * H, N = N1 - 1, PF = NF / 2;
+  constexpr bool IMP = !HEVE && STAGE == 1;       // the implicit operator at q^n too
+  constexpr bool ZDT = HEVE || STAGE == 1;        // vertical DENS/RHOT fluxes are needed
+  using Sm = ElemSm<N1, IMP>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  Tab<N1>& T = *reinterpret_cast<Tab<N1>*>(smraw);
+  TabF<N1>* F = reinterpret_cast<TabF<N1>*>(smraw + sizeof(Tab<N1>));
+  unsigned char* sm_el = smraw + sizeof(Tab<N1>) + (STAGE == 3 ? sizeof(TabF<N1>) : 0);
+  const int le = threadIdx.x / NH, t = threadIdx.x - le * NH;
   const int ke = ke0 + blockIdx.x * EPB + le;  // elements [ke0, Ne)
   const bool valid = ke < Ne;
-  const int i = p % N1, j = (p / N1) % N1, k = p / NF;
+  const int i = t % N1, j = (t / N1) % N1, k = t / NF;  // nodes k and k + H
   const int nxy = op.NeX * op.NeY;
   const int ez = valid ? ke / nxy : 0;
   const int ey = valid ? (ke - ez * nxy) / op.NeX : 0;
   const int ex = valid ? ke - ez * nxy - ey * op.NeX : 0;
-  float2* st = s_st + le * 6 * Np;
-  float2* fl = s_fl + le * 15 * Np;
-  float2* df = s_df + le * 5 * 6 * NF;
-  float2* di = s_di + le * 5 * 2 * NF;
-  const size_t g = (size_t)ke * Np + p;
-  const int lev = ez * N1 + k;
-  const f2 U = f2_of(op.Uref), V = f2_of(op.Vref);
+  Sm& sm = reinterpret_cast<Sm*>(sm_el)[le];
+  const size_t gA = (size_t)ke * Np + t, gB = gA + NH;
+  const int levA = ez * N1 + k, levB = levA + H;
+  const p2 U = p2_dup(op.Uref), V = p2_dup(op.Vref);
 
-  f2 qv[5], dp = Z2;
-#pragma unroll
-  for (int v = 0; v < 5; ++v) qv[v] = valid ? ld2(B.qs[v] + g) : Z2;
-  const f2 dh = valid ? ld2(pf.dh + lev) : f2{1.f, 0.f};
-  if (valid) dp = dpres2(op, qv[VRT], ld2(pf.rth + lev), ld2(pf.ph + lev));
-#pragma unroll
-  for (int v = 0; v < 5; ++v) st[v * Np + p] = f2_pack(qv[v]);
-  st[5 * Np + p] = f2_pack(dp);
-  {
-    const f2 mxd = qv[VMX], myd = qv[VMY], mz = qv[VMZ], dd = qv[VD];
-    const f2 mxr = dh * U, myr = dh * V;
-    const f2 rdens = f2_recip(dd + dh);
-    const f2 ptr = valid ? ld2(pf.ptr + lev) : Z2;
-    const f2 ptd = (qv[VRT] - ptr * dd) * rdens, pt = ptr + ptd;
-    const f2 ud = (mxd - U * dd) * rdens, vd = (myd - V * dd) * rdens;
-    const f2 u = U + ud, vv = V + vd, w = mz * rdens;
-    fl[(0 * 5 + VD) * Np + p] = f2_pack(mxd);
-    fl[(1 * 5 + VD) * Np + p] = f2_pack(myd);
-    fl[(2 * 5 + VD) * Np + p] = f2_pack(mz);
-    fl[(0 * 5 + VRT) * Np + p] = f2_pack(mxr * ptd + mxd * pt);
-    fl[(1 * 5 + VRT) * Np + p] = f2_pack(myr * ptd + myd * pt);
-    fl[(2 * 5 + VRT) * Np + p] = f2_pack(mz * pt);
-    fl[(0 * 5 + VMZ) * Np + p] = f2_pack((mxr + mxd) * w);
-    fl[(1 * 5 + VMZ) * Np + p] = f2_pack((myr + myd) * w);
-    fl[(2 * 5 + VMZ) * Np + p] = f2_pack(HEVE ? mz * w + dp : mz * w);
-    fl[(0 * 5 + VMX) * Np + p] = f2_pack(mxr * ud + mxd * u + dp);
-    fl[(1 * 5 + VMX) * Np + p] = f2_pack(myr * ud + myd * u);
-    fl[(2 * 5 + VMX) * Np + p] = f2_pack(mz * u);
-    fl[(0 * 5 + VMY) * Np + p] = f2_pack(mxr * vd + mxd * vv);
-    fl[(1 * 5 + VMY) * Np + p] = f2_pack(myr * vd + myd * vv + dp);
-    fl[(2 * 5 + VMY) * Np + p] = f2_pack(mz * vv);
+  fill_tables<N1, STAGE == 3>(op, T, F);
+  const p2 dh = ld2(pf.dh, levA, levB);
+  if (valid) {
+    const p2 dd = ld2(B.qs[VD], gA, gB), mx = ld2(B.qs[VMX], gA, gB), my = ld2(B.qs[VMY], gA, gB);
+    const p2 mz = ld2(B.qs[VMZ], gA, gB), dr = ld2(B.qs[VRT], gA, gB);
+    const p2 dp = dpres2(op, dr, ld2(pf.rth, levA, levB), ld2(pf.ph, levA, levB));
+    st(sm.st[VD * NH + t], dd);
+    st(sm.st[VMX * NH + t], mx);
+    st(sm.st[VMY * NH + t], my);
+    st(sm.st[VMZ * NH + t], mz);
+    st(sm.st[VRT * NH + t], dr);
+    st(sm.st[5 * NH + t], dp);
+    const p2 rd = p2_recip(dd + dh);
+    const p2 ptr = ld2(pf.ptr, levA, levB);
+    const p2 ptd = (dr - ptr * dd) * rd, pt = ptr + ptd;
+    const p2 ud = (mx - U * dd) * rd, vd = (my - V * dd) * rd;
+    const p2 u = U + ud, v = V + vd, w = mz * rd;
+    auto put = [&](int dir, int var, p2 x) { st(sm.fl[(dir * 5 + var) * NH + t], x); };
+    {
+      const p2 R = dh * U;
+      put(0, VD, mx);
+      put(0, VRT, R * ptd + mx * pt);
+      put(0, VMZ, (R + mx) * w);
+      put(0, VMX, R * ud + mx * u + dp);
+      put(0, VMY, R * vd + mx * v);
+    }
+    {
+      const p2 R = dh * V;
+      put(1, VD, my);
+      put(1, VRT, R * ptd + my * pt);
+      put(1, VMZ, (R + my) * w);
+      put(1, VMX, R * ud + my * u);
+      put(1, VMY, R * vd + my * v + dp);
+    }
+    if (ZDT) {
+      put(2, VD, mz);
+      put(2, VRT, mz * pt);
+    }
+    put(2, VMZ, HEVE ? mz * w + dp : mz * w);
+    put(2, VMX, mz * u);
+    put(2, VMY, mz * v);
   }
   __syncthreads();
 
-  // --- HEVI Rusanov face flux in pairs (wave speed in FP32) ---
+  // --- Rusanov face flux, own side minus neighbour in pairs (wave speed in FP32); two face nodes per
+  // pass: (a, b) and (a, b + H) ---
   if (valid) {
     const float gamm = op.kap.x;
-    for (int fi = p; fi < 6 * NF; fi += Np) {
-      const int f = fi / NF, ab = fi - f * NF, a = ab % N1, b = ab / N1;
-      int iM, jM, kM;
-      face_node<N1>(f, a, b, iM, jM, kM);
-      const int pM = iM + N1 * jM + NF * kM;
+    for (int task = t; task < 6 * PF; task += NH) {
+      const int f = task / PF, ab = task - f * PF, a = ab % N1, b = ab / N1;
+      const bool vert = f >= 4, isx = (f & 1) != 0;
+      const int dir = vert ? 2 : (isx ? 0 : 1);
+      const float sg = (f == 1 || f == 2 || f == 5) ? 1.f : -1.f;
+      // own side: entry of the two nodes (lateral), or node a, b (+H) of the bottom / top plane
+      const int e = vert ? a + N1 * b + (f == 5 ? NF * (H - 1) : 0) : (isx ? (f == 1 ? N : 0) + N1 * a : a + (f == 2 ? N1 * N : 0)) + NF * b;
+      auto own = [&](const p2m* s) -> p2 {
+        if (!vert) return ld(s[e]);
+        const float* x = reinterpret_cast<const float*>(s + e) + (f == 5 ? 1 : 0);
+        return p2{pk(x[0], x[4 * N1 * H]), pk(x[2], x[2 + 4 * N1 * H])};
+      };
+      // exterior side: neighbour element, or the own node with MOMZ reflected at a lid
       long kn;
-      int levP;
-      face_nb<N1>(op, f, ke, ex, ey, ez, nxy, kn, levP, kM);
+      switch (f) {
+        case 0: kn = (long)ke + (ey > 0 ? -op.NeX : (op.NeY - 1) * op.NeX); break;
+        case 1: kn = (long)ke + (ex < op.NeX - 1 ? 1 : -(op.NeX - 1)); break;
+        case 2: kn = (long)ke + (ey < op.NeY - 1 ? op.NeX : -(op.NeY - 1) * op.NeX); break;
+        case 3: kn = (long)ke + (ex > 0 ? -1 : op.NeX - 1); break;
+        case 4: kn = ez > 0 ? (long)ke - nxy : -1; break;
+        default: kn = ez < op.NeZ - 1 ? (long)ke + nxy : -1; break;
+      }
+      const bool lid = kn < 0;
+      const int plM = f == 5 ? N : 0;                    // own plane of a vertical face
+      const int plP = lid ? plM : (f == 5 ? 0 : N);
+      const int lM0 = vert ? ez * N1 + plM : ez * N1 + b, lM1 = vert ? lM0 : lM0 + H;
+      const int lP0 = vert ? (lid ? lM0 : (f == 5 ? lM0 + 1 : lM0 - 1)) : lM0, lP1 = vert ? lP0 : lM1;
+      size_t gP = (size_t)(lid ? ke : kn) * Np;
+      if (vert) gP += a + N1 * b + NF * plP;
+      else if (isx) gP += (f == 1 ? 0 : N) + N1 * a + NF * b;
+      else gP += a + (f == 2 ? 0 : N1 * N) + NF * b;
+      const size_t gP1 = gP + (vert ? N1 * H : NF * H);
+      p2 ddP, mxP, myP, mzP, drP;
       // a boundary of a decomposed mesh: the exterior face layer comes from the halo exchange
       const int hsd = halo_side(f, ex, ey, op.NeX, op.NeY);
       const float2* hxs = hsd >= 0 ? op.hx[hsd] : nullptr;
-      const int levM = ez * N1 + kM;
-      const f2 ddM = f2_of(st[VD * Np + pM]), mxM = f2_of(st[VMX * Np + pM]), myM = f2_of(st[VMY * Np + pM]);
-      const f2 mzM = f2_of(st[VMZ * Np + pM]), drM = f2_of(st[VRT * Np + pM]), dpM = f2_of(st[5 * Np + pM]);
-      f2 ddP, mxP, myP, mzP, drP, dpP;
       if (hxs) {
-        const size_t per = halo_stride(hsd, op.NeX, op.NeY, op.NeZ, NF), h = halo_index(hsd, ex, ey, ez, ab, op.NeX, op.NeY, NF);
-        ddP = ld2(hxs + h); mxP = ld2(hxs + per + h); myP = ld2(hxs + 2 * per + h);
-        mzP = ld2(hxs + 3 * per + h); drP = ld2(hxs + 4 * per + h);
-        dpP = dpres2(op, drP, ld2(pf.rth + levP), ld2(pf.ph + levP));
-      } else if (kn >= 0) {
-        int i2, j2, k2;
-        face_node<N1>(face_opp(f), a, b, i2, j2, k2);
-        const size_t gP = (size_t)kn * Np + i2 + N1 * j2 + NF * k2;
-        ddP = ld2(B.qs[VD] + gP); mxP = ld2(B.qs[VMX] + gP); myP = ld2(B.qs[VMY] + gP);
-        mzP = ld2(B.qs[VMZ] + gP); drP = ld2(B.qs[VRT] + gP);
-        dpP = dpres2(op, drP, ld2(pf.rth + levP), ld2(pf.ph + levP));
+        const size_t per = halo_stride(hsd, op.NeX, op.NeY, op.NeZ, NF), h0 = halo_index(hsd, ex, ey, ez, ab, op.NeX, op.NeY, NF);
+        const size_t h1 = h0 + N1 * H;
+        ddP = ld2(hxs, h0, h1); mxP = ld2(hxs + per, h0, h1); myP = ld2(hxs + 2 * per, h0, h1);
+        mzP = ld2(hxs + 3 * per, h0, h1); drP = ld2(hxs + 4 * per, h0, h1);
       } else {
-        levP = levM;
-        ddP = ddM; mxP = mxM; myP = myM; mzP = -mzM; drP = drM; dpP = dpM;
+        ddP = ld2(B.qs[VD], gP, gP1); mxP = ld2(B.qs[VMX], gP, gP1); myP = ld2(B.qs[VMY], gP, gP1);
+        mzP = ld2(B.qs[VMZ], gP, gP1); drP = ld2(B.qs[VRT], gP, gP1);
+        if (lid) mzP = p2_neg(mzP);
       }
-      const float nx = (f == 1) ? 1.f : (f == 3 ? -1.f : 0.f);
-      const float ny = (f == 2) ? 1.f : (f == 0 ? -1.f : 0.f);
-      const float nz = (f == 5) ? 1.f : (f == 4 ? -1.f : 0.f);
-      const f2 fs = f >= 4 ? f2_of(op.FSz) : ((f & 1) ? f2_of(op.FSx) : f2_of(op.FSy));
-      const f2 dhM = ld2(pf.dh + levM), dhP = ld2(pf.dh + levP);
-      const f2 rdM = f2_recip(ddM + dhM), rdP = f2_recip(ddP + dhP);
-      const f2 ptrM = ld2(pf.ptr + levM), ptrP = ld2(pf.ptr + levP);
-      const f2 udM = (mxM - U * ddM) * rdM, udP = (mxP - U * ddP) * rdP;
-      const f2 vdM = (myM - V * ddM) * rdM, vdP = (myP - V * ddP) * rdP;
-      const f2 ptdM = (drM - ptrM * ddM) * rdM, ptdP = (drP - ptrP * ddP) * rdP;
-      const f2 uM = U + udM, uP = U + udP, vM = V + vdM, vP = V + vdP;
-      const f2 wM = mzM * rdM, wP = mzP * rdP;
-      const f2 mxrM = dhM * U, mxrP = dhP * U, myrM = dhM * V, myrP = dhP * V;
-      // wave speed (FP32): max(|u.n| + c) over both sides, horizontal faces only (swV)
-      const float velM = uM.h * nx + vM.h * ny + wM.h * nz, velP = uP.h * nx + vP.h * ny + wP.h * nz;
-      const float csM = sqrtf(gamm * (__ldg(pf.phf + levM) + dpM.h) * rdM.h);
-      const float csP = sqrtf(gamm * (__ldg(pf.phf + levP) + dpP.h) * rdP.h);
-      const float swV = HEVE ? 1.f : 1.f - nz * nz;
-      const float alpha = swV * fmaxf(csM + fabsf(velM), csP + fabsf(velP));
-      // normal flux deviations F.n (the reference parts cancel: same level on both sides)
-      f2 fD_M = mxM * nx + myM * ny, fD_P = mxP * nx + myP * ny;
-      f2 fR_M = (mxrM * ptdM + mxM * (ptrM + ptdM)) * nx + (myrM * ptdM + myM * (ptrM + ptdM)) * ny;
-      f2 fR_P = (mxrP * ptdP + mxP * (ptrP + ptdP)) * nx + (myrP * ptdP + myP * (ptrP + ptdP)) * ny;
-      if (HEVE) {  // vertical mass and RHOT fluxes (the reference state has no vertical flux)
-        fD_M = fD_M + mzM * nz;
-        fD_P = fD_P + mzP * nz;
-        fR_M = fR_M + mzM * (ptrM + ptdM) * nz;
-        fR_P = fR_P + mzP * (ptrP + ptdP) * nz;
+      const p2 dhM = ld2(pf.dh, lM0, lM1), dhP = ld2(pf.dh, lP0, lP1), ptrP = ld2(pf.ptr, lP0, lP1);
+      const p2 dpP = dpres2(op, drP, ld2(pf.rth, lP0, lP1), ld2(pf.ph, lP0, lP1));
+      const p2 ddM = own(sm.st + VD * NH), dpM = own(sm.st + 5 * NH);
+      const p2 rdM = p2_recip(ddM + dhM), rdP = p2_recip(ddP + dhP);
+      const p2 udP = (mxP - U * ddP) * rdP, vdP = (myP - V * ddP) * rdP;
+      const p2 uP = U + udP, vP = V + vdP, wP = mzP * rdP;
+      const p2 ptdP = (drP - ptrP * ddP) * rdP, ptP = ptrP + ptdP;
+      const p2 jdd = ddP - ddM, jdr = drP - own(sm.st + VRT * NH);
+      const p2 jmx = mxP - own(sm.st + VMX * NH), jmy = myP - own(sm.st + VMY * NH), jmz = mzP - own(sm.st + VMZ * NH);
+      // normal velocities (leading parts) and the exterior side's normal fluxes
+      float2 vnM, vnP;
+      p2 fD, fT, fX, fY, fZ;
+      if (vert) {
+        vnM = unpk((own(sm.st + VMZ * NH) * rdM).h);
+        vnP = unpk(wP.h);
+        fD = mzP;
+        fT = mzP * ptP;
+        fX = mzP * uP;
+        fY = mzP * vP;
+        fZ = HEVE ? mzP * wP + dpP : mzP * wP;
+      } else {
+        const p2 Wn = isx ? U : V, mnP = isx ? mxP : myP, R = dhP * Wn;
+        vnM = unpk((Wn + (own(sm.st + (isx ? VMX : VMY) * NH) - Wn * ddM) * rdM).h);
+        vnP = unpk(isx ? uP.h : vP.h);
+        fD = mnP;
+        fT = R * ptdP + mnP * ptP;
+        fZ = (R + mnP) * wP;
+        fX = R * udP + mnP * uP;
+        fY = R * vdP + mnP * vP;
+        if (isx) fX = fX + dpP;
+        else fY = fY + dpP;
       }
-      const f2 velM2 = uM * nx + vM * ny + wM * nz, velP2 = uP * nx + vP * ny + wP * nz;
-      const f2 fZ_M = mzM * velM2, fZ_P = mzP * velP2;
-      const f2 fX_M = (mxrM * udM + mxM * uM) * nx + (myrM * udM + myM * uM) * ny + mzM * uM * nz;
-      const f2 fX_P = (mxrP * udP + mxP * uP) * nx + (myrP * udP + myP * uP) * ny + mzP * uP * nz;
-      const f2 fY_M = (mxrM * vdM + mxM * vM) * nx + (myrM * vdM + myM * vM) * ny + mzM * vM * nz;
-      const f2 fY_P = (mxrP * vdP + mxP * vP) * nx + (myrP * vdP + myP * vP) * ny + mzP * vP * nz;
-      const f2 tmp1 = fs * 0.5f;
-      float2* o = df + ab + f * NF;
-      const int S = 6 * NF;
-      o[VD * S] = f2_pack(tmp1 * (fD_P - fD_M - (ddP - ddM) * alpha));
-      o[VRT * S] = f2_pack(tmp1 * (fR_P - fR_M - (drP - drM) * alpha));
-      o[VMZ * S] = f2_pack(HEVE ? tmp1 * (fZ_P - fZ_M + (dpP - dpM) * nz - (mzP - mzM) * alpha)
-                                : tmp1 * (fZ_P - fZ_M - (mzP - mzM) * alpha));
-      o[VMX * S] = f2_pack(tmp1 * (fX_P - fX_M + (dpP - dpM) * nx - (mxP - mxM) * alpha));
-      o[VMY * S] = f2_pack(tmp1 * (fY_P - fY_M + (dpP - dpM) * ny - (myP - myM) * alpha));
-      if (!HEVE && STAGE == 1 && f >= 4) {
-        // vertical faces of the implicit operator at var0 = q^n (hevi_common_2.F90:1016-1328)
-        const float al = fmaxf(fabsf(wM.h) + csM, fabsf(wP.h) + csP);
-        const f2 tm = f2_of(op.FSz) * 0.5f;
-        const f2 potM = (ld2(pf.th + levM) + drM) * rdM, potP = (ld2(pf.th + levP) + drP) * rdP;
-        float2* oi = di + ab + (f - 4) * NF;
-        const int S2 = 2 * NF;
-        oi[VD * S2] = f2_pack(tm * ((mzP - mzM) * nz - (ddP - ddM) * al));
-        oi[VMZ * S2] = f2_pack(tm * ((dpP - dpM) * nz - (mzP - mzM) * al));
-        oi[VRT * S2] = f2_pack(tm * ((potP * mzP - potM * mzM) * nz - (drP - drM) * al));
-        oi[VMX * S2] = f2_pack(-(tm * ((mxP - mxM) * al)));
-        oi[VMY * S2] = f2_pack(-(tm * ((myP - myM) * al)));
+      const float2 dpMh = unpk(dpM.h), dpPh = unpk(dpP.h), rMh = unpk(rdM.h), rPh = unpk(rdP.h);
+      const float csM0 = sqrtf(gamm * (__ldg(pf.phf + lM0) + dpMh.x) * rMh.x), csM1 = sqrtf(gamm * (__ldg(pf.phf + lM1) + dpMh.y) * rMh.y);
+      const float csP0 = sqrtf(gamm * (__ldg(pf.phf + lP0) + dpPh.x) * rPh.x), csP1 = sqrtf(gamm * (__ldg(pf.phf + lP1) + dpPh.y) * rPh.y);
+      const u64x al = pk(fmaxf(csM0 + fabsf(vnM.x), csP0 + fabsf(vnP.x)), fmaxf(csM1 + fabsf(vnM.y), csP1 + fabsf(vnP.y)));
+      const u64x sg2 = pk1(sg);
+      const p2m* flM = sm.fl + dir * 5 * NH;
+      auto jump = [&](p2 fP, int var) { return p2_scale(fP - own(flM + var * NH), sg2); };
+      if (!vert) {
+        p2m* o = sm.df + f * PF + ab;
+        constexpr int S = 4 * PF;
+        st(o[VD * S], jump(fD, VD) - p2_mul_x(jdd, al));
+        st(o[VRT * S], jump(fT, VRT) - p2_mul_x(jdr, al));
+        st(o[VMZ * S], jump(fZ, VMZ) - p2_mul_x(jmz, al));
+        st(o[VMX * S], jump(fX, VMX) - p2_mul_x(jmx, al));
+        st(o[VMY * S], jump(fY, VMY) - p2_mul_x(jmy, al));
+      } else {
+        auto putz = [&](float2* s, int var, p2 x) {
+          float2* o = s + (var * 2 + (f - 4)) * NF + ab;
+          st2(o, 0, N1 * H, x);
+        };
+        if (HEVE) {
+          putz(sm.dz, VD, jump(fD, VD) - p2_mul_x(jdd, al));
+          putz(sm.dz, VRT, jump(fT, VRT) - p2_mul_x(jdr, al));
+          putz(sm.dz, VMZ, jump(fZ, VMZ) - p2_mul_x(jmz, al));
+          putz(sm.dz, VMX, jump(fX, VMX) - p2_mul_x(jmx, al));
+          putz(sm.dz, VMY, jump(fY, VMY) - p2_mul_x(jmy, al));
+        } else {  // HEVI: no vertical mass and RHOT flux, no vertical wave speed
+          putz(sm.dz, VMZ, jump(fZ, VMZ));
+          putz(sm.dz, VMX, jump(fX, VMX));
+          putz(sm.dz, VMY, jump(fY, VMY));
+        }
+        if (IMP) {  // vertical faces of the implicit operator at var0 = q^n (hevi_common_2.F90:1016-1328)
+          putz(sm.di, VD, p2_scale(jmz, sg2) - p2_mul_x(jdd, al));
+          putz(sm.di, VMZ, p2_scale(dpP - dpM, sg2) - p2_mul_x(jmz, al));
+          putz(sm.di, VRT, jump(fT, VRT) - p2_mul_x(jdr, al));
+          putz(sm.di, VMX, p2_neg(p2_mul_x(jmx, al)));
+          putz(sm.di, VMY, p2_neg(p2_mul_x(jmy, al)));
+        }
+      }
+    }
+  }
+  // --- the derivative along x, y and z and the Lift, one compensated sum per variable; the
+  // derivatives need the volume fluxes only, so they run before the barrier that completes the faces
+  // (the loops stay rolled: the kernel's code competes for the instruction caches) ---
+  const int col = i + N1 * j;
+  p2acc s[5];
+  if (valid) {
+#pragma unroll 1
+    for (int l = 0; l < N1; ++l) {
+      const p2 dx = ld(T.dx[l * N1 + i]), dy = ld(T.dy[l * N1 + j]);
+#pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        s[v].add(dx, ld(sm.fl[v * NH + l + N1 * j + NF * k]));
+        s[v].add(dy, ld(sm.fl[(5 + v) * NH + i + N1 * l + NF * k]));
+      }
+    }
+#pragma unroll 1
+    for (int l = 0; l < H; ++l) {
+      const p2 d0 = ld(T.dz[l * H + k]), d1 = ld(T.dz[(l + H) * H + k]);
+#pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        if (!HEVE && (v == VD || v == VRT)) continue;
+        const p2 z = ld(sm.fl[(10 + v) * NH + col + NF * l]);
+        s[v].add(d0, p2_dup(p2_a(z)));
+        s[v].add(d1, p2_dup(p2_b(z)));
+      }
+    }
+    if (HEVE) {  // -g VFilterPM1(DDENS) (heve.F90:447-452)
+#pragma unroll 1
+      for (int l = 0; l < H; ++l) {
+        const p2 z = ld(sm.st[VD * NH + col + NF * l]);
+        s[VMZ].add(ld(T.tg[l * H + k]), p2_dup(p2_a(z)));
+        s[VMZ].add(ld(T.tg[(l + H) * H + k]), p2_dup(p2_b(z)));
       }
     }
   }
   __syncthreads();
 
-  f2 tex[5], tim[5];
+  p2 tex[5], tim[5];
   if (valid) {
-    const int S = 6 * NF;
-    f2 szv[5];
+    {
+      const p2 lyb = ld(T.lyb[j]), lxt = ld(T.lxt[i]), lyt = ld(T.lyt[j]), lxb = ld(T.lxb[i]);
+      const p2 lzb = ld(T.lzb[k]), lzt = ld(T.lzt[k]);
 #pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      f2acc sx, sy, sz;
-#pragma unroll
-      for (int l = 0; l < N1; ++l) {
-        sx.add(f2_of(op.D[i * N1 + l]), f2_of(fl[(0 * 5 + v) * Np + l + N1 * j + NF * k]));
-        sy.add(f2_of(op.D[j * N1 + l]), f2_of(fl[(1 * 5 + v) * Np + i + N1 * l + NF * k]));
-        sz.add(f2_of(op.D[k * N1 + l]), f2_of(fl[(2 * 5 + v) * Np + i + N1 * j + NF * l]));
-      }
-      szv[v] = sz.get();
-      const float2* d = df + v * S;
-      f2acc lf;
-      lf.add(f2_of(op.Lb[j]), f2_of(d[0 * NF + i + N1 * k]));
-      lf.add(f2_of(op.Lt[i]), f2_of(d[1 * NF + j + N1 * k]));
-      lf.add(f2_of(op.Lt[j]), f2_of(d[2 * NF + i + N1 * k]));
-      lf.add(f2_of(op.Lb[i]), f2_of(d[3 * NF + j + N1 * k]));
-      lf.add(f2_of(op.Lb[k]), f2_of(d[4 * NF + i + N1 * j]));
-      lf.add(f2_of(op.Lt[k]), f2_of(d[5 * NF + i + N1 * j]));
-      const bool horiz_only = !HEVE && (v == VD || v == VRT);
-      f2 s = f2_of(op.E11) * sx.get() + f2_of(op.E22) * sy.get() + lf.get();
-      if (!horiz_only) s = s + f2_of(op.E33) * szv[v];
-      tex[v] = -s;
-    }
-    tex[VMX] = tex[VMX] + f2_of(op.cor) * (qv[VMY] + dh * V);
-    tex[VMY] = tex[VMY] - f2_of(op.cor) * (qv[VMX] + dh * U);
-    if (pf.sl) {  // sponge layer on the explicit tendency (driver_nonhydro3d.F90:831-841)
-      const f2 cz = ld2(pf.sl + lev);
-      tex[VMZ] = tex[VMZ] - cz * qv[VMZ];
-      if (pf.sl_h != 0.f) {
-        tex[VMX] = tex[VMX] - cz * (qv[VMX] + dh * U);
-        tex[VMY] = tex[VMY] - cz * (qv[VMY] + dh * V);
+      for (int v = 0; v < 5; ++v) {
+        const p2m* d = sm.df + v * 4 * PF;
+        s[v].add(lyb, ld(d[i + N1 * k]));
+        s[v].add(lxt, ld(d[PF + j + N1 * k]));
+        s[v].add(lyt, ld(d[2 * PF + i + N1 * k]));
+        s[v].add(lxb, ld(d[3 * PF + j + N1 * k]));
+        if (HEVE || (v != VD && v != VRT)) {
+          s[v].add(lzb, p2_dup(sm.dz[v * 2 * NF + col]));
+          s[v].add(lzt, p2_dup(sm.dz[(v * 2 + 1) * NF + col]));
+        }
       }
     }
-    if (HEVE) {  // -g VFilterPM1(DDENS) (heve.F90:447-452)
-      f2acc drho;
 #pragma unroll
-      for (int l = 0; l < N1; ++l) drho.add(f2_of(op.T[k * N1 + l]), f2_of(st[VD * Np + i + N1 * j + NF * l]));
-      tex[VMZ] = tex[VMZ] - f2_of(op.grav) * drho.get();
-#pragma unroll
-      for (int v = 0; v < 5; ++v) tim[v] = Z2;
-    } else if (STAGE == 1) {
-      f2acc sdp, drho;
-#pragma unroll
-      for (int l = 0; l < N1; ++l) {
-        sdp.add(f2_of(op.D[k * N1 + l]), f2_of(st[5 * Np + i + N1 * j + NF * l]));
-        drho.add(f2_of(op.T[k * N1 + l]), f2_of(st[VD * Np + i + N1 * j + NF * l]));
+    for (int v = 0; v < 5; ++v) tex[v] = p2_neg(s[v].get());
+    if (op.cor.x != 0.f || pf.sl) {
+      const p2 mx = ld(sm.st[VMX * NH + t]) + dh * U, my = ld(sm.st[VMY * NH + t]) + dh * V;
+      tex[VMX] = tex[VMX] + p2_dup(op.cor) * my;
+      tex[VMY] = tex[VMY] - p2_dup(op.cor) * mx;
+      if (pf.sl) {  // sponge layer on the explicit tendency (driver_nonhydro3d.F90:831-841)
+        const p2 cz = ld2(pf.sl, levA, levB);
+        tex[VMZ] = tex[VMZ] - cz * ld(sm.st[VMZ * NH + t]);
+        if (pf.sl_h != 0.f) {
+          tex[VMX] = tex[VMX] - cz * mx;
+          tex[VMY] = tex[VMY] - cz * my;
+        }
       }
-      const int S2 = 2 * NF, fb = i + N1 * j, ft = NF + i + N1 * j;
-      const f2 lb = f2_of(op.Lb[k]), lt = f2_of(op.Lt[k]), E33 = f2_of(op.E33);
-      auto dv = [&](int v, int o) { return f2_of(di[v * S2 + o]); };
-      tim[VD] = -(E33 * szv[VD] + lb * dv(VD, fb) + lt * dv(VD, ft));
-      tim[VMZ] = -(E33 * sdp.get() + lb * dv(VMZ, fb) + lt * dv(VMZ, ft) + f2_of(op.grav) * drho.get());
-      tim[VRT] = -(E33 * szv[VRT] + lb * dv(VRT, fb) + lt * dv(VRT, ft));
-      tim[VMX] = -(lb * dv(VMX, fb) + lt * dv(VMX, ft));
-      tim[VMY] = -(lb * dv(VMY, fb) + lt * dv(VMY, ft));
+    }
+    if constexpr (IMP) {  // the implicit operator at q^n
+      p2acc a[5];
+      const p2 lzb = ld(T.lzb[k]), lzt = ld(T.lzt[k]);
+#pragma unroll 1
+      for (int l = 0; l < H; ++l) {
+        const p2 d0 = ld(T.dz[l * H + k]), d1 = ld(T.dz[(l + H) * H + k]);
+        const p2 g0 = ld(T.tg[l * H + k]), g1 = ld(T.tg[(l + H) * H + k]);
+        const p2 m = ld(sm.fl[(10 + VD) * NH + col + NF * l]), r = ld(sm.fl[(10 + VRT) * NH + col + NF * l]);
+        const p2 p = ld(sm.st[5 * NH + col + NF * l]), d = ld(sm.st[VD * NH + col + NF * l]);
+        a[VD].add(d0, p2_dup(p2_a(m)));
+        a[VD].add(d1, p2_dup(p2_b(m)));
+        a[VRT].add(d0, p2_dup(p2_a(r)));
+        a[VRT].add(d1, p2_dup(p2_b(r)));
+        a[VMZ].add(d0, p2_dup(p2_a(p)));
+        a[VMZ].add(d1, p2_dup(p2_b(p)));
+        a[VMZ].add(g0, p2_dup(p2_a(d)));
+        a[VMZ].add(g1, p2_dup(p2_b(d)));
+      }
+#pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        a[v].add(lzb, p2_dup(sm.di[v * 2 * NF + col]));
+        a[v].add(lzt, p2_dup(sm.di[(v * 2 + 1) * NF + col]));
+        tim[v] = p2_neg(a[v].get());
+      }
       if (B.a0[0]) {
-        B.a0[0][g] = f2_pack(tim[VD]);
-        B.a0[1][g] = f2_pack(tim[VMZ]);
-        B.a0[2][g] = f2_pack(tim[VRT]);
+        st2(B.a0[0], gA, gB, tim[VD]);
+        st2(B.a0[1], gA, gB, tim[VMZ]);
+        st2(B.a0[2], gA, gB, tim[VRT]);
       }
-    } else {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) tim[v] = ld2(B.TI[v] + g);
     }
   }
 
   // --- fused RK epilogue in pairs ---
-  const f2 dt = f2_of(cf.dt);
+  auto qn64 = [&](int v) { return p2_split(__ldg(B.qn[v] + gA), __ldg(B.qn[v] + gB)); };
   if constexpr (HEVE) {
     // ERK_SSP_3s3o on the deviations (the reference state does not change in time): q1 = qn + dt t(qn),
     // q2 = 3/4 qn + 1/4 (q1 + dt t(q1)), q3 = 1/3 qn + 2/3 (q2 + dt t(q2)); the stage inputs and
     // outputs are deviation pairs, qn is split from the FP64 state
-    f2 dev[5], ref[5];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      ref[v] = v == VMX ? dh * U : (v == VMY ? dh * V : Z2);
-      dev[v] = Z2;
-      if (valid) {
-        const f2 qnd = f2_split(__ldg(B.qn[v] + g)) - ref[v];
-        const f2 up = qv[v] + dt * tex[v];
-        dev[v] = STAGE == 1 ? up
-                            : (STAGE == 2 ? f2_of(cf.ssp[0]) * qnd + f2_of(cf.ssp[1]) * up
-                                          : f2_of(cf.ssp[2]) * qnd + f2_of(cf.ssp[3]) * up);
-      }
-    }
     if (STAGE < 3) {
       if (valid) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) B.qi[v][g] = f2_pack(dev[v]);
-      }
-      return;
-    }
-    if (B.dtrc && valid) B.dtrc[g] = (double)dev[VD].h + (double)dev[VD].l;  // DDENS_TRC: before the filter
-    if (!filter_on) {
-      if (valid) {
-#pragma unroll
         for (int v = 0; v < 5; ++v) {
-          const f2 out = ref[v] + dev[v];
-          const double o64 = (double)out.h + (double)out.l;
-          B.qn[v][g] = o64;
-          if (B.qh[0]) B.qh[v][g] = o64;
-          B.qnf[v][g] = f2_pack(dev[v]);
+          const p2 up = ld(sm.st[v * NH + t]) + p2_dup(cf.dt) * tex[v];
+          p2 dev = up;
+          if (STAGE == 2) {
+            p2 qnd = qn64(v);
+            if (v == VMX || v == VMY) qnd = qnd - dh * (v == VMX ? U : V);
+            dev = p2_dup(cf.ssp[0]) * qnd + p2_dup(cf.ssp[1]) * up;
+          }
+          st2(B.qi[v], gA, gB, dev);
         }
       }
       return;
     }
-    __syncthreads();  // everyone is done with the shared arrays
-    filter_store<N1>(op, s_st + le * 6 * Np, s_fl + le * 15 * Np, dev, ref, B, g, valid, i, j, k, p);
-    return;
   }
-  if (STAGE == 1 || STAGE == 2) {
-    float xq[3] = {0.f, 0.f, 0.f};
+  if constexpr (!HEVE && STAGE < 3) {
+    float xqA[3] = {0.f, 0.f, 0.f}, xqB[3] = {0.f, 0.f, 0.f};
     if (valid) {
 #pragma unroll
       for (int v = 0; v < 5; ++v) {
-        const f2 qn = f2_split(__ldg(B.qn[v] + g));
-        f2 qs;
+        p2 qs;
         if (STAGE == 1) {
-          qs = qn + dt * (f2_of(cf.a21e) * tex[v] + f2_of(cf.a21i) * tim[v]);
-          B.S3[v][g] = f2_pack(f2_of(cf.a31e) * tex[v] + f2_of(cf.a31i) * tim[v]);
-          B.SF[v][g] = f2_pack(f2_of(cf.b1) * (tex[v] + tim[v]));
+          qs = qn64(v) + (p2_dup(cf.q1e) * tex[v] + p2_dup(cf.q1i) * tim[v]);
+          st2(B.S3[v], gA, gB, p2_dup(cf.s3e) * tex[v] + p2_dup(cf.s3i) * tim[v]);
+          st2(B.SF[v], gA, gB, p2_dup(cf.sf1) * (tex[v] + tim[v]));
         } else {
-          const f2 s3 = ld2(B.S3[v] + g) + f2_of(cf.a32e) * tex[v] + f2_of(cf.a32i) * tim[v];
-          qs = qn + dt * s3;
-          B.SF[v][g] = f2_pack(ld2(B.SF[v] + g) + f2_of(cf.b2) * (tex[v] + tim[v]));
+          const p2 ti = ld2(B.TI[v], gA, gB);
+          qs = qn64(v) + (ld2(B.S3[v], gA, gB) + p2_dup(cf.q2e) * tex[v] + p2_dup(cf.q2i) * ti);
+          st2(B.SF[v], gA, gB, ld2(B.SF[v], gA, gB) + p2_dup(cf.sf2) * (tex[v] + ti));
         }
-        B.qi[v][g] = f2_pack(qs);
-        if (v == VD) xq[0] = qs.h;
-        if (v == VMZ) xq[1] = qs.h;
-        if (v == VRT) xq[2] = qs.h;
+        st2(B.qi[v], gA, gB, qs);
+        const int m = v == VD ? 0 : (v == VMZ ? 1 : (v == VRT ? 2 : -1));
+        if (m >= 0) {
+          xqA[m] = unpk(qs.h).x;
+          xqB[m] = unpk(qs.h).y;
+        }
       }
     }
     if (B.X) {  // the element's q* as feature rows of the guess network
       __syncthreads();
-      __nv_bfloat16* sx = reinterpret_cast<__nv_bfloat16*>(st);  // [NF][3][N1]
+      __nv_bfloat16* sx = reinterpret_cast<__nv_bfloat16*>(sm.st);  // [NF][3][N1]
 #pragma unroll
-      for (int v = 0; v < 3; ++v) sx[((i + N1 * j) * 3 + v) * N1 + k] = __float2bfloat16_rn(xq[v] * B.xs[v]);
+      for (int v = 0; v < 3; ++v) {
+        sx[((i + N1 * j) * 3 + v) * N1 + k] = __float2bfloat16_rn(xqA[v] * B.xs[v]);
+        sx[((i + N1 * j) * 3 + v) * N1 + k + H] = __float2bfloat16_rn(xqB[v] * B.xs[v]);
+      }
       __syncthreads();
-      if (valid && p < 3 * NF) {
-        const int cij = p / 3, v = p - 3 * cij;
-        const size_t row = (size_t)(ex + op.NeX * ey) * NF + cij;
-        __nv_bfloat16* dst = B.X + row * B.xdinp + v * op.L + ez * N1;
-        if constexpr (N1 == 8) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(sx + (cij * 3 + v) * N1);
-        else *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(sx + (cij * 3 + v) * N1);
+      if (valid) {
+        for (int c = t; c < 3 * NF; c += NH) {
+          const int cij = c / 3, v = c - 3 * cij;
+          const size_t row = (size_t)(ex + op.NeX * ey) * NF + cij;
+          __nv_bfloat16* dst = B.X + row * B.xdinp + v * op.L + ez * N1;
+          if constexpr (N1 == 8) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(sx + (cij * 3 + v) * N1);
+          else *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(sx + (cij * 3 + v) * N1);
+        }
       }
     }
     return;
   }
-  // STAGE 3: q^{n+1} = q^n + dt (SF + b3 (t_ex + t_im)), then the modal filter of the deviation
-  // from the reference state (DENS_hyd*(Uref, Vref) for MOMX/MOMY, 0 otherwise)
-  f2 qnew[5], dev[5], ref[5];
+  if constexpr (STAGE == 3) {
+    // q^{n+1}, then the modal filter (tensorprod3D_kernel.F90:2555-2618) of its deviation from the
+    // reference state (DENS_hyd*(Uref, Vref) for MOMX/MOMY, 0 otherwise)
+    p2 dev[5], ref[5];
 #pragma unroll
-  for (int v = 0; v < 5; ++v) {
-    qnew[v] = Z2;
-    dev[v] = Z2;
-    ref[v] = v == VMX ? dh * U : (v == VMY ? dh * V : Z2);
-    if (valid) {
-      qnew[v] = f2_split(__ldg(B.qn[v] + g)) + dt * (ld2(B.SF[v] + g) + f2_of(cf.b3) * (tex[v] + tim[v]));
-      dev[v] = qnew[v] - ref[v];
-    }
-  }
-  if (B.dtrc && valid) B.dtrc[g] = (double)qnew[VD].h + (double)qnew[VD].l;  // DDENS_TRC: before the filter
-  if (!filter_on) {
-    if (valid) {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) {
-        const double o64 = (double)qnew[v].h + (double)qnew[v].l;
-        B.qn[v][g] = o64;
-        if (B.qh[0]) B.qh[v][g] = o64;
-        B.qnf[v][g] = f2_pack(dev[v]);
+    for (int v = 0; v < 5; ++v) {
+      const bool mom = v == VMX || v == VMY;
+      ref[v] = mom ? dh * (v == VMX ? U : V) : p2_zero();
+      dev[v] = p2_zero();
+      if (!valid) continue;
+      const p2 qn = qn64(v);
+      if (HEVE) {
+        const p2 up = ld(sm.st[v * NH + t]) + p2_dup(cf.dt) * tex[v];
+        dev[v] = p2_dup(cf.ssp[2]) * (mom ? qn - ref[v] : qn) + p2_dup(cf.ssp[3]) * up;
+      } else {
+        const p2 qnew = qn + (ld2(B.SF[v], gA, gB) + p2_dup(cf.sf3) * (tex[v] + ld2(B.TI[v], gA, gB)));
+        dev[v] = mom ? qnew - ref[v] : qnew;
       }
     }
-    return;
+    if (B.dtrc && valid) {  // DDENS_TRC: before the filter
+      B.dtrc[gA] = to64(p2_a(dev[VD]));
+      B.dtrc[gB] = to64(p2_b(dev[VD]));
+    }
+    if (!filter_on) {
+      if (valid) {
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+          const p2 out = v == VMX || v == VMY ? ref[v] + dev[v] : dev[v];
+          const double a = to64(p2_a(out)), b = to64(p2_b(out));
+          B.qn[v][gA] = a;
+          B.qn[v][gB] = b;
+          if (B.qh[0]) {
+            B.qh[v][gA] = a;
+            B.qh[v][gB] = b;
+          }
+          st2(B.qnf[v], gA, gB, dev[v]);
+        }
+      }
+      return;
+    }
+    // every thread of the block is past its reads of the other nodes' state (HEVE reads it in the
+    // gravity term above), and the own entries are read; the flux arrays are read until here
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < 5; ++v) st(sm.st[v * NH + t], dev[v]);
+    filter_store<N1>(*F, sm.st, sm.fl, ref, B, gA, gB, valid, i, j, k, t);
   }
-  __syncthreads();  // everyone is done with the shared arrays
-  filter_store<N1>(op, s_st + le * 6 * Np, s_fl + le * 15 * Np, dev, ref, B, g, valid, i, j, k, p);
 }
 
 template <int N1>
-constexpr int epb_p() { return N1 == 4 ? 4 : 1; }
+constexpr int epb_p() { return N1 == 4 ? 2 : 1; }
+template <int N1>
+constexpr int minb_p() { return N1 == 4 ? 8 : 2; }
 
 template <int N1, int STAGE, bool HEVE = false>
-int launch_pair_n(const OpsP& op, const ProfP& pf, const double* dens64, const StagePairBufs& B, const PairCoef& cf,
-                  int Ne, int filt, cudaStream_t s, int ke0 = 0) {
-  constexpr int EPB = epb_p<N1>(), Np = N1 * N1 * N1, NF = N1 * N1;
-  const size_t smem = sizeof(float2) * EPB * (21 * Np + 5 * 6 * NF + 5 * 2 * NF);
-  auto kfn = k_stage_pair<N1, EPB, STAGE, HEVE>;
+int launch_pair_n(const OpsP& op, const ProfP& pf, const StagePairBufs& B, const PairCoef& cf, int Ne, int filt,
+                  cudaStream_t s, int ke0 = 0) {
+  constexpr int EPB = epb_p<N1>(), Np = N1 * N1 * N1;
+  constexpr size_t smem = sizeof(Tab<N1>) + (STAGE == 3 ? sizeof(TabF<N1>) : 0) + EPB * sizeof(ElemSm<N1, !HEVE && STAGE == 1>);
+  auto kfn = k_stage_pair<N1, EPB, minb_p<N1>(), STAGE, HEVE>;
   cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (Ne <= ke0) return (int)cudaSuccess;
-  // the grid's resident width in elements: the block that follows a block on its SM starts about
-  // that many elements further on
-  int dev = 0, nsm = 0, nb = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kfn, EPB * Np, smem);
-  const int pf_next = nsm * nb * EPB;
-  kfn<<<(Ne - ke0 + EPB - 1) / EPB, EPB * Np, smem, s>>>(op, pf, dens64, B, cf, Ne, filt, ke0, pf_next);
+  kfn<<<(Ne - ke0 + EPB - 1) / EPB, EPB * Np / 2, smem, s>>>(op, pf, B, cf, Ne, filt, ke0);
   return (int)cudaGetLastError();
 }
 
 }  // namespace
 
-int launch_stage_pair_heve(int N1, int stage, const OpsP& op, const ProfP& pf, const double* dens64,
-                           const StagePairBufs& B, const PairCoef& cf, int Ne, int filt, cudaStream_t s) {
+int launch_stage_pair_heve(int N1, int stage, const OpsP& op, const ProfP& pf, const StagePairBufs& B,
+                           const PairCoef& cf, int Ne, int filt, cudaStream_t s) {
   if (N1 == 8) {
-    if (stage == 1) return launch_pair_n<8, 1, true>(op, pf, dens64, B, cf, Ne, filt, s);
-    if (stage == 2) return launch_pair_n<8, 2, true>(op, pf, dens64, B, cf, Ne, filt, s);
-    return launch_pair_n<8, 3, true>(op, pf, dens64, B, cf, Ne, filt, s);
+    if (stage == 1) return launch_pair_n<8, 1, true>(op, pf, B, cf, Ne, filt, s);
+    if (stage == 2) return launch_pair_n<8, 2, true>(op, pf, B, cf, Ne, filt, s);
+    return launch_pair_n<8, 3, true>(op, pf, B, cf, Ne, filt, s);
   }
   if (N1 == 4) {
-    if (stage == 1) return launch_pair_n<4, 1, true>(op, pf, dens64, B, cf, Ne, filt, s);
-    if (stage == 2) return launch_pair_n<4, 2, true>(op, pf, dens64, B, cf, Ne, filt, s);
-    return launch_pair_n<4, 3, true>(op, pf, dens64, B, cf, Ne, filt, s);
+    if (stage == 1) return launch_pair_n<4, 1, true>(op, pf, B, cf, Ne, filt, s);
+    if (stage == 2) return launch_pair_n<4, 2, true>(op, pf, B, cf, Ne, filt, s);
+    return launch_pair_n<4, 3, true>(op, pf, B, cf, Ne, filt, s);
   }
   return (int)cudaErrorInvalidValue;
 }
 
-int launch_stage_pair(int N1, int stage, const OpsP& op, const ProfP& pf, const double* dens64,
-                      const StagePairBufs& B, const PairCoef& cf, int Ne, int filt, cudaStream_t s, int ke0) {
+int launch_stage_pair(int N1, int stage, const OpsP& op, const ProfP& pf, const StagePairBufs& B,
+                      const PairCoef& cf, int Ne, int filt, cudaStream_t s, int ke0) {
   if (N1 == 8) {
-    if (stage == 1) return launch_pair_n<8, 1>(op, pf, dens64, B, cf, Ne, filt, s, ke0);
-    if (stage == 2) return launch_pair_n<8, 2>(op, pf, dens64, B, cf, Ne, filt, s, ke0);
-    return launch_pair_n<8, 3>(op, pf, dens64, B, cf, Ne, filt, s, ke0);
+    if (stage == 1) return launch_pair_n<8, 1>(op, pf, B, cf, Ne, filt, s, ke0);
+    if (stage == 2) return launch_pair_n<8, 2>(op, pf, B, cf, Ne, filt, s, ke0);
+    return launch_pair_n<8, 3>(op, pf, B, cf, Ne, filt, s, ke0);
   }
   if (N1 == 4) {
-    if (stage == 1) return launch_pair_n<4, 1>(op, pf, dens64, B, cf, Ne, filt, s, ke0);
-    if (stage == 2) return launch_pair_n<4, 2>(op, pf, dens64, B, cf, Ne, filt, s, ke0);
-    return launch_pair_n<4, 3>(op, pf, dens64, B, cf, Ne, filt, s, ke0);
+    if (stage == 1) return launch_pair_n<4, 1>(op, pf, B, cf, Ne, filt, s, ke0);
+    if (stage == 2) return launch_pair_n<4, 2>(op, pf, B, cf, Ne, filt, s, ke0);
+    return launch_pair_n<4, 3>(op, pf, B, cf, Ne, filt, s, ke0);
   }
   return (int)cudaErrorInvalidValue;
 }
