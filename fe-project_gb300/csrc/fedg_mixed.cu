@@ -666,6 +666,7 @@ struct MixedState {
   OpsP opp;
   OpsF opf;
   OpsX opx;
+  float hyd[3] = {};         // DENS_hyd and RHOT_hyd of the lowest level, smallest DENS_hyd
   double Uref = 0.0, Vref = 0.0;
   bool wind_set = false;
   float2* qi(int v) { return qpair + (size_t)v * n; }
@@ -768,6 +769,9 @@ static int mixed_setup(fedg_ctx* c) {
     pf2[2 * L + l] = split_host(hp[3 * L + l]);
     pf2[3 * L + l] = split_host(1.0 / hp[3 * L + l]);
   }
+  m->hyd[0] = pfh[0];
+  m->hyd[1] = (float)hp[3 * L];
+  m->hyd[2] = *std::min_element(pfh.begin(), pfh.begin() + L);
   float* hptr[13];
   for (int v = 0; v < 5; ++v) hptr[v] = m->TI(v);
   for (int v = 0; v < 3; ++v) hptr[5 + v] = m->GU(v);
@@ -1186,6 +1190,16 @@ int mixed_update(fedg_ctx* c, double* const q[5], int nsteps, const fedg_update_
     }
     return tracked(c, FEDG_K_MVI, [&] {
       const A3 a0{{m->a0buf, m->a0buf + c->n, m->a0buf + 2 * c->n}};
+      // pairs from var0: the series kernel first, then block LU for the columns it leaves.  FP32 outputs,
+      // the learned iterate and the LU-only setting take the LU kernel alone
+      if (pair && !gptr && va.neumann > 0) {
+        const int rs = launch_vi_series(c->N1, c->op, m->opx, px, qin, z, a0, qo, to, m->gsc, c->d_status, c->d_cnt, va,
+                                        m->hyd, c->stream);
+        if (rs > 0) return rs;
+        if (rs == 0)
+          return launch_vi_cols(c->N1, c->op, m->opx, px, qin, z, a0, gptr, qo, to, m->gsc, c->d_status, c->d_cnt, va, pair,
+                                c->stream, true);
+      }
       return launch_vi_cols(c->N1, c->op, m->opx, px, qin, z, a0, gptr, qo, to, m->gsc, c->d_status, c->d_cnt, va, pair,
                             c->stream);
     });

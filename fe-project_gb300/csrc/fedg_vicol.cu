@@ -1,5 +1,6 @@
-// fedg_vicol.cu -- HEVI column Newton solve of the mixed-precision path (cal_vi), N1 lanes per
-// column and 32/N1 columns per warp.
+// fedg_vicol.cu -- HEVI column Newton solve of the mixed-precision path (cal_vi) by block LU, N1 lanes
+// per column and 32/N1 columns per warp: every column of the FP32 mode, of the learned iterate and of the
+// LU-only setting, and the columns that the float-pair mode's series kernel (fedg_viseries.cu) leaves.
 //
 // FElib's cal_vi (FElib/src/atmosphere/dynamics/scale_atm_dyn_dgm_nonhydro3d_rhot_hevi.F90:
 // 772-965, the operators of scale_atm_dyn_dgm_nonhydro3d_hevi_common_2.F90) solves, column by
@@ -847,7 +848,7 @@ __device__ void col_neumann(const Ops& op, const ProfX& px, float kapf, const Co
 }
 
 // ---------------------------------------------------------------------------------------------
-template <int N1, bool PO>
+template <int N1, bool PO, bool REDO>
 __global__ void __launch_bounds__(64, 6) k_vi_cols(const Ops op, const OpsX ox, const ProfX px, const X5 qin, const F5c z,
                                                 const A3 a0, const float* const* guess, void* const* qsf, void* const* tout,
                                                 float* __restrict__ gsc, int* status, unsigned long long* cnt,
@@ -859,9 +860,11 @@ __global__ void __launch_bounds__(64, 6) k_vi_cols(const Ops op, const OpsX ox, 
   // reservation cost a whole warp of occupancy per SM
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int grp = lane / N1, k = lane % N1;
-  const int col0 = (blockIdx.x * 2 + wib) * C;
-  if (col0 >= ncol) return;  // ncol is a multiple of C: warps are all-valid or all-invalid (no block barriers)
+  // ncol is a multiple of C: a warp's columns are all valid or none (no block barriers).  REDO: only the
+  // warps with a column marked VI_REDO by the series kernel, which the grid's warps look for in turn
+  for (int col0 = (blockIdx.x * 2 + wib) * C; col0 < ncol; col0 += gridDim.x * 2 * C) {
   const int col = col0 + grp;
+  if (REDO && !__any_sync(FULL, status[col] == VI_REDO)) continue;
   const int NeZ = op.NeZ, L = op.L;
   const ColLayout lay(N1, NeZ);
   unsigned char* base = smraw + (size_t)(wib * C + grp) * lay.stride;
@@ -1153,9 +1156,11 @@ __global__ void __launch_bounds__(64, 6) k_vi_cols(const Ops op, const OpsX ox, 
       atomicAdd(cnt + 2, (unsigned long long)nok);
     }
   }
+  if (!REDO) break;
+  }
 }
 
-template <int N1, bool PO>
+template <int N1, bool PO, bool REDO = false>
 int launch_n(const Ops& op, const OpsX& ox, const ProfX& px, const X5& qin, const F5c& z, const A3& a0,
              const float* const* guess,
              void* const* qsf, void* const* tout, float* gsc, int* status, unsigned long long* cnt,
@@ -1165,12 +1170,18 @@ int launch_n(const Ops& op, const OpsX& ox, const ProfX& px, const X5& qin, cons
   const size_t smem = (size_t)lay.stride * 2 * C;
   if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
   const int ncol = op.NeX * op.NeY * N1 * N1;
-  auto kfn = k_vi_cols<N1, PO>;
+  auto kfn = k_vi_cols<N1, PO, REDO>;
   // the limit is raised to 227 KB, the same value from every caller: contexts of different column
   // heights launching from several host threads never lower it under one another's launch
   cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-  kfn<<<(ncol + 2 * C - 1) / (2 * C), 64, smem, s>>>(op, ox, px, qin, z, a0, guess, qsf, tout, gsc, status, cnt, a,
-                                                     ncol);
+  int grid = (ncol + 2 * C - 1) / (2 * C);
+  if (REDO) {  // hardly any column as a rule: one resident wave of blocks looks through the marks
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    grid = std::min(grid, 6 * nsm);
+  }
+  kfn<<<grid, 64, smem, s>>>(op, ox, px, qin, z, a0, guess, qsf, tout, gsc, status, cnt, a, ncol);
   return (int)cudaGetLastError();
 }
 
@@ -1180,7 +1191,10 @@ size_t vi_cols_scratch_floats(size_t nodes) { return (size_t)12 * nodes; }  // G
 
 int launch_vi_cols(int N1, const Ops& op, const OpsX& ox, const ProfX& px, const X5& qin, const F5c& z,
                    const A3& a0, const float* const* guess, void* const* qsf, void* const* tout, float* gsc, int* status,
-                   unsigned long long* cnt, const MixViArgs& a, bool pair_out, cudaStream_t s) {
+                   unsigned long long* cnt, const MixViArgs& a, bool pair_out, cudaStream_t s, bool redo) {
+  if (redo)
+    return N1 == 4 ? launch_n<4, true, true>(op, ox, px, qin, z, a0, guess, qsf, tout, gsc, status, cnt, a, s)
+                   : launch_n<8, true, true>(op, ox, px, qin, z, a0, guess, qsf, tout, gsc, status, cnt, a, s);
   switch (N1 * 2 + (pair_out ? 1 : 0)) {
     case 8: return launch_n<4, false>(op, ox, px, qin, z, a0, guess, qsf, tout, gsc, status, cnt, a, s);
     case 9: return launch_n<4, true>(op, ox, px, qin, z, a0, guess, qsf, tout, gsc, status, cnt, a, s);

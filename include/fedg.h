@@ -175,15 +175,18 @@ int fedg_update(fedg_ctx* ctx, double* const q[5], int nsteps, const fedg_update
 int fedg_update_host(fedg_ctx* ctx, double* const host_q[5], int nsteps, const fedg_update_opts* opts,
                      double* iters_out);
 
-/* Newton corrections of the FEDG_PREC_MIXED / FEDG_PREC_PAIR column solve.  Every column's first
- * correction solves the FP32 Jacobian by block-Thomas and element LU, like FElib's solve
- * (hevi_common_2.F90:329-479).  Later corrections, which only refine that FP32 solution, use a
- * truncated Neumann series of the same Jacobian J = I + K: delta = (I - K + K^2 - ...) b with nterm
- * products K v (default 2), as long as each one cuts the certifying residual fourfold; a column
- * whose residual does not contract (large vertical Courant numbers, where ||K|| is not small) goes
- * back to LU corrections.  The converged state is the same: convergence is judged by the
- * float-pair residual to tol either way.  nterm = 0: LU corrections only.  No counterpart in
- * FElib, whose solve is a single LU correction. */
+/* Newton corrections of the FEDG_PREC_MIXED / FEDG_PREC_PAIR column solve.
+ * FEDG_PREC_PAIR from var0 (no learned iterate), nterm > 0: each correction J delta = b, J = I + K, is
+ * solved by the fixed point x <- (1 - w) x + w (b - K x) to FP32 accuracy; columns where it does not
+ * contract (large vertical Courant numbers, where ||K|| is not small) are solved as below instead.
+ * FEDG_PREC_MIXED, the learned iterate and those columns: every column's first correction solves the
+ * FP32 Jacobian by block-Thomas and element LU, like FElib's solve (hevi_common_2.F90:329-479).  Later
+ * corrections, which only refine that FP32 solution, use a truncated Neumann series of the same
+ * Jacobian, delta = (I - K + K^2 - ...) b with nterm products K v (default 2), as long as each one cuts
+ * the certifying residual fourfold; a column whose residual does not contract goes back to LU
+ * corrections.  The converged state is the same: convergence is judged by the float-pair residual to
+ * tol either way.  nterm = 0: LU corrections only.  No counterpart in FElib, whose solve is a single LU
+ * correction. */
 int fedg_update_set_vi_neumann(fedg_ctx* ctx, int nterm);
 
 /* Bounded waits of the update path's tensor-core contractions (the FEDG_PREC_MIXED stage kernels):
