@@ -304,7 +304,7 @@ int fedg_ctx_create(const fedg_mesh_desc* d, fedg_ctx** out) {
   op.N1 = c->N1; op.Np = c->Np; op.L = c->L;
   cudaError_t e;
   if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
-      (e = cudaMalloc(&c->d_prof, sizeof(double) * 4 * c->L)) != cudaSuccess ||
+      (e = cudaMalloc(&c->d_prof, sizeof(double) * 5 * c->L)) != cudaSuccess ||
       (e = cudaMalloc(&c->d_status, sizeof(int) * c->ncol)) != cudaSuccess ||
       (e = cudaMalloc(&c->d_cnt, sizeof(unsigned long long) * 4)) != cudaSuccess ||
       (e = cudaMallocHost(&c->h_cnt, sizeof(unsigned long long) * 4)) != cudaSuccess) {
@@ -378,7 +378,7 @@ int fedg_set_base_state(fedg_ctx* c, const double* DENS_hyd, const double* PRES_
   }
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(c->h_cnt, c->d_cnt, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-  std::vector<double> hp(2 * L);
+  std::vector<double> hp(3 * L);
   CK(cudaMemcpyAsync(hp.data(), c->d_prof + L, sizeof(double) * L, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   if (c->h_cnt[0] != 0)
@@ -386,7 +386,8 @@ int fedg_set_base_state(fedg_ctx* c, const double* DENS_hyd, const double* PRES_
                 "CORIOLIS (" + std::to_string(c->h_cnt[0]) + " mismatching entries)");
   for (int l = 0; l < L; ++l)  // RHOT_hyd recomputed from PRES_hyd as cal_vi does (hevi_common_2.F90:236-237)
     hp[L + l] = c->op.pres00 / c->op.rdry * std::pow(hp[l] / c->op.pres00, c->op.rgamm);
-  CK(cudaMemcpyAsync(c->d_prof + 3 * L, hp.data() + L, sizeof(double) * L, cudaMemcpyHostToDevice, c->stream));
+  for (int l = 0; l < L; ++l) hp[2 * L + l] = 1.0 / hp[L + l];
+  CK(cudaMemcpyAsync(c->d_prof + 3 * L, hp.data() + L, sizeof(double) * 2 * L, cudaMemcpyHostToDevice, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   c->op.coriolis_f = f;
   c->base_set = true;
@@ -405,7 +406,7 @@ int fedg_drhot2pres(fedg_ctx* c, const double* DRHOT, double* PRES, double* DPRE
   return 0;
 }
 
-// the FP64 column solve's block-Thomas scratch (sized by its launch plan for this mesh)
+// the FP64 column solves' scratch (sized by their launch plans for this mesh)
 static double* vi_scratch(fedg_ctx* c, size_t* ndouble) {
   const size_t need = vi_fp64_scratch_doubles(c->op);
   *ndouble = need;
@@ -486,16 +487,14 @@ int fedg_cal_vi(fedg_ctx* c, const double* const in[12], double impl_fac, double
   }
   F5c q{{in[0], in[1], in[2], in[3], in[4]}};
   F5c z{{in[7], in[8], in[9], in[10], in[11]}};
-  F5c none{{nullptr, nullptr, nullptr, nullptr, nullptr}};
   F5 t{{out[0], out[1], out[2], out[3], out[4]}};
-  F5 qo{{nullptr, nullptr, nullptr, nullptr, nullptr}};
   ViArgs a{impl_fac, dt, tol, max_iter, 340.0};
   int* st = col_status ? col_status : c->d_status;
   size_t ngsc = 0;
   double* gsc = vi_scratch(c, &ngsc);
   if (!gsc) return fail(ngsc ? "fedg_cal_vi: out of device memory" : "fedg_cal_vi: the column does not fit in shared memory");
   CK((cudaError_t)tracked(c, FEDG_K_VI, [&] {
-    return launch_vi_fp64(c->op, c->prof(), q, z, none, qo, t, st, a, gsc, ngsc, c->stream);
+    return launch_vi_fp64(c->op, c->prof(), q, z, t, st, a, gsc, ngsc, c->stream);
   }));
   if (st != c->d_status) CK(cudaMemcpyAsync(c->d_status, st, sizeof(int) * c->ncol, cudaMemcpyDeviceToDevice, c->stream));
   return count_status(c, nullptr, nullptr);
@@ -687,14 +686,12 @@ static int update_impl(fedg_ctx* c, double* const q[5], int nsteps, const fedg_u
         const double fac = fedg_tint_implicit_diagfac(t, s);
         F5c qc{{q[0], q[1], q[2], q[3], q[4]}};
         F5c z{{t->var0(0), t->var0(1), t->var0(2), t->var0(3), t->var0(4)}};
-        F5c none{{nullptr, nullptr, nullptr, nullptr, nullptr}};
         F5 tim{{t->tim(s - 1, 0), t->tim(s - 1, 1), t->tim(s - 1, 2), t->tim(s - 1, 3), t->tim(s - 1, 4)}};
-        F5 qo{{nullptr, nullptr, nullptr, nullptr, nullptr}};
         // stage 1: var0 is the state itself (StoreImplicit copies it at stage 1)
         if (s == 1) z = qc;
         ViArgs a{fac, o->dt, o->tol, o->max_iter, 340.0};
         r = tracked(c, FEDG_K_VI, [&] {
-          return launch_vi_fp64(c->op, c->prof(), qc, z, none, qo, tim, c->d_status, a, gsc, ngsc, c->stream);
+          return launch_vi_fp64(c->op, c->prof(), qc, z, tim, c->d_status, a, gsc, ngsc, c->stream);
         });
         if (r) return cuda_fail((cudaError_t)r, "fedg_update: cal_vi");
         if (fac != 0.0) {

@@ -52,6 +52,7 @@ struct Prof {
   const double* pres;   // PRES_hyd
   const double* therm;  // THERM_hyd (cal_tend_ex)
   const double* rhyd;   // P00/Rd (PRES_hyd/P00)^(cv/cp) (cal_vi recomputes it, hevi_common_2.F90:236-237)
+  const double* rhinv;  // 1/rhyd
 };
 
 __host__ __device__ inline int face_opp(int f) { return f ^ ((f < 4) ? 2 : 1); }

@@ -21,7 +21,7 @@ struct fedg_ctx {
   int N1, Np, Ne, L, ncol;
   size_t nxy, n;  // n = Np*Ne
   cudaStream_t stream = nullptr;
-  double* d_prof = nullptr;  // [4][L]: dens, pres, therm, rhyd
+  double* d_prof = nullptr;  // [5][L]: dens, pres, therm, rhyd, 1/rhyd
   bool base_set = false;
   const void* base_ptr[10] = {};
   int* d_status = nullptr;
@@ -30,7 +30,7 @@ struct fedg_ctx {
   // fused-update scratch
   double* work = nullptr;
   size_t work_doubles = 0;
-  double* vi_gsc = nullptr;  // block-Thomas scratch of the FP64 column solve
+  double* vi_gsc = nullptr;  // scratch of the FP64 column solves
   size_t vi_gsc_doubles = 0;
   MixedState* mixed = nullptr;
   fedg_tint* upd_tint = nullptr;  // RK buffers of fedg_update, kept between calls
@@ -68,7 +68,7 @@ struct fedg_ctx {
   long long nlaunch[FEDG_K_COUNT] = {};
   struct Rec { int id; cudaEvent_t a, b; };
   std::vector<Rec> recs;
-  Prof prof() const { return Prof{d_prof, d_prof + L, d_prof + 2 * L, d_prof + 3 * L}; }
+  Prof prof() const { return Prof{d_prof, d_prof + L, d_prof + 2 * L, d_prof + 3 * L, d_prof + 4 * L}; }
 };
 
 namespace fedg {

@@ -26,13 +26,18 @@ int launch_drhot2pres(const Ops& op, const Prof& pf, const double* drhot, double
                       cudaStream_t s);
 
 // Vertical-implicit column solve (cal_vi).  qin: stage input q*, z: guess/var0 (also the
-// state alph is frozen at).  qout (may be NULL): new state; tout (may be NULL): tendency
-// (qout - qin)/impl_fac, or A(z) when impl_fac == 0.  status[ncol]: solves used, -1 not
-// converged, -2 non-finite.  guess (may be NULL): initial Newton iterate of the var3 part
-// (DDENS, MOMZ, DRHOT), overriding z for the iterate but not for alph.  gsc: block-Thomas scratch of
-// at least vi_fp64_scratch_doubles(op) doubles (0 when the column does not fit in shared memory).
+// state alph is frozen at).  tout: tendency (Q - q*)/impl_fac, or A(z) when impl_fac == 0.
+// status[ncol]: solves used, -1 not converged, -2 non-finite.  gsc: scratch of at least
+// vi_fp64_scratch_doubles(op) doubles (0 when the column does not fit in shared memory).
 size_t vi_fp64_scratch_doubles(const Ops& op);
-int launch_vi_fp64(const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, const F5c& guess, const F5& qout,
-                   const F5& tout, int* status, const ViArgs& a, double* gsc, size_t gsc_doubles, cudaStream_t s);
+int launch_vi_fp64(const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, const F5& tout, int* status,
+                   const ViArgs& a, double* gsc, size_t gsc_doubles, cudaStream_t s);
+
+// Its first pass, by iterative refinement (fedg_vi64.cu): columns it leaves get status VI_REDO and are
+// solved by block LU.  Returns -1 if the columns are too tall for its shared memory (nothing launched).
+constexpr int VI_REDO = -100;
+size_t vi64_scratch_doubles(const Ops& op);
+int launch_vi64(const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, const F5& tout, int* status, const ViArgs& a,
+                double* gsc, size_t gsc_doubles, cudaStream_t s);
 
 }  // namespace fedg

@@ -423,8 +423,8 @@ __host__ __device__ inline int vi_col_doubles(int N1, int L, int NeZ) {
 
 template <int N1>
 __global__ void __launch_bounds__(128) k_vi_fp64(const Ops op, const Prof pf, const F5c qin, const F5c z,
-                                                  const F5c guess, const F5 qout, const F5 tout, int* status,
-                                                  const ViArgs args, int ncol, int per_col, double* gsc) {
+                                                  const F5 tout, int* status, const ViArgs args, int ncol,
+                                                  int per_col, double* gsc, bool redo) {
   constexpr int N = N1 - 1, n3 = 3 * N1, NF = N1 * N1, Np = N1 * N1 * N1;
   extern __shared__ double sm[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, h = lane >> 4, hl = lane & 15;
@@ -448,14 +448,16 @@ __global__ void __launch_bounds__(128) k_vi_fp64(const Ops op, const Prof pf, co
     const int col_h = 2 * pair + h;
     const bool live = col_h < ncol;  // an odd column count leaves the last half-warp a copy to idle on
     const int col = live ? col_h : ncol - 1;
+    // redo: only the columns that the refinement kernel marked (a warp's two are marked together)
+    if (redo && !__any_sync(0xffffffffu, status[col] == VI_REDO)) continue;
     const int ij = col % NF, exy = col / NF;
     c.gxy = (size_t)exy * Np + ij % N1 + N1 * (ij / N1);
 
-    // --- the iterate (guess or var0), and alph from var0 (eval_Ax_uv :1149-1155) ---
+    // --- the iterate (var0), and alph from var0 (eval_Ax_uv :1149-1155) ---
     for (int l = hl; l < L; l += 16) {
       const size_t g = c.g(l);
 #pragma unroll
-      for (int m = 0; m < 3; ++m) c.P[3 * l + m] = guess.v[0] ? __ldg(guess.v[gv[m]] + g) : __ldg(z.v[gv[m]] + g);
+      for (int m = 0; m < 3; ++m) c.P[3 * l + m] = __ldg(z.v[gv[m]] + g);
       // sound speed + |w| of var0 -> fr (temporary)
       const double rdens0 = 1.0 / (__ldg(pf.dens + l) + __ldg(z.v[VD] + g));
       const double wt0 = __ldg(z.v[VMZ] + g) * rdens0;
@@ -490,11 +492,10 @@ __global__ void __launch_bounds__(128) k_vi_fp64(const Ops op, const Prof pf, co
           const double dBy = tm * c.alB[ez] * (Pu[2 * lbP + 1] - Pu[2 * lb + 1]),
                        dTy = tm * c.alT[ez] * (Pu[2 * ltP + 1] - Pu[2 * lt + 1]);
           const size_t g = c.g(l);
-          if (live && tout.v[0]) {
+          if (live) {
             tout.v[VMX][g] = -(op.Lb[pv] * dBx + op.Lt[pv] * dTx);
             tout.v[VMY][g] = -(op.Lb[pv] * dBy + op.Lt[pv] * dTy);
           }
-          if (live && qout.v[0]) { qout.v[VMX][g] = __ldg(qin.v[VMX] + g); qout.v[VMY][g] = __ldg(qin.v[VMY] + g); }
         }
       } else {
         // The element blocks are the identity plus the Lift face terms in columns 0 and N, coupled to
@@ -555,11 +556,8 @@ __global__ void __launch_bounds__(128) k_vi_fp64(const Ops op, const Prof pf, co
           for (int l = hl; l < L; l += 16) {
             const double px = Pu[2 * l] + bu[2 * l], py = Pu[2 * l + 1] + bu[2 * l + 1];
             const size_t g = c.g(l);
-            if (qout.v[0]) { qout.v[VMX][g] = px; qout.v[VMY][g] = py; }
-            if (tout.v[0]) {
-              tout.v[VMX][g] = (px - __ldg(qin.v[VMX] + g)) / impl_fac;
-              tout.v[VMY][g] = (py - __ldg(qin.v[VMY] + g)) / impl_fac;
-            }
+            tout.v[VMX][g] = (px - __ldg(qin.v[VMX] + g)) / impl_fac;
+            tout.v[VMY][g] = (py - __ldg(qin.v[VMY] + g)) / impl_fac;
           }
         }
       }
@@ -574,10 +572,7 @@ __global__ void __launch_bounds__(128) k_vi_fp64(const Ops op, const Prof pf, co
         for (int l = hl; l < L; l += 16) {
           const size_t g = c.g(l);
 #pragma unroll
-          for (int m = 0; m < 3; ++m) {
-            if (tout.v[0]) tout.v[gv[m]][g] = c.bh[3 * l + m];
-            if (qout.v[0]) qout.v[gv[m]][g] = __ldg(qin.v[gv[m]] + g);
-          }
+          for (int m = 0; m < 3; ++m) tout.v[gv[m]][g] = c.bh[3 * l + m];
         }
       }
     } else {
@@ -602,11 +597,7 @@ __global__ void __launch_bounds__(128) k_vi_fp64(const Ops op, const Prof pf, co
         for (int l = hl; l < L; l += 16) {
           const size_t g = c.g(l);
 #pragma unroll
-          for (int m = 0; m < 3; ++m) {
-            const double pnew = c.P[3 * l + m];
-            if (qout.v[0]) qout.v[gv[m]][g] = pnew;
-            if (tout.v[0]) tout.v[gv[m]][g] = (pnew - __ldg(qin.v[gv[m]] + g)) / impl_fac;
-          }
+          for (int m = 0; m < 3; ++m) tout.v[gv[m]][g] = (c.P[3 * l + m] - __ldg(qin.v[gv[m]] + g)) / impl_fac;
         }
       }
     }
@@ -666,33 +657,38 @@ int plan_vi(const Ops& op, ViPlan& p) {
 }
 
 template <int N1>
-int launch_vi_n(const ViPlan& p, const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, const F5c& guess,
-                const F5& qout, const F5& tout, int* status, const ViArgs& a, double* gsc, cudaStream_t s) {
+int launch_vi_n(const ViPlan& p, const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, const F5& tout,
+                int* status, const ViArgs& a, double* gsc, bool redo, cudaStream_t s) {
   const int ncol = op.NeX * op.NeY * N1 * N1;
   auto kfn = k_vi_fp64<N1>;
-  kfn<<<p.grid, 32 * p.wpb, p.smem, s>>>(op, pf, qin, z, guess, qout, tout, status, a, ncol, p.per_col, gsc);
+  kfn<<<p.grid, 32 * p.wpb, p.smem, s>>>(op, pf, qin, z, tout, status, a, ncol, p.per_col, gsc, redo);
   return (int)cudaGetLastError();
 }
 }  // namespace
 
 size_t vi_fp64_scratch_doubles(const Ops& op) {
   ViPlan p;
-  return plan_vi(op, p) ? 0 : p.scratch;
+  return plan_vi(op, p) ? 0 : std::max(p.scratch, vi64_scratch_doubles(op));
 }
 
-int launch_vi_fp64(const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, const F5c& guess, const F5& qout,
-                   const F5& tout, int* status, const ViArgs& a, double* gsc, size_t gsc_doubles, cudaStream_t s) {
+int launch_vi_fp64(const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, const F5& tout, int* status,
+                   const ViArgs& a, double* gsc, size_t gsc_doubles, cudaStream_t s) {
   ViPlan p;
   if (const int r = plan_vi(op, p)) return r;
   if (!gsc || gsc_doubles < p.scratch) return (int)cudaErrorInvalidValue;
+  // the refinement kernel first, then block LU for the columns it leaves (for all, if it was not launched)
+  const int first = launch_vi64(op, pf, qin, z, tout, status, a, gsc, gsc_doubles, s);
+  if (first > 0) return first;
+  if (first == 0 && a.impl_fac == 0.0) return 0;  // nothing to solve
+  const bool redo = first == 0;
   switch (op.N1) {
-    case 2: return launch_vi_n<2>(p, op, pf, qin, z, guess, qout, tout, status, a, gsc, s);
-    case 3: return launch_vi_n<3>(p, op, pf, qin, z, guess, qout, tout, status, a, gsc, s);
-    case 4: return launch_vi_n<4>(p, op, pf, qin, z, guess, qout, tout, status, a, gsc, s);
-    case 5: return launch_vi_n<5>(p, op, pf, qin, z, guess, qout, tout, status, a, gsc, s);
-    case 6: return launch_vi_n<6>(p, op, pf, qin, z, guess, qout, tout, status, a, gsc, s);
-    case 7: return launch_vi_n<7>(p, op, pf, qin, z, guess, qout, tout, status, a, gsc, s);
-    case 8: return launch_vi_n<8>(p, op, pf, qin, z, guess, qout, tout, status, a, gsc, s);
+    case 2: return launch_vi_n<2>(p, op, pf, qin, z, tout, status, a, gsc, redo, s);
+    case 3: return launch_vi_n<3>(p, op, pf, qin, z, tout, status, a, gsc, redo, s);
+    case 4: return launch_vi_n<4>(p, op, pf, qin, z, tout, status, a, gsc, redo, s);
+    case 5: return launch_vi_n<5>(p, op, pf, qin, z, tout, status, a, gsc, redo, s);
+    case 6: return launch_vi_n<6>(p, op, pf, qin, z, tout, status, a, gsc, redo, s);
+    case 7: return launch_vi_n<7>(p, op, pf, qin, z, tout, status, a, gsc, redo, s);
+    case 8: return launch_vi_n<8>(p, op, pf, qin, z, tout, status, a, gsc, redo, s);
   }
   return (int)cudaErrorInvalidValue;
 }

@@ -36,11 +36,10 @@
 #include "fedg_ctx.cuh"
 #include "fedg_mixed.cuh"
 #include "fedg_p2.cuh"
+#include "fedg_sweep.cuh"
 
 namespace fedg {
 namespace {
-
-constexpr unsigned FULL = 0xffffffffu;
 
 // shared memory of one column pair (bytes): two vectors [3][L], x and b (the residual adds x to the
 // iterate, writes the new b over it and uses the old b's space for its ring of level quantities, then
@@ -106,126 +105,12 @@ __device__ __forceinline__ float grp_max_nan(float e, int width) {
   }
   return e;
 }
-__device__ __forceinline__ float warp_max_bits(float e) {  // e >= 0 or NaN (which wins)
-  return __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(e) & 0x7fffffffu));
-}
-
 template <int N1>
-struct Pair {
-  u64x* X;   // x [3][L]
-  u64x* B;   // b [3][L]
-  unsigned char* E;
-  u64x* A;   // wave speed of face e (0 .. NeZ)
-  p2m* P;    // iterate: planes of the three variables
-  u64x* J;   // pot, wt, dpd planes
-  size_t pn, pb, ps;  // plane size; entry of element 0; stride of one element
-  size_t gb, gs;      // node index of the first column's node (0, 0) and the element-layer stride
-  int k, NeZ, L;
-  __device__ size_t pi(int v, int e) const { return (size_t)v * pn + pb + (size_t)e * ps; }
+struct Pair : SweepCtx<N1, N1> {
+  p2m* P;         // iterate: planes of the three variables, indexed like J
+  size_t gb, gs;  // node index of the first column's node (0, 0) and the element-layer stride
   __device__ size_t g(int e, int k) const { return gb + (size_t)e * gs + (size_t)(N1 * N1) * k; }
 };
-
-// One sweep x <- (1 - w) x + w (b - K x), from x = w b if first; returns the lane's largest weighted
-// change.  (A NaN can drop out of the change; the certifying residual looks at every node.)
-template <int N1>
-__device__ __forceinline__ float sweep(const Pair<N1>& c, const u64x (&Dk)[N1], const u64x (&Tk)[N1],
-                                       u64x facB, u64x facT, u64x w, u64x w1, float c1, float c2, bool first) {
-  constexpr int N = N1 - 1;
-  constexpr u64x SG = 0x8000000080000000ull;
-  const int L = c.L, NeZ = c.NeZ;
-  constexpr int SLOT = 32 * N1 + 16;
-  u64x xn[3], jn[3];  // x and the Jacobian quantities of the element ahead
-  auto load = [&](int e) {
-#pragma unroll
-    for (int v = 0; v < 3; ++v) jn[v] = c.J[c.pi(v, e)];
-  };
-  auto put = [&](int e) {  // quantities of element e into its slot
-    unsigned char* s = c.E + (e & 1) * SLOT;
-    const int k = c.k, l = e * N1 + k;
-#pragma unroll
-    for (int v = 0; v < 3; ++v) xn[v] = first ? xmul(w, c.B[v * L + l]) : c.X[v * L + l];
-    const u64x p = xmul(jn[2], xn[2]);
-    const u64x t = xfma(jn[0], xfma(jn[1], xn[0] ^ SG, xn[1]), xmul(jn[1], xn[2]));
-    ulonglong2* q = reinterpret_cast<ulonglong2*>(s + 32 * k);
-    q[0] = make_ulonglong2(xn[0], xn[1]);
-    q[1] = make_ulonglong2(p, t);
-    if (c.k == 0) *reinterpret_cast<u64x*>(s + 32 * N1) = xn[2];
-    if (c.k == N1 - 1) *reinterpret_cast<u64x*>(s + 32 * N1 + 8) = xn[2];
-  };
-  load(0);
-  put(0);
-  if (NeZ > 1) load(1);
-  u64x pr = 0, pm = 0, pp = 0, pt = 0, ph = 0;  // node N of the element below
-  float dmax = 0.f;
-  for (int e = 0; e < NeZ; ++e) {
-    u64x xo[3], be[3];  // this element's x and b
-#pragma unroll
-    for (int v = 0; v < 3; ++v) {
-      xo[v] = xn[v];
-      be[v] = c.B[v * L + e * N1 + c.k];
-    }
-    if (e + 1 < NeZ) {
-      put(e + 1);
-      if (e + 2 < NeZ) load(e + 2);
-    }
-    __syncwarp();
-    const unsigned char* s = c.E + (e & 1) * SLOT;
-    u64x y0 = 0, y1 = 0, y2 = 0, z1 = 0;
-    u64x r0, m0, p0, t0, rN, mN, pN, tN;
-#pragma unroll
-    for (int m = 0; m < N1; ++m) {
-      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(s + 32 * m);
-      const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(s + 32 * m + 16);
-      y0 = xfma(Dk[m], a.y, y0);
-      z1 = xfma(Tk[m], a.x, z1);
-      y1 = xfma(Dk[m], b.x, y1);
-      y2 = xfma(Dk[m], b.y, y2);
-      if (m == 0) { r0 = a.x; m0 = a.y; p0 = b.x; t0 = b.y; }
-      if (m == N) { rN = a.x; mN = a.y; pN = b.x; tN = b.y; }
-    }
-    const u64x h0 = *reinterpret_cast<const u64x*>(s + 32 * N1), hN = *reinterpret_cast<const u64x*>(s + 32 * N1 + 8);
-    {  // bottom face (nz = -1); a slip lid reflects MOMZ and the heat flux
-      u64x dr = xsub(r0, pr), dm = xsub(m0, pm), dp = xsub(p0, pp), dt = xsub(t0, pt), dh = xsub(h0, ph);
-      if (e == 0) { dr = dp = dh = 0; dm = xadd(m0, m0); dt = xadd(t0, t0); }
-      const u64x al = c.A[e], f0 = xfma(al, dr, dm), f1 = xfma(al, dm, dp), f2 = xfma(al, dh, dt);
-      y0 = xfma(facB, f0, y0);
-      y1 = xfma(facB, f1, y1);
-      y2 = xfma(facB, f2, y2);
-    }
-    {  // top face (nz = +1)
-      u64x dr, dm, dp, dt, dh;
-      if (e + 1 < NeZ) {
-        const unsigned char* sn = c.E + ((e + 1) & 1) * SLOT;
-        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(sn);
-        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(sn + 16);
-        const u64x hn = *reinterpret_cast<const u64x*>(sn + 32 * N1);
-        dr = xsub(rN, a.x); dm = xsub(a.y, mN); dp = xsub(b.x, pN); dt = xsub(b.y, tN); dh = xsub(hN, hn);
-      } else {
-        dr = dp = dh = 0;
-        dm = xadd(mN, mN) ^ SG;
-        dt = xadd(tN, tN) ^ SG;
-      }
-      const u64x al = c.A[e + 1], f0 = xfma(al, dr, dm), f1 = xfma(al, dm ^ SG, dp), f2 = xfma(al, dh, dt);
-      y0 = xfma(facT, f0, y0);
-      y1 = xfma(facT, f1, y1);
-      y2 = xfma(facT, f2, y2);
-    }
-    pr = rN; pm = mN; pp = pN; pt = tN; ph = hN;
-    const int l = e * N1 + c.k;
-    const u64x nr = xfma(w, xsub(be[0], y0), xmul(w1, xo[0]));
-    const u64x nm = xfma(w, xsub(be[1], xadd(y1, z1)), xmul(w1, xo[1]));
-    const u64x nh = xfma(w, xsub(be[2], y2), xmul(w1, xo[2]));
-    c.X[l] = nr;
-    c.X[L + l] = nm;
-    c.X[2 * L + l] = nh;
-    const float2 a = unpk(xsub(nr, xo[0])), b = unpk(xsub(nm, xo[1])), d = unpk(xsub(nh, xo[2]));
-    const float ma = fmaxf(fmaxf(fabsf(a.x), c1 * fabsf(b.x)), c2 * fabsf(d.x));
-    const float mb = fmaxf(fmaxf(fabsf(a.y), c1 * fabsf(b.y)), c2 * fabsf(d.y));
-    dmax = fmaxf(dmax, fmaxf(ma, mb));
-    __syncwarp();
-  }
-  return dmax;
-}
 
 // The certifying residual b = impl_fac A(P) + q* - P in float pairs (col_residual of fedg_vicol.cu) of
 // P + x, which becomes the iterate; b goes over x and the two vectors change places.  errA, errB: the two
@@ -400,7 +285,7 @@ __global__ void __launch_bounds__(64, N1 == 8 ? 6 : 4)
   c.B = reinterpret_cast<u64x*>(base + lay.oB);
   c.E = base + lay.oE;
   c.A = reinterpret_cast<u64x*>(base + lay.oA);
-  c.k = k; c.NeZ = NeZ; c.L = L;
+  c.k = k; c.act = true; c.NeZ = NeZ; c.L = L;
   c.pn = (size_t)ncp * L;
   c.P = reinterpret_cast<p2m*>(gsc);
   c.J = reinterpret_cast<u64x*>(gsc + 12 * c.pn);
@@ -505,42 +390,13 @@ __global__ void __launch_bounds__(64, N1 == 8 ? 6 : 4)
   int nsolve = 0, stA = 0, stB = 0;
   bool give_up = false, emitted = false;
   {
-    const float fi = (float)va.impl_fac;
-    const float fdzs = (float)op.E33 * fi;
-    // relaxation: the face dissipation's diagonal entry with the wave speed of the lowest face
-    const float2 a0f = unpk(c.A[0]);
-    const float ds = 0.5f * fi * (float)op.Lb[0] * (float)op.FSz * fmaxf(a0f.x, a0f.y);
-    const float wr = __shfl_sync(FULL, 1.f / (1.f + ds), 0);
-    const u64x w = pk1(wr), w1 = pk1(1.f - wr);
+    const SweepCoef<N1> sc(op, va.impl_fac, k, c.A[0]);
     const float ctol = 0.02f * (float)va.tol * args.dmin;
     while (true) {
-      // sweeps from x = w b until the change that the next one would make (the last change times the
-      // observed contraction) is small against the first one, which FP32 resolves to 1e-7, or against
-      // the tolerance (2 % of it, so that what is accepted lies well inside, as after the LU kernel's
-      // corrections); a later correction goes on from the pair residual.  A contraction above 0.4 is
-      // left to the LU kernel, unless it is FP32's floor
-      const float d0 = wr * warp_max_bits(bmax);
-      const float stop = fmaxf(2.0e-6f * d0, ctol);
-      float prev = d0;
-      bool ok = false;
-      {
-        u64x Dk[N1], Tk[N1], facB, facT;
-        const int k = c.k;
-#pragma unroll
-        for (int m = 0; m < N1; ++m) {
-          Dk[m] = pk1(fdzs * (float)op.D[k * N1 + m]);
-          Tk[m] = pk1(fi * (float)op.grav * (float)op.T[k * N1 + m]);
-        }
-        facB = pk1(0.5f * fi * (float)op.Lb[k] * (float)op.FSz);
-        facT = pk1(0.5f * fi * (float)op.Lt[k] * (float)op.FSz);
-        for (int n = 0; n < 24; ++n) {
-          const float d = warp_max_bits(sweep<N1>(c, Dk, Tk, facB, facT, w, w1, args.c1, args.c2, n == 0));
-          const float r = __fdividef(d, prev);
-          if (d * r <= stop || (!(r <= 0.4f) && d <= 1.0e-4f * d0)) { ok = true; break; }
-          if (!(r <= 0.4f) && n >= 2) break;
-          prev = d;
-        }
-      }
+      // to 2e-6 of the first change, which FP32 resolves to 1e-7 (a later correction goes on from the pair
+      // residual), or 2 % of the tolerance, so that what is accepted lies well inside, as after the LU
+      // kernel's corrections
+      const bool ok = sweeps<N1, N1>(c, sc, op, va.impl_fac, warp_max_bits(bmax), 2.0e-6f, ctol, args.c1, args.c2);
       if (!ok) { give_up = true; break; }
       ++nsolve;
       __syncwarp();
