@@ -1,5 +1,4 @@
-// fedg_sweep.cuh -- the fixed-point sweeps of the series column solves (fedg_viseries.cu in float pairs,
-// fedg_vi64.cu in FP64): FP32 solutions of J x = b, J = I + K the Jacobian of the DENS/MOMZ/RHOT system, for
+// fedg_sweep.cuh -- the fixed-point sweeps of the FP64 column solve (fedg_vi64.cu): FP32 solutions of J x = b, J = I + K the Jacobian of the DENS/MOMZ/RHOT system, for
 // two columns per lane in packed arithmetic.
 //
 // x <- (1 - w) x + w (b - K x) with w = 1 / (1 + d), d the face dissipation's diagonal entry: K's spectrum
