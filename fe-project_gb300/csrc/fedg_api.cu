@@ -253,14 +253,14 @@ __global__ void k_rk(RKPtrs P, int kind, int stage, int nst, RKC c, size_t n, in
     } else {  // low storage: c0 = sig_ss, c1 = gam_ss, c2 = sig_Ns, c3 = gam_Ns, c4 = final flag, c5 = use Ns
       const double t = P.tex[0][v][g];
       if (c.c[4] != 0.0) {
-        P.q[v][g] = P.vtmp[v][g] + c.c[0] * q + c.c[1] * t;
+        P.q[v][g] = rk_low(1.0, P.vtmp[v][g], c.c[0], q, c.c[1], t);
       } else {
         if (first_stage) {
           P.var0[v][g] = q;
           P.vtmp[v][g] = 0.0;
         }
-        if (c.c[5] != 0.0) P.vtmp[v][g] = P.vtmp[v][g] + c.c[2] * q + c.c[3] * t;
-        P.q[v][g] = (1.0 - c.c[0]) * P.var0[v][g] + c.c[0] * q + c.c[1] * t;
+        if (c.c[5] != 0.0) P.vtmp[v][g] = rk_low(1.0, P.vtmp[v][g], c.c[2], q, c.c[3], t);
+        P.q[v][g] = rk_low(1.0 - c.c[0], P.var0[v][g], c.c[0], q, c.c[1], t);
       }
     }
   }
@@ -300,11 +300,14 @@ int fedg_ctx_create(const fedg_mesh_desc* d, fedg_ctx** out) {
   op.grav = d->grav; op.rdry = d->rdry; op.cpdry = d->cpdry; op.cvdry = d->cvdry; op.pres00 = d->pres00;
   op.kap = d->cpdry / d->cvdry;
   op.rgamm = d->cvdry / d->cpdry;
+  double bn = 1.0;
+  for (int m = 0; m < 13; ++m) op.pb[m] = bn *= (op.kap - m) / (m + 1);
+  op.pb_on = op.kap >= 1.0 && op.kap <= 2.0;
   op.NeX = d->NeX; op.NeY = d->NeY; op.NeZ = d->NeZ;
   op.N1 = c->N1; op.Np = c->Np; op.L = c->L;
   cudaError_t e;
   if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
-      (e = cudaMalloc(&c->d_prof, sizeof(double) * 5 * c->L)) != cudaSuccess ||
+      (e = cudaMalloc(&c->d_prof, sizeof(double) * 8 * c->L)) != cudaSuccess ||
       (e = cudaMalloc(&c->d_status, sizeof(int) * c->ncol)) != cudaSuccess ||
       (e = cudaMalloc(&c->d_cnt, sizeof(unsigned long long) * 4)) != cudaSuccess ||
       (e = cudaMallocHost(&c->h_cnt, sizeof(unsigned long long) * 4)) != cudaSuccess) {
@@ -378,16 +381,23 @@ int fedg_set_base_state(fedg_ctx* c, const double* DENS_hyd, const double* PRES_
   }
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(c->h_cnt, c->d_cnt, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-  std::vector<double> hp(3 * L);
-  CK(cudaMemcpyAsync(hp.data(), c->d_prof + L, sizeof(double) * L, cudaMemcpyDeviceToHost, c->stream));
+  std::vector<double> hp(8 * L);  // the arrays of Prof; the first three are the caller's
+  CK(cudaMemcpyAsync(hp.data(), c->d_prof, sizeof(double) * 3 * L, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   if (c->h_cnt[0] != 0)
     return fail("fedg_set_base_state: base state is not horizontally homogeneous dry air with DPhyd = 0 and constant "
                 "CORIOLIS (" + std::to_string(c->h_cnt[0]) + " mismatching entries)");
-  for (int l = 0; l < L; ++l)  // RHOT_hyd recomputed from PRES_hyd as cal_vi does (hevi_common_2.F90:236-237)
-    hp[L + l] = c->op.pres00 / c->op.rdry * std::pow(hp[l] / c->op.pres00, c->op.rgamm);
-  for (int l = 0; l < L; ++l) hp[2 * L + l] = 1.0 / hp[L + l];
-  CK(cudaMemcpyAsync(c->d_prof + 3 * L, hp.data() + L, sizeof(double) * 2 * L, cudaMemcpyHostToDevice, c->stream));
+  const double p00 = c->op.pres00, rd = c->op.rdry;
+  for (int l = 0; l < L; ++l) {
+    const double pres = hp[L + l], therm = hp[2 * L + l];
+    // RHOT_hyd recomputed from PRES_hyd as cal_vi does (hevi_common_2.F90:236-237)
+    hp[3 * L + l] = p00 / rd * std::pow(pres / p00, c->op.rgamm);
+    hp[4 * L + l] = 1.0 / hp[3 * L + l];
+    hp[5 * L + l] = p00 * std::pow(rd / p00 * therm, c->op.kap);
+    hp[6 * L + l] = hp[5 * L + l] - pres;
+    hp[7 * L + l] = 1.0 / therm;
+  }
+  CK(cudaMemcpyAsync(c->d_prof + 3 * L, hp.data() + 3 * L, sizeof(double) * 5 * L, cudaMemcpyHostToDevice, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   c->op.coriolis_f = f;
   c->base_set = true;
@@ -677,6 +687,31 @@ static int update_impl(fedg_ctx* c, double* const q[5], int nsteps, const fedg_u
   int nfail = 0;
   double* const* tf = c->trc_flux;
   const size_t nb64 = sizeof(double) * c->n;
+  // HEVE with nothing between tendency and update (sponge, mass-flux sums, a halo exchange): a kernel per stage.
+  // q1 and q2 live in the RK object's var0 and varTmp, DPRES alternates between two buffers.
+  const bool fused = o->eqs == FEDG_HEVE && !tf[0] && !(c->sl_tau > 0.0) && !fedg::slab(c);
+  if (fused && nsteps > 0) {
+    double* dpb[2] = {dp, t->tex(0, 0)};
+    const F5 qb[3] = {{{q[0], q[1], q[2], q[3], q[4]}},
+                      {{t->var0(0), t->var0(1), t->var0(2), t->var0(3), t->var0(4)}},
+                      {{t->vtmp(0), t->vtmp(1), t->vtmp(2), t->vtmp(3), t->vtmp(4)}}};
+    auto cst = [](const F5& f) { return F5c{{f.v[0], f.v[1], f.v[2], f.v[3], f.v[4]}}; };
+    r = tracked(c, FEDG_K_PRES, [&] { return launch_drhot2pres(c->op, c->prof(), q[4], nullptr, dpb[0], c->n, c->stream); });
+    if (r) return cuda_fail((cudaError_t)r, "fedg_update: drhot2pres");
+    int cur = 0;
+    for (int st = 0; st < 3 * nsteps; ++st) {
+      const int s = st % 3 + 1;
+      const bool last = s == 3;
+      const SspArgs x{cst(qb[0]), qb[s % 3], st + 1 < 3 * nsteps ? dpb[cur ^ 1] : nullptr,
+                      last ? t->sig[3][0] : 1.0 - t->sig[s][s - 1], t->sig[s][s - 1], o->dt * t->gam[s][s - 1],
+                      last && c->d.mf_on};
+      r = tracked(c, FEDG_K_TEND, [&] { return launch_ssp_stage_fp64(c->op, c->prof(), cst(qb[s - 1]), dpb[cur], x, c->Ne, c->stream); });
+      if (r) return cuda_fail((cudaError_t)r, "fedg_update: SSP stage");
+      cur ^= 1;
+    }
+    if (iters_out) *iters_out = 0.0;
+    return 0;
+  }
   for (int step = 0; step < nsteps && r >= 0; ++step) {
     if (tf[0] && cudaMemcpyAsync(tf[6], q[0], nb64, cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess)
       return fail("fedg_update: DDENS0_TRC copy");

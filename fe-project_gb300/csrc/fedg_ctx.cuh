@@ -21,7 +21,7 @@ struct fedg_ctx {
   int N1, Np, Ne, L, ncol;
   size_t nxy, n;  // n = Np*Ne
   cudaStream_t stream = nullptr;
-  double* d_prof = nullptr;  // [5][L]: dens, pres, therm, rhyd, 1/rhyd
+  double* d_prof = nullptr;  // [8][L], the arrays of Prof
   bool base_set = false;
   const void* base_ptr[10] = {};
   int* d_status = nullptr;
@@ -68,7 +68,8 @@ struct fedg_ctx {
   long long nlaunch[FEDG_K_COUNT] = {};
   struct Rec { int id; cudaEvent_t a, b; };
   std::vector<Rec> recs;
-  Prof prof() const { return Prof{d_prof, d_prof + L, d_prof + 2 * L, d_prof + 3 * L, d_prof + 4 * L}; }
+  Prof prof() const { return Prof{d_prof, d_prof + L, d_prof + 2 * L, d_prof + 3 * L, d_prof + 4 * L, d_prof + 5 * L,
+                                 d_prof + 6 * L, d_prof + 7 * L}; }
 };
 
 namespace fedg {

@@ -74,7 +74,7 @@ __global__ void k_halo_pack_f64(const Ops op, const Prof pf, const HaloGeom hg, 
   } else {  // DRHOT -> DPRES as k_drhot2pres forms it
     const int N1 = hg.N1, NF = N1 * N1;
     const int lev = (int)((g / ((size_t)NF * N1)) / ((size_t)hg.NeX * hg.NeY)) * N1 + (int)(g % ((size_t)NF * N1)) / NF;
-    dp = dpres_of(op, __ldg(pf.therm + lev) + __ldg(q.v[4] + g), __ldg(pf.pres + lev));
+    dp = dpres_of(op, pf, lev, __ldg(q.v[4] + g));
   }
   o[5 * per + r] = dp;
 }

@@ -21,6 +21,17 @@ void lgl_nodes_1d(int N, double* x);
 
 int launch_tend_fp64(const Ops& op, const Prof& pf, const F5c& q, const double* dpres, const F5& t, int Ne,
                      int hevi, cudaStream_t s);
+// A whole SSP-RK3 stage of the HEVE equations: qn = A q0 + B q + C tend(q), the modal filter if `filter`, and
+// DPRES of qn into dpn unless NULL.  q0 may be qn's buffers; q and dpres, which neighbours read, may not.
+struct SspArgs {
+  F5c q0;
+  F5 qn;
+  double* dpn;
+  double A, B, C;
+  int filter;
+};
+int launch_ssp_stage_fp64(const Ops& op, const Prof& pf, const F5c& q, const double* dpres, const SspArgs& x, int Ne,
+                          cudaStream_t s);
 int launch_filter_fp64(const Ops& op, const F5& q, int Ne, cudaStream_t s);
 int launch_drhot2pres(const Ops& op, const Prof& pf, const double* drhot, double* pres, double* dpres, size_t n,
                       cudaStream_t s);
