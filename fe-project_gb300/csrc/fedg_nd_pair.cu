@@ -7,291 +7,343 @@
 // pair reciprocals.  The update adds the pair increment dt*tend to the FP64 field in FP64 (two
 // adds), so the field keeps all of its bits.
 // Why: the FP64 passes keep GB300's FP64 pipe ~87 % busy; the FP32 pipe issues 64x faster.
+//
+// Layout: one thread carries the same node of two consecutive elements in the packed pair arithmetic of
+// fedg_p2.cuh, so operator tables, indices along a line and the kernels of odd orders are shared by both.
+// An interior face's flux is nonzero only on one of its two sides (the gradient takes the lower neighbour,
+// the divergence the upper), so an element computes three faces, and a lid face only where the
+// reflection leaves a jump.  Coefficients and dt are multiplied into E on the host.
+//
+// A thread owns NPT = 2 nodes (k and k + N1/2) for even N1, which share the loads of the x and y tables; an
+// odd N1 has one.
+//
+// What bounds it: the latency of the loads and the barriers between them, the faces and the sums (FP32 pipe 40 %
+// busy with two blocks of 512 threads per SM), so the blocks are small and many.  Update of five fields, 32x32x16
+// elements, p = 7: six blocks of 256 threads per SM (40 registers) 1.59 ms, five 1.62; in an earlier form of the
+// sums six 1.51, four of 256 (64 registers) 1.78, three of 512 threads with one node each 1.97, eight of 128 with
+// four nodes each 1.77.  With one element and scalar pairs per thread, six faces and 512 threads it took 3.47 ms.
+// The neighbours' face values are loaded with the element's own.
 #include <cmath>
 #include <cstring>
 
 #include "fedg_ctx.cuh"
-#include "fedg_f2.cuh"
+#include "fedg_p2.cuh"
 
 namespace fedg {
 namespace {
 
-__device__ __forceinline__ f2 operator+(f2 a, f2 b) { return f2_add(a, b); }
-__device__ __forceinline__ f2 operator-(f2 a, f2 b) { return f2_sub(a, b); }
-__device__ __forceinline__ f2 operator*(f2 a, f2 b) { return f2_mul(a, b); }
-__device__ __forceinline__ f2 z2() { return f2{0.f, 0.f}; }
-__device__ __forceinline__ f2 ld64(const double* p, size_t g) { return f2_split(__ldg(p + g)); }
-__device__ __forceinline__ f2 ldp(const float2* p, size_t g) { return f2_of(__ldg(p + g)); }
-
+// operator tables, [l][i]: D(i, l); the Lift of the face an interior element takes its flux from (lf) and of the
+// opposite face, a lid (lo), with the face flux's sign; E of each direction, the pass's factor multiplied in
 struct NdOpsP {
   float2 D[FEDG_MAXN1 * FEDG_MAXN1];
-  float2 Lb[FEDG_MAXN1], Lt[FEDG_MAXN1];
-  float2 E[3], FS[3];  // E11, E22, E33; Fscale of x, y, z faces
+  float2 E[3], lf[FEDG_MAXN1], lo[FEDG_MAXN1];
   int NeX, NeY, NeZ;
 };
-
-__device__ __forceinline__ int face_dir_p(int f) { return f >= 4 ? 2 : ((f & 1) ? 0 : 1); }
-__device__ __forceinline__ float face_n_p(int f) { return (f == 1 || f == 2 || f == 5) ? 1.f : -1.f; }
-
-// lid exteriors (even: wall-normal momentum reflected; odd: normal gradient reflected except for the
-// wall-normal momentum); the normals are +-1, so the reflection is an exact sign change
-__device__ __forceinline__ f2 even_ext_p(int var, int dir, f2 vM) {
-  const bool refl = (var == VMX && dir == 0) || (var == VMY && dir == 1) || (var == VMZ && dir == 2);
-  return refl ? f2_neg(vM) : vM;
-}
-__device__ __forceinline__ f2 odd_ext_p(int var, int dir, f2 gM) {
-  const bool keep = (var == VMX && dir == 0) || (var == VMY && dir == 1) || (var == VMZ && dir == 2);
-  return keep ? gM : f2_neg(gM);
-}
-
 template <int N1>
-__device__ __forceinline__ void face_nodes_nd(const NdOpsP& op, int f, int a, int b, long ke, int ex, int ey, int ez,
-                                              int nxy, int& pM, size_t& gP, long& kn) {
-  constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
-  int iM, jM, kM;
-  face_node<N1>(f, a, b, iM, jM, kM);
-  pM = iM + N1 * jM + NF * kM;
-  switch (f) {
-    case 0: kn = ke + (ey > 0 ? -op.NeX : (long)(op.NeY - 1) * op.NeX); break;
-    case 1: kn = ke + (ex < op.NeX - 1 ? 1 : -(op.NeX - 1)); break;
-    case 2: kn = ke + (ey < op.NeY - 1 ? op.NeX : -(long)(op.NeY - 1) * op.NeX); break;
-    case 3: kn = ke + (ex > 0 ? -1 : op.NeX - 1); break;
-    case 4: kn = ez > 0 ? ke - nxy : -1; break;
-    default: kn = ez < op.NeZ - 1 ? ke + nxy : -1; break;
-  }
-  if (kn >= 0) {
-    int i2, j2, k2;
-    face_node<N1>(face_opp(f), a, b, i2, j2, k2);
-    gP = (size_t)kn * Np + i2 + N1 * j2 + NF * k2;
-  } else {
-    gP = (size_t)ke * Np + pM;
-  }
-}
-
-template <int N1>
-__device__ __forceinline__ f2 dsum_p(const NdOpsP& op, const float2* u, int dir, int i, int j, int k) {
-  constexpr int NF = N1 * N1;
-  f2acc s;
-#pragma unroll
-  for (int l = 0; l < N1; ++l) {
-    const int p = dir == 0 ? l + N1 * j + NF * k : (dir == 1 ? i + N1 * l + NF * k : i + N1 * j + NF * l);
-    s.add(f2_of(op.D[(dir == 0 ? i : (dir == 1 ? j : k)) * N1 + l]), f2_of(u[p]));
-  }
-  return s.get();
-}
-// Lift of the faces of one direction (x: faces 1, 3; y: 0, 2; z: 4, 5)
-template <int N1>
-__device__ __forceinline__ void lift_dir_p(f2acc& s, const NdOpsP& op, const float2* fv, int dir, int i, int j, int k) {
-  constexpr int NF = N1 * N1;
-  if (dir == 0) {
-    s.add(f2_of(op.Lt[i]), f2_of(fv[1 * NF + j + N1 * k]));
-    s.add(f2_of(op.Lb[i]), f2_of(fv[3 * NF + j + N1 * k]));
-  } else if (dir == 1) {
-    s.add(f2_of(op.Lb[j]), f2_of(fv[0 * NF + i + N1 * k]));
-    s.add(f2_of(op.Lt[j]), f2_of(fv[2 * NF + i + N1 * k]));
-  } else {
-    s.add(f2_of(op.Lb[k]), f2_of(fv[4 * NF + i + N1 * j]));
-    s.add(f2_of(op.Lt[k]), f2_of(fv[5 * NF + i + N1 * j]));
-  }
-}
-
-struct NdIdx {
-  long ke;
-  int p, le, i, j, k, ex, ey, ez, nxy;
-  bool valid;
+struct NdTab {
+  p2m D[N1 * N1], lf[N1], lo[N1];
 };
-template <int N1, int EPB>
-__device__ __forceinline__ NdIdx nd_idx(const NdOpsP& op, int Ne) {
-  constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
-  NdIdx e;
-  const int tid = threadIdx.x;
-  e.le = tid / Np;
-  e.p = tid - e.le * Np;
-  e.ke = (long)blockIdx.x * EPB + e.le;
-  e.valid = e.ke < Ne;
-  e.i = e.p % N1;
-  e.j = (e.p / N1) % N1;
-  e.k = e.p / NF;
-  e.nxy = op.NeX * op.NeY;
-  e.ez = e.valid ? (int)(e.ke / e.nxy) : 0;
-  e.ey = e.valid ? (int)((e.ke - (long)e.ez * e.nxy) / op.NeX) : 0;
-  e.ex = e.valid ? (int)(e.ke - (long)e.ez * e.nxy - (long)e.ey * op.NeX) : 0;
-  return e;
+template <int N1>
+__device__ __forceinline__ void nd_tables(const NdOpsP& op, NdTab<N1>& T) {
+  for (int c = threadIdx.x; c < N1 * N1; c += blockDim.x) {
+    st(T.D[c], p2_dup(op.D[c]));
+    if (c < N1) {
+      st(T.lf[c], p2_dup(op.lf[c]));
+      st(T.lo[c], p2_dup(op.lo[c]));
+    }
+  }
+}
+
+// position of node (i, row = j + N1 k): rows permuted so that one column of neighbouring rows falls on
+// different banks
+template <int N1>
+__device__ __forceinline__ int nd_at(int i, int row) {
+  if (N1 == 8) i ^= row & 7;
+  if (N1 == 4) i ^= (row >> 1) & 3;
+  return row * N1 + i;
+}
+
+// blocks per SM: 48 warps of 40 registers
+constexpr int nd_minb(int threads) { return 1536 / ((threads + 31) / 32 * 32); }
+
+// the thread's (first) node in elements e[0] and e[1] (e[1] = e[0] where the last element has no partner)
+struct NdIdx {
+  int e[2], ex[2], ey[2], ez[2], nxy, p, i, j, k;
+  bool valid, both;
+};
+template <int N1, int PPB, int NT>
+__device__ __forceinline__ NdIdx nd_idx(const NdOpsP& op, int Ne, int& pair) {
+  constexpr int NF = N1 * N1;
+  NdIdx x;
+  pair = threadIdx.x / NT;
+  x.p = threadIdx.x - pair * NT;
+  const int e0 = 2 * (blockIdx.x * PPB + pair);
+  x.valid = e0 < Ne;
+  x.both = e0 + 1 < Ne;
+  x.nxy = op.NeX * op.NeY;
+  x.i = x.p % N1;
+  x.j = (x.p / N1) % N1;
+  x.k = x.p / NF;
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    x.e[m] = x.valid ? (x.both ? e0 + m : e0) : 0;
+    x.ez[m] = x.e[m] / x.nxy;
+    x.ey[m] = (x.e[m] - x.ez[m] * x.nxy) / op.NeX;
+    x.ex[m] = x.e[m] - x.ez[m] * x.nxy - x.ey[m] * op.NeX;
+  }
+  return x;
+}
+// the neighbour across face dir (0 x, 1 y, 2 z) on the lower (up = 0) or upper side; -1 at a lid
+__device__ __forceinline__ int nd_nbr(const NdOpsP& op, const NdIdx& x, int m, int dir, int up) {
+  const int e = x.e[m];
+  if (dir == 0) return up ? (x.ex[m] < op.NeX - 1 ? e + 1 : e - (op.NeX - 1)) : (x.ex[m] > 0 ? e - 1 : e + op.NeX - 1);
+  if (dir == 1)
+    return up ? (x.ey[m] < op.NeY - 1 ? e + op.NeX : e - (op.NeY - 1) * op.NeX)
+              : (x.ey[m] > 0 ? e - op.NeX : e + (op.NeY - 1) * op.NeX);
+  return up ? (x.ez[m] < op.NeZ - 1 ? e + x.nxy : -1) : (x.ez[m] > 0 ? e - x.nxy : -1);
+}
+// node (i, j, k) of face node ab on side `s` (0 lower, 1 upper) of direction dir
+template <int N1>
+__device__ __forceinline__ void nd_face_node(int dir, int s, int ab, int& i, int& row) {
+  const int a = ab % N1, b = ab / N1, w = s * (N1 - 1);
+  i = dir == 0 ? w : a;
+  row = dir == 0 ? a + N1 * b : (dir == 1 ? w + N1 * b : b + N1 * w);
 }
 
 // a field read either as FP64 (the prognostic variable) or as pairs (an intermediate)
 struct Src {
   const double* d;
   const float2* p;
-  __device__ __forceinline__ f2 at(size_t g) const { return d ? ld64(d, g) : ldp(p, g); }
+  __device__ __forceinline__ f2 at(size_t g) const { return d ? f2_split(__ldg(d + g)) : f2_of(__ldg(p + g)); }
 };
+__device__ __forceinline__ p2 nd_dens(const double* __restrict__ prof, const double* __restrict__ dd, const int (&lev)[2],
+                                      const size_t (&g)[2]) {
+  return p2_split(__ldg(dd + g[0]), __ldg(dd + g[1])) + p2_split(__ldg(prof + lev[0]), __ldg(prof + lev[1]));
+}
 
-// gradient pass: G = (d/dx Vh, d/dy Vh, d/dz Vv), divided by the density when dens_div; the even
-// routine's lid exterior of Vh (and of Vv when bc_v)
-template <int N1, int EPB>
-__global__ void __launch_bounds__(EPB* N1* N1* N1)
-    k_nd_grad_p(const NdOpsP op, const double* __restrict__ dens_prof, const Src Vh, const Src Vv,
-                const double* __restrict__ ddens, int var, int dens_div, int bc_v, float2* __restrict__ Gx,
+// E times (the contraction along direction dir + the Lift of its faces): Fscale and Escale are the same 2/dx, and
+// one factor keeps its rounding common to both terms, which cancel to a large part.  Each direction has a sum of
+// its own: the rounding of a compensated sum's error term grows with the number of terms (the update's 27 in one
+// sum: an error of 1.05e-14 of the change at p = 7; as here 6.2e-15)
+template <int N1, int NPT>
+__device__ __forceinline__ void nd_dir(p2 (&r)[NPT], const NdTab<N1>& T, p2 E, const p2m* u, const p2m* df, int dir, int i,
+                                       int j, int k, bool lid) {
+  constexpr int NF = N1 * N1, KH = N1 / NPT;
+  const int row = dir == 0 ? i : j;
+  p2acc s[NPT];
+#pragma unroll
+  for (int l = 0; l < N1; ++l) {
+    p2 d, v;
+    if (dir < 2) d = ld(T.D[l * N1 + row]);
+    else v = ld(u[nd_at<N1>(i, j + N1 * l)]);
+#pragma unroll
+    for (int h = 0; h < NPT; ++h) {
+      const int kh = k + h * KH;
+      if (dir < 2) v = ld(u[dir == 0 ? nd_at<N1>(l, j + N1 * kh) : nd_at<N1>(i, l + N1 * kh)]);
+      else d = ld(T.D[l * N1 + kh]);
+      s[h].add(d, v);
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < NPT; ++h) {
+    const int kh = k + h * KH, rw = dir == 2 ? kh : row;
+    const int ab = dir == 0 ? j + N1 * kh : (dir == 1 ? i + N1 * kh : i + N1 * j);
+    s[h].add(ld(T.lf[rw]), ld(df[dir * NF + ab]));
+    if (dir == 2 && lid) s[h].add(ld(T.lo[rw]), ld(df[3 * NF + ab]));
+    r[h] = E * s[h].get();
+  }
+}
+
+// gradient pass: G = (d/dx Vh, d/dy Vh, d/dz Vv), divided by the density when dens_div; at a lid the even
+// routine's exterior of Vv (when bc_v), which leaves a jump only for the wall-normal momentum.
+// ONE: Vh and Vv are the same field.
+template <int N1, int PPB, int NPT, bool ONE>
+__global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, nd_minb(PPB * N1 * N1 * N1 / NPT))
+    k_nd_grad_p(const __grid_constant__ NdOpsP op, const double* __restrict__ dens_prof, const Src Vh, const Src Vv,
+                const double* __restrict__ ddens, int dens_div, int refl, float2* __restrict__ Gx,
                 float2* __restrict__ Gy, float2* __restrict__ Gz, int Ne) {
-  constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
-  extern __shared__ float2 smp[];
-  const NdIdx e = nd_idx<N1, EPB>(op, Ne);
-  float2* vh = smp + e.le * (2 * Np + 6 * NF);
-  float2* vv = vh + Np;
-  float2* df = vv + Np;
-  const size_t g = (size_t)e.ke * Np + e.p;
-  if (e.valid) {
-    const f2 rd = dens_div ? f2_recip(ld64(ddens, g) + f2_split(__ldg(dens_prof + e.ez * N1 + e.k))) : f2{1.f, 0.f};
-    vh[e.p] = f2_pack(Vh.at(g) * rd);
-    vv[e.p] = f2_pack(Vv.at(g) * rd);
-    for (int fi = e.p; fi < 6 * NF; fi += Np) {
-      const int f = fi / NF, ab = fi - f * NF, a = ab % N1, b = ab / N1;
-      int pM;
-      size_t gP;
-      long kn;
-      face_nodes_nd<N1>(op, f, a, b, e.ke, e.ex, e.ey, e.ez, e.nxy, pM, gP, kn);
-      const size_t gM = (size_t)e.ke * Np + pM;
-      const int dir = face_dir_p(f);
-      const float n = face_n_p(f);
-      f2 wM{1.f, 0.f}, wP{1.f, 0.f};
+  constexpr int Np = N1 * N1 * N1, NF = N1 * N1, NT = Np / NPT, KH = N1 / NPT;
+  extern __shared__ p2m smp[];
+  NdTab<N1>& T = *reinterpret_cast<NdTab<N1>*>(smp);
+  int pair;
+  const NdIdx x = nd_idx<N1, PPB, NT>(op, Ne, pair);
+  p2m* vh = smp + sizeof(NdTab<N1>) / sizeof(p2m) + pair * ((ONE ? 1 : 2) * Np + 4 * NF);
+  p2m* vv = ONE ? vh : vh + Np;
+  p2m* df = vv + Np;
+  const size_t g[2] = {(size_t)x.e[0] * Np + x.p, (size_t)x.e[1] * Np + x.p};
+  nd_tables<N1>(op, T);
+  if (x.valid) {
+#pragma unroll
+    for (int h = 0; h < NPT; ++h) {
+      const size_t gh[2] = {g[0] + h * NT, g[1] + h * NT};
+      p2 a = p2_of(Vh.at(gh[0]), Vh.at(gh[1])), b = ONE ? a : p2_of(Vv.at(gh[0]), Vv.at(gh[1]));
       if (dens_div) {
-        const int levM = e.ez * N1 + pM / NF;
-        const int levP = (kn >= 0 ? (int)(kn / e.nxy) : e.ez) * N1 + (int)((gP % Np) / NF);
-        wP = f2_recip(ld64(ddens, gP) + f2_split(__ldg(dens_prof + levP)));
-        wM = f2_recip(ld64(ddens, gM) + f2_split(__ldg(dens_prof + levM)));
+        const int lev[2] = {x.ez[0] * N1 + x.k + h * KH, x.ez[1] * N1 + x.k + h * KH};
+        const p2 rd = p2_recip(nd_dens(dens_prof, ddens, lev, gh));
+        a = a * rd;
+        if (!ONE) b = b * rd;
       }
-      const bool lid = kn < 0;
+      const int at = nd_at<N1>(x.i, x.j + N1 * (x.k + h * KH));
+      st(vh[at], a);
+      if (!ONE) st(vv[at], b);
+    }
+  }
+  const bool top = refl && (x.ez[0] == op.NeZ - 1 || x.ez[1] == op.NeZ - 1);
+  if (x.valid) {
+    for (int fi = x.p; fi < 3 * NF; fi += NT) {
+      const int dir = fi / NF, ab = fi - dir * NF;
+      int iP, rP;
+      nd_face_node<N1>(dir, 1, ab, iP, rP);
+      size_t gP[2];
+      int lev[2];
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int kn = nd_nbr(op, x, m, dir, 0);
+        gP[m] = (size_t)(kn < 0 ? x.e[m] : kn) * Np + rP * N1 + iP;
+        lev[m] = (dir == 2 && kn >= 0 ? x.ez[m] - 1 : x.ez[m]) * N1 + rP / N1;
+      }
       const Src& S = dir == 2 ? Vv : Vh;
-      const f2 sM = S.at(gM);
-      f2 sP = S.at(gP);
-      if (lid && (dir != 2 || bc_v)) sP = even_ext_p(var, dir, sM);
-      const f2 d = f2_mul_f(sP * wP - sM * wM, 0.5f);
-      // (1 - sign n) on interior faces: 2 on faces with n = -1, 0 with n = +1; 1 at a lid
-      const float fac = lid ? n : (n < 0.f ? -2.f : 0.f);
-      df[fi] = f2_pack(f2_mul_f(f2_of(op.FS[dir]) * d, fac));
+      p2 sP = p2_of(S.at(gP[0]), S.at(gP[1]));
+      if (dens_div) sP = sP * p2_recip(nd_dens(dens_prof, ddens, lev, gP));
+      st(df[fi], sP);
     }
   }
   __syncthreads();
-  if (!e.valid) return;
-  f2acc sx, sy, sz;
-  sx.add(f2_of(op.E[0]), dsum_p<N1>(op, vh, 0, e.i, e.j, e.k));
-  lift_dir_p<N1>(sx, op, df, 0, e.i, e.j, e.k);
-  sy.add(f2_of(op.E[1]), dsum_p<N1>(op, vh, 1, e.i, e.j, e.k));
-  lift_dir_p<N1>(sy, op, df, 1, e.i, e.j, e.k);
-  sz.add(f2_of(op.E[2]), dsum_p<N1>(op, vv, 2, e.i, e.j, e.k));
-  lift_dir_p<N1>(sz, op, df, 2, e.i, e.j, e.k);
-  Gx[g] = f2_pack(sx.get());
-  Gy[g] = f2_pack(sy.get());
-  Gz[g] = f2_pack(sz.get());
-}
-
-// Laplacian pass with the odd routine's lid exterior of G: horizontal and vertical parts
-template <int N1, int EPB>
-__global__ void __launch_bounds__(EPB* N1* N1* N1)
-    k_nd_lap_p(const NdOpsP op, const float2* __restrict__ Gx, const float2* __restrict__ Gy,
-               const float2* __restrict__ Gz, int var, float2* __restrict__ lh, float2* __restrict__ lv, int Ne) {
-  constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
-  extern __shared__ float2 smp[];
-  const NdIdx e = nd_idx<N1, EPB>(op, Ne);
-  float2* gx = smp + e.le * (3 * Np + 6 * NF);
-  float2* gy = gx + Np;
-  float2* gz = gy + Np;
-  float2* df = gz + Np;
-  const size_t g = (size_t)e.ke * Np + e.p;
-  if (e.valid) {
-    gx[e.p] = __ldg(Gx + g);
-    gy[e.p] = __ldg(Gy + g);
-    gz[e.p] = __ldg(Gz + g);
-    for (int fi = e.p; fi < 6 * NF; fi += Np) {
-      const int f = fi / NF, ab = fi - f * NF, a = ab % N1, b = ab / N1;
-      int pM;
-      size_t gP;
-      long kn;
-      face_nodes_nd<N1>(op, f, a, b, e.ke, e.ex, e.ey, e.ez, e.nxy, pM, gP, kn);
-      const size_t gM = (size_t)e.ke * Np + pM;
-      const int dir = face_dir_p(f);
-      const float n = face_n_p(f);
-      const float2* Gd = dir == 0 ? Gx : (dir == 1 ? Gy : Gz);
-      const f2 gMc = ldp(Gd, gM);
-      const bool lid = kn < 0;
-      const f2 gPc = lid ? odd_ext_p(var, dir, gMc) : ldp(Gd, gP);
-      // 0.5 (1 + sign n) (g+ - g-) n on interior faces; 0.5 (g+ - g-) n at a lid
-      const float fac = lid ? 0.5f * n : (n > 0.f ? 1.f : 0.f);
-      df[fi] = f2_pack(f2_mul_f(f2_of(op.FS[dir]) * (gPc - gMc), fac));
-    }
-  }
-  __syncthreads();
-  if (!e.valid) return;
-  f2acc sh, sv;
-  sh.add(f2_of(op.E[0]), dsum_p<N1>(op, gx, 0, e.i, e.j, e.k));
-  sh.add(f2_of(op.E[1]), dsum_p<N1>(op, gy, 1, e.i, e.j, e.k));
-  lift_dir_p<N1>(sh, op, df, 0, e.i, e.j, e.k);
-  lift_dir_p<N1>(sh, op, df, 1, e.i, e.j, e.k);
-  sv.add(f2_of(op.E[2]), dsum_p<N1>(op, gz, 2, e.i, e.j, e.k));
-  lift_dir_p<N1>(sv, op, df, 2, e.i, e.j, e.k);
-  lh[g] = f2_pack(sh.get());
-  lv[g] = f2_pack(sv.get());
-}
-
-// tendency pass with the odd routine's lid exterior of G, then V += dt tend (the increment in pairs,
-// added to the FP64 field in FP64)
-template <int N1, int EPB>
-__global__ void __launch_bounds__(EPB* N1* N1* N1)
-    k_nd_tend_p(const NdOpsP op, const double* __restrict__ dens_prof, const float2* __restrict__ Gx,
-                const float2* __restrict__ Gy, const float2* __restrict__ Gz, const double* ddens, int var, int mul_dens,
-                float2 ch, float2 cv, float2 dt, double* V, int Ne) {
-  constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
-  extern __shared__ float2 smp[];
-  const NdIdx e = nd_idx<N1, EPB>(op, Ne);
-  float2* fx = smp + e.le * (3 * Np + 6 * NF);
-  float2* fy = fx + Np;
-  float2* fz = fy + Np;
-  float2* df = fz + Np;
-  const size_t g = (size_t)e.ke * Np + e.p;
-  if (e.valid) {
-    // DDENS is read only when it weights the variable (for DDENS itself V aliases it)
-    const f2 dens = mul_dens ? f2_split(__ldg(dens_prof + e.ez * N1 + e.k)) + ld64(ddens, g) : f2{1.f, 0.f};
-    const f2 h = f2_of(ch) * dens, v = f2_of(cv) * dens;
-    fx[e.p] = f2_pack(h * ldp(Gx, g));
-    fy[e.p] = f2_pack(h * ldp(Gy, g));
-    fz[e.p] = f2_pack(v * ldp(Gz, g));
-    for (int fi = e.p; fi < 6 * NF; fi += Np) {
-      const int f = fi / NF, ab = fi - f * NF, a = ab % N1, b = ab / N1;
-      int pM;
-      size_t gP;
-      long kn;
-      face_nodes_nd<N1>(op, f, a, b, e.ke, e.ex, e.ey, e.ez, e.nxy, pM, gP, kn);
-      const size_t gM = (size_t)e.ke * Np + pM;
-      const int dir = face_dir_p(f);
-      const float n = face_n_p(f);
-      const float2* Gd = dir == 0 ? Gx : (dir == 1 ? Gy : Gz);
-      const f2 gMc = ldp(Gd, gM);
-      const bool lid = kn < 0;
-      const f2 gPc = lid ? odd_ext_p(var, dir, gMc) : ldp(Gd, gP);
-      f2 wM{0.5f, 0.f}, wP{0.5f, 0.f};
-      if (mul_dens) {
-        const int levM = e.ez * N1 + pM / NF;
-        const int levP = (kn >= 0 ? (int)(kn / e.nxy) : e.ez) * N1 + (int)((gP % Np) / NF);
-        wM = f2_mul_f(f2_split(__ldg(dens_prof + levM)) + ld64(ddens, gM), 0.5f);
-        wP = f2_mul_f(f2_split(__ldg(dens_prof + levP)) + ld64(ddens, gP), 0.5f);
+  // jumps of the lower faces of x, y, z, then the upper lid's
+  if (x.valid) {
+    for (int fi = x.p; fi < (top ? 4 : 3) * NF; fi += NT) {
+      const int f = fi / NF, ab = fi - f * NF, dir = f < 2 ? f : 2;
+      int iM, rM;
+      nd_face_node<N1>(dir, f == 3, ab, iM, rM);
+      const p2 own = ld((dir == 2 ? vv : vh)[nd_at<N1>(iM, rM)]);
+      const int lz = f == 3 ? op.NeZ - 1 : 0;  // lid layer; -2 v there against the coefficient's 1/2
+      const bool la = f >= 2 && x.ez[0] == lz, lb = f >= 2 && x.ez[1] == lz;
+      p2 d = f == 3 ? p2_zero() : ld(df[fi]) - own;
+      if (la || lb) {
+        const p2 r = refl ? p2_neg(own) : p2_zero();
+        d = p2_of(la ? p2_a(r) : p2_a(d), lb ? p2_b(r) : p2_b(d));
       }
-      const f2 c = f2_of(dir == 2 ? cv : ch);
-      // (1 + sign n) on interior faces: 2 with n = +1, 0 with n = -1; 1 at a lid
-      const float fac = lid ? n : (n > 0.f ? 2.f : 0.f);
-      df[fi] = f2_pack(f2_mul_f(f2_of(op.FS[dir]) * (c * (wP * gPc - wM * gMc)), fac));
+      st(df[fi], d);
     }
   }
   __syncthreads();
-  if (!e.valid) return;
-  f2acc s;
-  s.add(f2_of(op.E[0]), dsum_p<N1>(op, fx, 0, e.i, e.j, e.k));
-  s.add(f2_of(op.E[1]), dsum_p<N1>(op, fy, 1, e.i, e.j, e.k));
-  s.add(f2_of(op.E[2]), dsum_p<N1>(op, fz, 2, e.i, e.j, e.k));
-  lift_dir_p<N1>(s, op, df, 0, e.i, e.j, e.k);
-  lift_dir_p<N1>(s, op, df, 1, e.i, e.j, e.k);
-  lift_dir_p<N1>(s, op, df, 2, e.i, e.j, e.k);
-  const f2 inc = f2_of(dt) * s.get();
-  V[g] = (V[g] + (double)inc.h) + (double)inc.l;
+  if (!x.valid) return;
+#pragma unroll
+  for (int dir = 0; dir < 3; ++dir) {
+    p2 r[NPT];
+    nd_dir<N1, NPT>(r, T, p2_dup(op.E[dir]), dir == 2 ? vv : vh, df, dir, x.i, x.j, x.k, top);
+    float2* G = dir == 0 ? Gx : (dir == 1 ? Gy : Gz);
+#pragma unroll
+    for (int h = 0; h < NPT; ++h) {
+      G[g[0] + h * NT] = f2_pack(p2_a(r[h]));
+      if (x.both) G[g[1] + h * NT] = f2_pack(p2_b(r[h]));
+    }
+  }
+}
+
+// divergence of the gradient (times the density when mul_dens), with the odd routine's lid exterior of
+// it, which leaves a jump except for the wall-normal momentum (keep).  TEND: V += the sum, whose
+// tables hold dt and the coefficients (the increment in pairs, added to the FP64 field in FP64); else the Laplacian's
+// horizontal and vertical parts.
+template <int N1, int PPB, int NPT, bool TEND>
+__global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, nd_minb(PPB * N1 * N1 * N1 / NPT))
+    k_nd_div_p(const __grid_constant__ NdOpsP op, const double* __restrict__ dens_prof, const float2* __restrict__ Gx,
+               const float2* __restrict__ Gy, const float2* __restrict__ Gz, const double* ddens, int mul_dens, int keep,
+               float2* __restrict__ lh, float2* __restrict__ lv, double* V, int Ne) {
+  constexpr int Np = N1 * N1 * N1, NF = N1 * N1, NT = Np / NPT, KH = N1 / NPT;
+  extern __shared__ p2m smp[];
+  NdTab<N1>& T = *reinterpret_cast<NdTab<N1>*>(smp);
+  int pair;
+  const NdIdx x = nd_idx<N1, PPB, NT>(op, Ne, pair);
+  p2m* fl = smp + sizeof(NdTab<N1>) / sizeof(p2m) + pair * (3 * Np + 4 * NF);
+  p2m* df = fl + 3 * Np;
+  const size_t g[2] = {(size_t)x.e[0] * Np + x.p, (size_t)x.e[1] * Np + x.p};
+  nd_tables<N1>(op, T);
+  if (x.valid) {
+#pragma unroll
+    for (int h = 0; h < NPT; ++h) {
+      const size_t gh[2] = {g[0] + h * NT, g[1] + h * NT};
+      p2 v[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const float2* G = d == 0 ? Gx : (d == 1 ? Gy : Gz);
+        v[d] = p2_of(__ldg(G + gh[0]), __ldg(G + gh[1]));
+      }
+      if (mul_dens) {  // DDENS is read only when it weights the variable (for DDENS itself V aliases it)
+        const int lev[2] = {x.ez[0] * N1 + x.k + h * KH, x.ez[1] * N1 + x.k + h * KH};
+        const p2 dens = nd_dens(dens_prof, ddens, lev, gh);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) v[d] = dens * v[d];
+      }
+#pragma unroll
+      for (int d = 0; d < 3; ++d) st(fl[d * Np + nd_at<N1>(x.i, x.j + N1 * (x.k + h * KH))], v[d]);
+    }
+  }
+  const bool bot = !keep && (x.ez[0] == 0 || x.ez[1] == 0);
+  if (x.valid) {
+    for (int fi = x.p; fi < 3 * NF; fi += NT) {
+      const int dir = fi / NF, ab = fi - dir * NF;
+      int iP, rP;
+      nd_face_node<N1>(dir, 0, ab, iP, rP);
+      size_t gP[2];
+      int lev[2];
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int kn = nd_nbr(op, x, m, dir, 1);
+        gP[m] = (size_t)(kn < 0 ? x.e[m] : kn) * Np + rP * N1 + iP;
+        lev[m] = (dir == 2 && kn >= 0 ? x.ez[m] + 1 : x.ez[m]) * N1 + rP / N1;
+      }
+      const float2* G = dir == 0 ? Gx : (dir == 1 ? Gy : Gz);
+      p2 sP = p2_of(__ldg(G + gP[0]), __ldg(G + gP[1]));
+      if (mul_dens) sP = nd_dens(dens_prof, ddens, lev, gP) * sP;
+      st(df[fi], sP);
+    }
+  }
+  __syncthreads();
+  // jumps of the upper faces of x, y, z, then the lower lid's
+  if (x.valid) {
+    for (int fi = x.p; fi < (bot ? 4 : 3) * NF; fi += NT) {
+      const int f = fi / NF, ab = fi - f * NF, dir = f < 2 ? f : 2;
+      int iM, rM;
+      nd_face_node<N1>(dir, f != 3, ab, iM, rM);
+      const p2 own = ld(fl[dir * Np + nd_at<N1>(iM, rM)]);
+      const int lz = f == 3 ? 0 : op.NeZ - 1;
+      const bool la = f >= 2 && x.ez[0] == lz, lb = f >= 2 && x.ez[1] == lz;
+      p2 d = f == 3 ? p2_zero() : ld(df[fi]) - own;
+      if (la || lb) {
+        const p2 r = keep ? p2_zero() : p2_neg(own);
+        d = p2_of(la ? p2_a(r) : p2_a(d), lb ? p2_b(r) : p2_b(d));
+      }
+      st(df[fi], d);
+    }
+  }
+  __syncthreads();
+  if (!x.valid) return;
+  p2 r[NPT], t[NPT];
+  nd_dir<N1, NPT>(r, T, p2_dup(op.E[0]), fl, df, 0, x.i, x.j, x.k, false);
+  nd_dir<N1, NPT>(t, T, p2_dup(op.E[1]), fl + Np, df, 1, x.i, x.j, x.k, false);
+#pragma unroll
+  for (int h = 0; h < NPT; ++h) {
+    r[h] = r[h] + t[h];
+    if (!TEND) {
+      lh[g[0] + h * NT] = f2_pack(p2_a(r[h]));
+      if (x.both) lh[g[1] + h * NT] = f2_pack(p2_b(r[h]));
+    }
+  }
+  nd_dir<N1, NPT>(t, T, p2_dup(op.E[2]), fl + 2 * Np, df, 2, x.i, x.j, x.k, bot);
+#pragma unroll
+  for (int h = 0; h < NPT; ++h) {
+    if (TEND) t[h] = r[h] + t[h];
+    const f2 a = p2_a(t[h]), b = p2_b(t[h]);
+    const size_t ga = g[0] + h * NT, gb = g[1] + h * NT;
+    if (TEND) {
+      V[ga] = (V[ga] + (double)a.h) + (double)a.l;
+      if (x.both) V[gb] = (V[gb] + (double)b.h) + (double)b.l;
+    } else {
+      lv[ga] = f2_pack(a);
+      if (x.both) lv[gb] = f2_pack(b);
+    }
+  }
 }
 
 float2 hsplit_nd(double x) {
@@ -299,45 +351,65 @@ float2 hsplit_nd(double x) {
   return make_float2(h, (float)(x - (double)h));
 }
 
-template <int N1>
-constexpr int nd_epb_p() { return N1 <= 4 ? (N1 <= 2 ? 16 : (N1 == 3 ? 8 : 4)) : 1; }
-
-template <int N1>
-int nd_pass_p_n(int pass, const NdOpsP& op, const double* dp, Src a, Src b, const float2* G0, const float2* G1,
-                const float2* G2, const double* ddens, int var, int f1, int f2, float2 ch, float2 cv, float2 dt,
-                float2* o1, float2* o2, float2* o3, double* V, int Ne, cudaStream_t s) {
-  constexpr int EPB = nd_epb_p<N1>(), Np = N1 * N1 * N1, NF = N1 * N1;
-  const int grid = (Ne + EPB - 1) / EPB;
-  if (pass == 0) {
-    const size_t sm = sizeof(float2) * EPB * (2 * Np + 6 * NF);
-    auto kf = k_nd_grad_p<N1, EPB>;
-    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kf<<<grid, EPB * Np, sm, s>>>(op, dp, a, b, ddens, var, f1, f2, o1, o2, o3, Ne);
-  } else if (pass == 1) {
-    const size_t sm = sizeof(float2) * EPB * (3 * Np + 6 * NF);
-    auto kf = k_nd_lap_p<N1, EPB>;
-    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kf<<<grid, EPB * Np, sm, s>>>(op, G0, G1, G2, var, o1, o2, Ne);
-  } else {
-    const size_t sm = sizeof(float2) * EPB * (3 * Np + 6 * NF);
-    auto kf = k_nd_tend_p<N1, EPB>;
-    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kf<<<grid, EPB * Np, sm, s>>>(op, dp, G0, G1, G2, ddens, var, f1, ch, cv, dt, V, Ne);
+// tables of a pass: factors of the three directions, and which side interior elements take their flux from
+NdOpsP nd_ops(const Ops& d, const double (&fac)[3], bool lower) {
+  NdOpsP op;
+  std::memset(&op, 0, sizeof(op));
+  const int N1 = d.N1;
+  const double E[3] = {d.E11, d.E22, d.E33};
+  for (int c = 0; c < 3; ++c) op.E[c] = hsplit_nd(fac[c] * E[c]);
+  for (int i = 0; i < N1; ++i) {
+    for (int l = 0; l < N1; ++l) op.D[l * N1 + i] = hsplit_nd(d.D[i * N1 + l]);
+    op.lf[i] = hsplit_nd(lower ? -d.Lb[i] : d.Lt[i]);
+    op.lo[i] = hsplit_nd(lower ? d.Lt[i] : -d.Lb[i]);
   }
-  return (int)cudaGetLastError();
+  op.NeX = d.NeX;
+  op.NeY = d.NeY;
+  op.NeZ = d.NeZ;
+  return op;
 }
 
-int nd_pass_p(int N1, int pass, const NdOpsP& op, const double* dp, Src a, Src b, const float2* G0, const float2* G1,
-              const float2* G2, const double* ddens, int var, int f1, int f2, float2 ch, float2 cv, float2 dt,
-              float2* o1, float2* o2, float2* o3, double* V, int Ne, cudaStream_t s) {
+// pairs of elements per block: 108 to 343 threads
+template <int N1>
+constexpr int nd_ppb() { return N1 <= 4 ? (N1 == 2 ? 32 : (N1 == 3 ? 8 : 4)) : 1; }
+
+struct NdPass {
+  int pass;  // 0 gradient, 1 Laplacian, 2 update
+  Src a, b;  // gradient: the fields of the horizontal and of the vertical derivative
+  const double* ddens;
+  int dens, wall;  // density division / weight; the lid's reflection (gradient), or none at it (divergence)
+  float2 *G[3], *lh, *lv;
+  double* V;
+};
+
+template <int N1>
+int nd_pass_n(const NdPass& P, const NdOpsP& op, const double* dp, int Ne, cudaStream_t s) {
+  constexpr int PPB = nd_ppb<N1>(), Np = N1 * N1 * N1, NF = N1 * N1, NPT = N1 % 2 == 0 ? 2 : 1;
+  const int grid = ((Ne + 1) / 2 + PPB - 1) / PPB;
+  const bool one = P.pass == 0 && P.a.d == P.b.d && P.a.p == P.b.p;
+  const size_t sm = sizeof(NdTab<N1>) + sizeof(p2m) * PPB * ((P.pass == 0 ? (one ? 1 : 2) : 3) * Np + 4 * NF);
+  auto go = [&](auto kf, auto... args) {
+    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    kf<<<grid, PPB * Np / NPT, sm, s>>>(op, dp, args..., Ne);
+    return (int)cudaGetLastError();
+  };
+  if (P.pass == 0)
+    return one ? go(k_nd_grad_p<N1, PPB, NPT, true>, P.a, P.b, P.ddens, P.dens, P.wall, P.G[0], P.G[1], P.G[2])
+               : go(k_nd_grad_p<N1, PPB, NPT, false>, P.a, P.b, P.ddens, P.dens, P.wall, P.G[0], P.G[1], P.G[2]);
+  const float2 *gx = P.G[0], *gy = P.G[1], *gz = P.G[2];
+  return P.pass == 1 ? go(k_nd_div_p<N1, PPB, NPT, false>, gx, gy, gz, P.ddens, P.dens, P.wall, P.lh, P.lv, P.V)
+                     : go(k_nd_div_p<N1, PPB, NPT, true>, gx, gy, gz, P.ddens, P.dens, P.wall, P.lh, P.lv, P.V);
+}
+
+int nd_pass_p(int N1, const NdPass& P, const NdOpsP& op, const double* dp, int Ne, cudaStream_t s) {
   switch (N1) {
-    case 2: return nd_pass_p_n<2>(pass, op, dp, a, b, G0, G1, G2, ddens, var, f1, f2, ch, cv, dt, o1, o2, o3, V, Ne, s);
-    case 3: return nd_pass_p_n<3>(pass, op, dp, a, b, G0, G1, G2, ddens, var, f1, f2, ch, cv, dt, o1, o2, o3, V, Ne, s);
-    case 4: return nd_pass_p_n<4>(pass, op, dp, a, b, G0, G1, G2, ddens, var, f1, f2, ch, cv, dt, o1, o2, o3, V, Ne, s);
-    case 5: return nd_pass_p_n<5>(pass, op, dp, a, b, G0, G1, G2, ddens, var, f1, f2, ch, cv, dt, o1, o2, o3, V, Ne, s);
-    case 6: return nd_pass_p_n<6>(pass, op, dp, a, b, G0, G1, G2, ddens, var, f1, f2, ch, cv, dt, o1, o2, o3, V, Ne, s);
-    case 7: return nd_pass_p_n<7>(pass, op, dp, a, b, G0, G1, G2, ddens, var, f1, f2, ch, cv, dt, o1, o2, o3, V, Ne, s);
-    case 8: return nd_pass_p_n<8>(pass, op, dp, a, b, G0, G1, G2, ddens, var, f1, f2, ch, cv, dt, o1, o2, o3, V, Ne, s);
+    case 2: return nd_pass_n<2>(P, op, dp, Ne, s);
+    case 3: return nd_pass_n<3>(P, op, dp, Ne, s);
+    case 4: return nd_pass_n<4>(P, op, dp, Ne, s);
+    case 5: return nd_pass_n<5>(P, op, dp, Ne, s);
+    case 6: return nd_pass_n<6>(P, op, dp, Ne, s);
+    case 7: return nd_pass_n<7>(P, op, dp, Ne, s);
+    case 8: return nd_pass_n<8>(P, op, dp, Ne, s);
   }
   return (int)cudaErrorInvalidValue;
 }
@@ -347,57 +419,29 @@ int nd_pass_p(int N1, int pass, const NdOpsP& op, const double* dp, Src a, Src b
 // fedg_numdiff_apply_prec with prec == FEDG_PREC_PAIR; scratch = 5 Np*Ne doubles reused as pairs
 int numdiff_apply_pair(fedg_ctx* c, double* const q[5], int nlap, double coef_h, double coef_v, double dt,
                        double* scratch) {
-  const Ops& d = c->op;
-  NdOpsP op;
-  std::memset(&op, 0, sizeof(op));
-  const int N1 = c->N1;
-  for (int a = 0; a < N1 * N1; ++a) op.D[a] = hsplit_nd(d.D[a]);
-  for (int a = 0; a < N1; ++a) {
-    op.Lb[a] = hsplit_nd(d.Lb[a]);
-    op.Lt[a] = hsplit_nd(d.Lt[a]);
-  }
-  op.E[0] = hsplit_nd(d.E11);
-  op.E[1] = hsplit_nd(d.E22);
-  op.E[2] = hsplit_nd(d.E33);
-  op.FS[0] = hsplit_nd(d.FSx);
-  op.FS[1] = hsplit_nd(d.FSy);
-  op.FS[2] = hsplit_nd(d.FSz);
-  op.NeX = d.NeX;
-  op.NeY = d.NeY;
-  op.NeZ = d.NeZ;
+  const double sgn = ((nlap + 1) % 2 == 0) ? 1.0 : -1.0;
+  const NdOpsP grad = nd_ops(c->op, {1.0, 1.0, 1.0}, true), lap = nd_ops(c->op, {1.0, 1.0, 1.0}, false),
+               upd = nd_ops(c->op, {dt * (sgn * coef_h), dt * (sgn * coef_h), dt * (sgn * coef_v)}, false);
   const size_t n = c->n;
   float2* Gx = reinterpret_cast<float2*>(scratch);
-  float2* Gy = Gx + n;
-  float2* Gz = Gy + n;
-  float2* lh = Gz + n;
-  float2* lv = lh + n;
-  const double sgn = ((nlap + 1) % 2 == 0) ? 1.0 : -1.0;
-  const float2 ch = hsplit_nd(sgn * coef_h), cv = hsplit_nd(sgn * coef_v), dtp = hsplit_nd(dt), zero = make_float2(0.f, 0.f);
+  float2 *Gy = Gx + n, *Gz = Gy + n, *lh = Gz + n, *lv = lh + n;
   const int order[5] = {VRT, VMZ, VMX, VMY, VD};
   for (int vi = 0; vi < 5; ++vi) {
     const int var = order[vi];
-    const int dw = var != VD;
-    const Src qv{q[var], nullptr};
-    int r = tracked(c, FEDG_K_ND, [&] {
-      return nd_pass_p(N1, 0, op, c->d_prof, qv, qv, nullptr, nullptr, nullptr, q[VD], var, dw, 1, zero, zero, zero,
-                       Gx, Gy, Gz, nullptr, c->Ne, c->stream);
-    });
+    const int dw = var != VD, wall = var == VMZ;
+    auto pass = [&](int kind, Src a, Src b, int dens, int wl, double* V) {
+      const NdPass P{kind, a, b, q[VD], dens, wl, {Gx, Gy, Gz}, lh, lv, V};
+      return tracked(c, FEDG_K_ND, [&] {
+        return nd_pass_p(c->N1, P, kind == 0 ? grad : (kind == 1 ? lap : upd), c->d_prof, c->Ne, c->stream);
+      });
+    };
+    const Src qv{q[var], nullptr}, L0{nullptr, lh}, L1{nullptr, lv};
+    int r = pass(0, qv, qv, dw, wall, nullptr);
     for (int it = 1; it < nlap && !r; ++it) {
-      r = tracked(c, FEDG_K_ND, [&] {
-        return nd_pass_p(N1, 1, op, c->d_prof, Src{}, Src{}, Gx, Gy, Gz, nullptr, var, 0, 0, zero, zero, zero, lh, lv,
-                         nullptr, nullptr, c->Ne, c->stream);
-      });
-      if (!r)
-        r = tracked(c, FEDG_K_ND, [&] {
-          return nd_pass_p(N1, 0, op, c->d_prof, Src{nullptr, lh}, Src{nullptr, lv}, nullptr, nullptr, nullptr, q[VD], var,
-                           0, 0, zero, zero, zero, Gx, Gy, Gz, nullptr, c->Ne, c->stream);
-        });
+      r = pass(1, Src{}, Src{}, 0, wall, nullptr);
+      if (!r) r = pass(0, L0, L1, 0, 0, nullptr);
     }
-    if (!r)
-      r = tracked(c, FEDG_K_ND, [&] {
-        return nd_pass_p(N1, 2, op, c->d_prof, Src{}, Src{}, Gx, Gy, Gz, q[VD], var, dw, 0, ch, cv, dtp, nullptr, nullptr,
-                         nullptr, q[var], c->Ne, c->stream);
-      });
+    if (!r) r = pass(2, Src{}, Src{}, dw, wall, q[var]);
     if (r) return api_cuda_fail((cudaError_t)r, "fedg_numdiff_apply (pair)");
   }
   return 0;
