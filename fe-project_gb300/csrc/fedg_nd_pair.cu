@@ -14,8 +14,7 @@
 // the divergence the upper), so an element computes three faces, and a lid face only where the
 // reflection leaves a jump.  Coefficients and dt are multiplied into E on the host.
 //
-// A thread owns NPT = 2 nodes (k and k + N1/2) for even N1, which share the loads of the x and y tables; an
-// odd N1 has one.
+// On large p = 7 meshes a thread owns NPT = 2 nodes (k and k + N1/2), which share the loads of the x and y tables.
 //
 // What bounds it: the latency of the loads and the barriers between them, the faces and the sums (FP32 pipe 40 %
 // busy with two blocks of 512 threads per SM), so the blocks are small and many.  Update of five fields, 32x32x16
@@ -27,7 +26,7 @@
 #include <cstring>
 
 #include "fedg_ctx.cuh"
-#include "fedg_p2.cuh"
+#include "fedg_two.cuh"
 
 namespace fedg {
 namespace {
@@ -52,62 +51,6 @@ __device__ __forceinline__ void nd_tables(const NdOpsP& op, NdTab<N1>& T) {
       st(T.lo[c], p2_dup(op.lo[c]));
     }
   }
-}
-
-// position of node (i, row = j + N1 k): rows permuted so that one column of neighbouring rows falls on
-// different banks
-template <int N1>
-__device__ __forceinline__ int nd_at(int i, int row) {
-  if (N1 == 8) i ^= row & 7;
-  if (N1 == 4) i ^= (row >> 1) & 3;
-  return row * N1 + i;
-}
-
-// blocks per SM: 48 warps of 40 registers
-constexpr int nd_minb(int threads) { return 1536 / ((threads + 31) / 32 * 32); }
-
-// the thread's (first) node in elements e[0] and e[1] (e[1] = e[0] where the last element has no partner)
-struct NdIdx {
-  int e[2], ex[2], ey[2], ez[2], nxy, p, i, j, k;
-  bool valid, both;
-};
-template <int N1, int PPB, int NT>
-__device__ __forceinline__ NdIdx nd_idx(const NdOpsP& op, int Ne, int& pair) {
-  constexpr int NF = N1 * N1;
-  NdIdx x;
-  pair = threadIdx.x / NT;
-  x.p = threadIdx.x - pair * NT;
-  const int e0 = 2 * (blockIdx.x * PPB + pair);
-  x.valid = e0 < Ne;
-  x.both = e0 + 1 < Ne;
-  x.nxy = op.NeX * op.NeY;
-  x.i = x.p % N1;
-  x.j = (x.p / N1) % N1;
-  x.k = x.p / NF;
-#pragma unroll
-  for (int m = 0; m < 2; ++m) {
-    x.e[m] = x.valid ? (x.both ? e0 + m : e0) : 0;
-    x.ez[m] = x.e[m] / x.nxy;
-    x.ey[m] = (x.e[m] - x.ez[m] * x.nxy) / op.NeX;
-    x.ex[m] = x.e[m] - x.ez[m] * x.nxy - x.ey[m] * op.NeX;
-  }
-  return x;
-}
-// the neighbour across face dir (0 x, 1 y, 2 z) on the lower (up = 0) or upper side; -1 at a lid
-__device__ __forceinline__ int nd_nbr(const NdOpsP& op, const NdIdx& x, int m, int dir, int up) {
-  const int e = x.e[m];
-  if (dir == 0) return up ? (x.ex[m] < op.NeX - 1 ? e + 1 : e - (op.NeX - 1)) : (x.ex[m] > 0 ? e - 1 : e + op.NeX - 1);
-  if (dir == 1)
-    return up ? (x.ey[m] < op.NeY - 1 ? e + op.NeX : e - (op.NeY - 1) * op.NeX)
-              : (x.ey[m] > 0 ? e - op.NeX : e + (op.NeY - 1) * op.NeX);
-  return up ? (x.ez[m] < op.NeZ - 1 ? e + x.nxy : -1) : (x.ez[m] > 0 ? e - x.nxy : -1);
-}
-// node (i, j, k) of face node ab on side `s` (0 lower, 1 upper) of direction dir
-template <int N1>
-__device__ __forceinline__ void nd_face_node(int dir, int s, int ab, int& i, int& row) {
-  const int a = ab % N1, b = ab / N1, w = s * (N1 - 1);
-  i = dir == 0 ? w : a;
-  row = dir == 0 ? a + N1 * b : (dir == 1 ? w + N1 * b : b + N1 * w);
 }
 
 // a field read either as FP64 (the prognostic variable) or as pairs (an intermediate)
@@ -135,11 +78,11 @@ __device__ __forceinline__ void nd_dir(p2 (&r)[NPT], const NdTab<N1>& T, p2 E, c
   for (int l = 0; l < N1; ++l) {
     p2 d, v;
     if (dir < 2) d = ld(T.D[l * N1 + row]);
-    else v = ld(u[nd_at<N1>(i, j + N1 * l)]);
+    else v = ld(u[two_at<N1>(i, j + N1 * l)]);
 #pragma unroll
     for (int h = 0; h < NPT; ++h) {
       const int kh = k + h * KH;
-      if (dir < 2) v = ld(u[dir == 0 ? nd_at<N1>(l, j + N1 * kh) : nd_at<N1>(i, l + N1 * kh)]);
+      if (dir < 2) v = ld(u[dir == 0 ? two_at<N1>(l, j + N1 * kh) : two_at<N1>(i, l + N1 * kh)]);
       else d = ld(T.D[l * N1 + kh]);
       s[h].add(d, v);
     }
@@ -158,7 +101,7 @@ __device__ __forceinline__ void nd_dir(p2 (&r)[NPT], const NdTab<N1>& T, p2 E, c
 // routine's exterior of Vv (when bc_v), which leaves a jump only for the wall-normal momentum.
 // ONE: Vh and Vv are the same field.
 template <int N1, int PPB, int NPT, bool ONE>
-__global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, nd_minb(PPB * N1 * N1 * N1 / NPT))
+__global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, two_minb(PPB * N1 * N1 * N1 / NPT, 1536))
     k_nd_grad_p(const __grid_constant__ NdOpsP op, const double* __restrict__ dens_prof, const Src Vh, const Src Vv,
                 const double* __restrict__ ddens, int dens_div, int refl, float2* __restrict__ Gx,
                 float2* __restrict__ Gy, float2* __restrict__ Gz, int Ne) {
@@ -166,7 +109,7 @@ __global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, nd_minb(PPB * N1 * N1 *
   extern __shared__ p2m smp[];
   NdTab<N1>& T = *reinterpret_cast<NdTab<N1>*>(smp);
   int pair;
-  const NdIdx x = nd_idx<N1, PPB, NT>(op, Ne, pair);
+  const TwoIdx x = two_idx<N1, PPB, NT>(op, Ne, pair);
   p2m* vh = smp + sizeof(NdTab<N1>) / sizeof(p2m) + pair * ((ONE ? 1 : 2) * Np + 4 * NF);
   p2m* vv = ONE ? vh : vh + Np;
   p2m* df = vv + Np;
@@ -183,7 +126,7 @@ __global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, nd_minb(PPB * N1 * N1 *
         a = a * rd;
         if (!ONE) b = b * rd;
       }
-      const int at = nd_at<N1>(x.i, x.j + N1 * (x.k + h * KH));
+      const int at = two_at<N1>(x.i, x.j + N1 * (x.k + h * KH));
       st(vh[at], a);
       if (!ONE) st(vv[at], b);
     }
@@ -193,12 +136,12 @@ __global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, nd_minb(PPB * N1 * N1 *
     for (int fi = x.p; fi < 3 * NF; fi += NT) {
       const int dir = fi / NF, ab = fi - dir * NF;
       int iP, rP;
-      nd_face_node<N1>(dir, 1, ab, iP, rP);
+      two_face_node<N1>(dir, 1, ab, iP, rP);
       size_t gP[2];
       int lev[2];
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
-        const int kn = nd_nbr(op, x, m, dir, 0);
+        const int kn = two_nbr(op, x, m, dir, 0);
         gP[m] = (size_t)(kn < 0 ? x.e[m] : kn) * Np + rP * N1 + iP;
         lev[m] = (dir == 2 && kn >= 0 ? x.ez[m] - 1 : x.ez[m]) * N1 + rP / N1;
       }
@@ -214,8 +157,8 @@ __global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, nd_minb(PPB * N1 * N1 *
     for (int fi = x.p; fi < (top ? 4 : 3) * NF; fi += NT) {
       const int f = fi / NF, ab = fi - f * NF, dir = f < 2 ? f : 2;
       int iM, rM;
-      nd_face_node<N1>(dir, f == 3, ab, iM, rM);
-      const p2 own = ld((dir == 2 ? vv : vh)[nd_at<N1>(iM, rM)]);
+      two_face_node<N1>(dir, f == 3, ab, iM, rM);
+      const p2 own = ld((dir == 2 ? vv : vh)[two_at<N1>(iM, rM)]);
       const int lz = f == 3 ? op.NeZ - 1 : 0;  // lid layer; -2 v there against the coefficient's 1/2
       const bool la = f >= 2 && x.ez[0] == lz, lb = f >= 2 && x.ez[1] == lz;
       p2 d = f == 3 ? p2_zero() : ld(df[fi]) - own;
@@ -246,7 +189,7 @@ __global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, nd_minb(PPB * N1 * N1 *
 // tables hold dt and the coefficients (the increment in pairs, added to the FP64 field in FP64); else the Laplacian's
 // horizontal and vertical parts.
 template <int N1, int PPB, int NPT, bool TEND>
-__global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, nd_minb(PPB * N1 * N1 * N1 / NPT))
+__global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, two_minb(PPB * N1 * N1 * N1 / NPT, 1536))
     k_nd_div_p(const __grid_constant__ NdOpsP op, const double* __restrict__ dens_prof, const float2* __restrict__ Gx,
                const float2* __restrict__ Gy, const float2* __restrict__ Gz, const double* ddens, int mul_dens, int keep,
                float2* __restrict__ lh, float2* __restrict__ lv, double* V, int Ne) {
@@ -254,7 +197,7 @@ __global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, nd_minb(PPB * N1 * N1 *
   extern __shared__ p2m smp[];
   NdTab<N1>& T = *reinterpret_cast<NdTab<N1>*>(smp);
   int pair;
-  const NdIdx x = nd_idx<N1, PPB, NT>(op, Ne, pair);
+  const TwoIdx x = two_idx<N1, PPB, NT>(op, Ne, pair);
   p2m* fl = smp + sizeof(NdTab<N1>) / sizeof(p2m) + pair * (3 * Np + 4 * NF);
   p2m* df = fl + 3 * Np;
   const size_t g[2] = {(size_t)x.e[0] * Np + x.p, (size_t)x.e[1] * Np + x.p};
@@ -276,7 +219,7 @@ __global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, nd_minb(PPB * N1 * N1 *
         for (int d = 0; d < 3; ++d) v[d] = dens * v[d];
       }
 #pragma unroll
-      for (int d = 0; d < 3; ++d) st(fl[d * Np + nd_at<N1>(x.i, x.j + N1 * (x.k + h * KH))], v[d]);
+      for (int d = 0; d < 3; ++d) st(fl[d * Np + two_at<N1>(x.i, x.j + N1 * (x.k + h * KH))], v[d]);
     }
   }
   const bool bot = !keep && (x.ez[0] == 0 || x.ez[1] == 0);
@@ -284,12 +227,12 @@ __global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, nd_minb(PPB * N1 * N1 *
     for (int fi = x.p; fi < 3 * NF; fi += NT) {
       const int dir = fi / NF, ab = fi - dir * NF;
       int iP, rP;
-      nd_face_node<N1>(dir, 0, ab, iP, rP);
+      two_face_node<N1>(dir, 0, ab, iP, rP);
       size_t gP[2];
       int lev[2];
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
-        const int kn = nd_nbr(op, x, m, dir, 1);
+        const int kn = two_nbr(op, x, m, dir, 1);
         gP[m] = (size_t)(kn < 0 ? x.e[m] : kn) * Np + rP * N1 + iP;
         lev[m] = (dir == 2 && kn >= 0 ? x.ez[m] + 1 : x.ez[m]) * N1 + rP / N1;
       }
@@ -305,8 +248,8 @@ __global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, nd_minb(PPB * N1 * N1 *
     for (int fi = x.p; fi < (bot ? 4 : 3) * NF; fi += NT) {
       const int f = fi / NF, ab = fi - f * NF, dir = f < 2 ? f : 2;
       int iM, rM;
-      nd_face_node<N1>(dir, f != 3, ab, iM, rM);
-      const p2 own = ld(fl[dir * Np + nd_at<N1>(iM, rM)]);
+      two_face_node<N1>(dir, f != 3, ab, iM, rM);
+      const p2 own = ld(fl[dir * Np + two_at<N1>(iM, rM)]);
       const int lz = f == 3 ? 0 : op.NeZ - 1;
       const bool la = f >= 2 && x.ez[0] == lz, lb = f >= 2 && x.ez[1] == lz;
       p2 d = f == 3 ? p2_zero() : ld(df[fi]) - own;
@@ -369,9 +312,9 @@ NdOpsP nd_ops(const Ops& d, const double (&fac)[3], bool lower) {
   return op;
 }
 
-// pairs of elements per block: 108 to 343 threads
+// pairs of elements per block: 108 to 512 threads
 template <int N1>
-constexpr int nd_ppb() { return N1 <= 4 ? (N1 == 2 ? 32 : (N1 == 3 ? 8 : 4)) : 1; }
+constexpr int nd_ppb() { return N1 <= 4 ? (N1 == 2 ? 16 : (N1 == 3 ? 4 : 2)) : 1; }
 
 struct NdPass {
   int pass;  // 0 gradient, 1 Laplacian, 2 update
@@ -382,9 +325,9 @@ struct NdPass {
   double* V;
 };
 
-template <int N1>
+template <int N1, int NPT>
 int nd_pass_n(const NdPass& P, const NdOpsP& op, const double* dp, int Ne, cudaStream_t s) {
-  constexpr int PPB = nd_ppb<N1>(), Np = N1 * N1 * N1, NF = N1 * N1, NPT = N1 % 2 == 0 ? 2 : 1;
+  constexpr int PPB = nd_ppb<N1>(), Np = N1 * N1 * N1, NF = N1 * N1;
   const int grid = ((Ne + 1) / 2 + PPB - 1) / PPB;
   const bool one = P.pass == 0 && P.a.d == P.b.d && P.a.p == P.b.p;
   const size_t sm = sizeof(NdTab<N1>) + sizeof(p2m) * PPB * ((P.pass == 0 ? (one ? 1 : 2) : 3) * Np + 4 * NF);
@@ -403,13 +346,17 @@ int nd_pass_n(const NdPass& P, const NdOpsP& op, const double* dp, int Ne, cudaS
 
 int nd_pass_p(int N1, const NdPass& P, const NdOpsP& op, const double* dp, int Ne, cudaStream_t s) {
   switch (N1) {
-    case 2: return nd_pass_n<2>(P, op, dp, Ne, s);
-    case 3: return nd_pass_n<3>(P, op, dp, Ne, s);
-    case 4: return nd_pass_n<4>(P, op, dp, Ne, s);
-    case 5: return nd_pass_n<5>(P, op, dp, Ne, s);
-    case 6: return nd_pass_n<6>(P, op, dp, Ne, s);
-    case 7: return nd_pass_n<7>(P, op, dp, Ne, s);
-    case 8: return nd_pass_n<8>(P, op, dp, Ne, s);
+    case 2: return nd_pass_n<2, 1>(P, op, dp, Ne, s);
+    case 3: return nd_pass_n<3, 1>(P, op, dp, Ne, s);
+    case 4: return nd_pass_n<4, 1>(P, op, dp, Ne, s);
+    case 5: return nd_pass_n<5, 1>(P, op, dp, Ne, s);
+    case 6: return nd_pass_n<6, 1>(P, op, dp, Ne, s);
+    case 7: return nd_pass_n<7, 1>(P, op, dp, Ne, s);
+    case 8:
+      // Two nodes per thread once the pairs are more than the SMs hold as three blocks of 512 threads.  Gradient +
+      // divergence in us, one / two nodes: 20 pairs 16.8 / 21.5, 320 pairs 28.6 / 30.4, 640 pairs
+      // 44.5 / 40.8, 1280 pairs 73 / 64.  At p = 3 one node is as good at 10,240 pairs (59) and better at 162 (13 / 20).
+      return (Ne + 1) / 2 > 3 * 152 ? nd_pass_n<8, 2>(P, op, dp, Ne, s) : nd_pass_n<8, 1>(P, op, dp, Ne, s);
   }
   return (int)cudaErrorInvalidValue;
 }

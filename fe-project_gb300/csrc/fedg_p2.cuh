@@ -116,6 +116,12 @@ __device__ __forceinline__ p2 p2_recip(p2 d) {
   return p2_fast_two_sum(y, xmul(y, e));
 }
 __device__ __forceinline__ p2 p2_split(double a, double b) { return p2_of(f2_split(a), f2_split(b)); }
+// the same normalised (h the nearest float; f2_split truncates), for values that enter reciprocals and products
+// whose l l term is dropped
+__device__ __forceinline__ p2 p2_split_n(double a, double b) {
+  const p2 v = p2_split(a, b);
+  return p2_fast_two_sum(v.h, v.l);
+}
 
 // compensated dot-product accumulator (f2acc)
 struct p2acc {

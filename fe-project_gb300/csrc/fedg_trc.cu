@@ -16,6 +16,7 @@
 // face-node arrays (NfpTot, Ne) with face f = 0..5 (y-, x+, y+, x-, z-, z+) and face node a + N1*b.
 // Exterior values: the periodic neighbour's node, or at a slip lid the element's own node with the
 // vertical mass flux reflected (FElib's halo copy + ApplyBC on the mass flux).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -786,7 +787,8 @@ int fedg_trc_update(fedg_ctx* c, double* QTRC, const double* const mflx[3], cons
   const double cn[3] = {0.0, 1.0, 0.5};
   const size_t n = c->n;
   if (!c->trc_buf) {
-    if (cudaMalloc(&c->trc_buf, sizeof(double) * (4 * n + (size_t)c->Ne)) != cudaSuccess) {
+    const size_t nfp = (size_t)6 * c->N1 * c->N1 * c->Ne;  // the float-pair path's face fluxes, in place of two fields
+    if (cudaMalloc(&c->trc_buf, sizeof(double) * (2 * n + std::max(2 * n, nfp) + 2 * (size_t)c->Ne)) != cudaSuccess) {
       c->trc_buf = nullptr;
       return api_fail("fedg_trc_update: out of device memory (4 tracer fields of scratch)");
     }

@@ -13,6 +13,7 @@ pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not have_gpu(), reason="needs 
 from fedg import cases  # noqa: E402
 from fedg import lib as fl  # noqa: E402
 from test_gpu_nd import VARS, setup  # noqa: E402
+from test_gpu_trc import setup as setup_trc, t1  # noqa: E402
 
 
 @pytest.mark.parametrize("porder", [1, 2, 3, 4, 5, 6, 7])
@@ -28,3 +29,29 @@ def test_numdiff_pair(porder, ne, nlap):
         dref = ref[v] - q[v]
         err = np.max(np.abs((qd[v].cpu().numpy() - q[v]) - dref)) / max(np.max(np.abs(dref)), 1e-300)
         assert err < 1e-10, (VARS[v], err)
+
+
+@pytest.mark.parametrize("porder", [1, 2, 3, 4, 5, 6, 7])
+@pytest.mark.parametrize("ne", [(1, 1, 1), (3, 1, 3), (1, 3, 5)])
+@pytest.mark.parametrize("limiter", [True, False])
+def test_tracer_pair(porder, ne, limiter):
+    """Two tracer steps with a source, distinct densities and (limiter) the filter, against the FP64 oracle, with
+    the float-pair tests' 1e-11 relative L2."""
+    case = t1(ne, porder)
+    o, ctx, q, b, _ = setup_trc(case, seed=60 + porder, wobble=0.3)
+    rng = np.random.default_rng(61)
+    Q = 1.0 + rng.random(o.shape)
+    mf = [q[1], q[2], q[3]]
+    aM, aP = o.trc_alphdens_advtest(q[0], q[1], q[2], q[3])
+    dd = [q[0] + s * b["dens_hyd"] * rng.standard_normal(o.shape) for s in (1e-4, 2e-4)]
+    rhoq = 1e-5 * rng.random(o.shape)
+    filt = dict(etac_h=2.0 / 3.0, alpha_h=36.0, ord_h=16, etac_v=0.5, alpha_v=30.0, ord_v=12) if limiter else None
+    dt = 0.05 * case.dt
+    ref = o.trc_step(Q, mf, aM, aP, dd[0], q[0], dt, nsteps=2, ddens=dd[1], rhoq_tp=rhoq, limiter=limiter, tmar=True,
+                     filter=filt)
+    Qd = ctx.tensor(Q)
+    ctx.trc_update(Qd, [ctx.tensor(m) for m in mf], ctx.tensor(aM), ctx.tensor(aP), ctx.tensor(dd[0]), ctx.tensor(q[0]), dt,
+                   nsteps=2, ddens=ctx.tensor(dd[1]), rhoq_tp=ctx.tensor(rhoq), limiter=limiter, tmar=True, filter=filt,
+                   prec=fl.PREC_PAIR)
+    got = Qd.cpu().numpy()
+    assert np.linalg.norm(got - ref) < 1e-11 * np.linalg.norm(ref)
