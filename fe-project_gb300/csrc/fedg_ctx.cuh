@@ -38,7 +38,7 @@ struct fedg_ctx {
   double* host_state = nullptr;   // device copy of the state of fedg_update_host (5 Np*Ne doubles)
   cudaStream_t copy_stream = nullptr;  // fedg_update_host's H2D copies, in z-ranges
   cudaEvent_t chunk_ev[4] = {};        // one per z-range: the range has arrived
-  double* trc_buf = nullptr;      // tracer update scratch: two stage fields, var0 and varTmp (or face fluxes), FCT per element
+  double* trc_buf = nullptr;      // tracer update scratch: two stage fields, face fluxes, FCT and face signs per element
   double* nd_buf = nullptr;       // numerical-diffusion scratch: gradient (3 fields), Laplacian (2 fields)
   double* sponge_coef = nullptr;  // sponge-layer coefficient per level
   double sponge_key[2] = {-1.0, -1.0};  // (tau, height) of the uploaded profile

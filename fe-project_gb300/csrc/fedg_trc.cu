@@ -41,21 +41,24 @@ struct TrcFct {          // calc_fct_coef
   double dt;             // dt * gam(s+1,s) / sig(s+1,s)
   double* fct_elem;      // [Ne] or NULL
   double* fct_node;      // (Np, Ne) or NULL
+  double* nf;            // with fct_elem: the face fluxes (NfpTot, Ne) and per element the signs of the face integrals
+  unsigned* sgn;         // (bit f: negative), for the stage kernel
 };
 
 struct TrcStage {        // cal_tend + Advance_trcvar (+ last-stage filter, TMAR and rescale)
-  const double* fct_elem;   // per-element coefficient (fused update) or NULL
+  const double* fct_elem;   // per-element coefficient (fused update) with TrcFct's nf and sgn, or NULL
+  const double* nf;
+  const unsigned* sgn;
   const double* fct_node;   // nodal coefficient field (FElib's fct_coef) or NULL; both NULL: 1
   double* tend;             // (Np, Ne) tendency output or NULL
   int advance;              // 0: tendency only
-  int first, last, acc;     // first stage (store var0), last stage, varTmp accumulation active
-  double sig_ss, gam_ss, sig_Ns, gam_Ns, c_ssm1, c_ss;  // gam_* include dt
+  int first, last;
+  int h_ssm1, h_ss;         // twice the time fraction of the stage's density and of the next one's
+  double sig_ss, gam_ss, sig_N1;  // gam_ss includes dt; sig_N1: the last stage's weight of q^n dens^n
   double* q_out;            // next stage's mixing ratio (not the last stage)
-  double* var0;             // q^n * dens^n
-  double* vtmp;             // varTmp
   int filter, tmar;         // last stage
   const double* ddens_fin;  // DDENS of the dynamics (final rescale); NULL: DDENS_TRC
-  double* qtrc_out;         // last stage: QTRC
+  double* qtrc;             // QTRC: q^n until the last stage writes it
 };
 
 struct TrcFilt {
@@ -84,41 +87,73 @@ __device__ __forceinline__ double trc_numflux(double qM, double qP, double mfM, 
   return __dmul_rn(0.5, __dadd_rn(__dsub_rn(s, __dmul_rn(aP, qP)), __dmul_rn(aM, qM)));
 }
 
-// sum of v over the Np threads of element le of the block, in a fixed order
-template <int N1, int EPB>
-__device__ __forceinline__ double elem_sum(double v, double* s_red, int le, int p) {
-  constexpr int Np = N1 * N1 * N1;
+// sums of v[c] over the Np threads of each element of the block, in a fixed order, into s_red[c EPB + le]; few
+// threads add up the warps' parts (every FP64 instruction takes its warp 16 cycles of the SM's pipe).  s_red: C EPB
+// (Np + 1) doubles.  Begins with a barrier; the caller synchronises.
+template <int N1, int EPB, int C>
+__device__ __forceinline__ void elem_sums(double (&v)[C], double* s_red, int le, int p) {
+  constexpr int Np = N1 * N1 * N1, NW = Np % 32 == 0 ? Np / 32 : Np;
+  double* part = s_red + C * EPB;
+  const int tid = threadIdx.x;
   __syncthreads();
   if constexpr (Np % 32 == 0) {
-    constexpr int NW = Np / 32;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((p & 31) == 0) s_red[le * NW + (p >> 5)] = v;
-    __syncthreads();
-    double s = 0.0;
+    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-    for (int w = 0; w < NW; ++w) s += s_red[le * NW + w];
-    return s;
-  } else {
-    s_red[le * Np + p] = v;
-    __syncthreads();
+      for (int c = 0; c < C; ++c) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
+  }
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    if (Np % 32 != 0) part[(c * EPB + le) * NW + p] = v[c];
+    else if ((p & 31) == 0) part[(c * EPB + le) * NW + (p >> 5)] = v[c];
+  }
+  __syncthreads();
+  if constexpr (NW > 8 && EPB == 1) {  // the first warp
+    if (tid < 32) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        double s = 0.0;
+        for (int w = tid; w < NW; w += 32) s += part[c * NW + w];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (tid == 0) s_red[c] = s;
+      }
+    }
+  } else if (tid < C * EPB) {
     double s = 0.0;
-    for (int q = 0; q < Np; ++q) s += s_red[le * Np + q];
-    return s;
+    for (int w = 0; w < NW; ++w) s += part[tid * NW + w];
+    s_red[tid] = s;
+  }
+}
+
+// FaceIntMat row f of the integrands sf[le][6 NF] in face-node order, into s_out[8 le + f]: consecutive threads of the
+// block
+template <int N1, int EPB>
+__device__ __forceinline__ void face_sums(const double* s_face, double* s_out) {
+  constexpr int NF = N1 * N1;
+  for (int t = threadIdx.x; t < 6 * EPB; t += EPB * N1 * NF) {
+    double s = 0.0;
+    for (int q = 0; q < NF; ++q) s = __dadd_rn(s, s_face[t * NF + q]);
+    s_out[t / 6 * 8 + t % 6] = s;
   }
 }
 
 // ---------------------------------------------------------------------------------------
 // calc_fct_coef: fct = max(0, min(1, Q_e / (sum_f max(0, outflux_f) + 1e-10)))
 // ---------------------------------------------------------------------------------------
+//
+// What bounds it: the FP64 pipe at p = 7 (16x16x8 elements 69 us), latency at p = 3 (20x20x5 elements 32 -> 17 us: the
+// quotient, the face sums and the sum over the warps by a few threads for all elements of the block instead
+// of by every warp).
 template <int N1, int EPB>
 __global__ void __launch_bounds__(EPB* N1* N1* N1)
-    k_trc_fct(const Ops op, const double* __restrict__ dens_prof, const TrcIn in, const TrcFct fc, int Ne) {
+    k_trc_fct(const __grid_constant__ Ops op, const double* __restrict__ dens_prof, const TrcIn in, const TrcFct fc,
+              const double3 JF3, double rdt, int Ne) {
   constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
   extern __shared__ double sm[];
   double* s_face = sm;                    // [EPB][6 NF] weighted face integrands
-  double* s_out = s_face + EPB * 6 * NF;  // [EPB][6]
-  double* s_red = s_out + EPB * 8;        // reduction scratch [EPB][Np]
+  double* s_out = s_face + EPB * 6 * NF;  // [EPB][8]
+  double* s_red = s_out + EPB * 8;        // reduction scratch [EPB][Np + 1]
   const int tid = threadIdx.x, le = tid / Np, p = tid - le * Np;
   const long ke = (long)blockIdx.x * EPB + le;
   const bool valid = ke < Ne;
@@ -140,33 +175,41 @@ __global__ void __launch_bounds__(EPB* N1* N1* N1)
       const double mfP = normal_comp(f, in.mf[0], in.mf[1], in.mf[2], gP, kn < 0);
       const size_t fa = (size_t)ke * 6 * NF + fi;
       const double nf = trc_numflux(__ldg(in.Q + gM), __ldg(in.Q + gP), mfM, mfP, __ldg(in.aM + fa), __ldg(in.aP + fa));
-      const double JF = J * (f >= 4 ? op.FSz : ((f & 1) ? op.FSx : op.FSy));
+      const double JF = f >= 4 ? JF3.z : ((f & 1) ? JF3.x : JF3.y);
+      if (fc.nf) fc.nf[fa] = nf;
       sf[fi] = __dmul_rn(__dmul_rn(op.w[a], op.w[b]), __dmul_rn(JF, nf));
     }
   }
-  // element integral of dens_ssm1 q / dt + RHOQ_tp with the LGL weights
-  double v = 0.0;
+  // element integral of dens_ssm1 q / dt + RHOQ_tp with the LGL weights (J after the sum)
+  double v[1] = {0.0};
   if (valid) {
     const size_t g = (size_t)ke * Np + p;
     const int i = p % N1, j = (p / N1) % N1, k = p / NF;
-    const double dens = __ldg(dens_prof + ez * N1 + k) + (1.0 - fc.c_ssm1) * __ldg(in.ddens0 + g) +
-                        fc.c_ssm1 * __ldg(in.ddens + g);
-    v = J * (op.w[i] * op.w[j] * op.w[k]) * (dens * __ldg(in.Q + g) / fc.dt + (in.rhoq ? __ldg(in.rhoq + g) : 0.0));
+    const double dens = fma(fc.c_ssm1, __ldg(in.ddens + g), fma(1.0 - fc.c_ssm1, __ldg(in.ddens0 + g), __ldg(dens_prof + ez * N1 + k)));
+    const double m = dens * __ldg(in.Q + g);
+    v[0] = (op.w[i] * op.w[j] * op.w[k]) * (in.rhoq ? fma(m, rdt, __ldg(in.rhoq + g)) : m * rdt);
   }
-  const double qe = elem_sum<N1, EPB>(v, s_red, le, p);  // (synchronises: the face integrands are visible)
-  if (valid && p < 6) {  // FaceIntMat row f, in face-node order
-    double s = 0.0;
-    for (int q = 0; q < NF; ++q) s = __dadd_rn(s, sf[p * NF + q]);
-    s_out[le * 8 + p] = s;
-  }
+  elem_sums<N1, EPB, 1>(v, s_red, le, p);  // (begins with a barrier: the face integrands are visible)
+  face_sums<N1, EPB>(s_face, s_out);
   __syncthreads();
-  if (valid) {
+  if (tid < EPB && (long)blockIdx.x * EPB + tid < Ne) {
+    const long e = (long)blockIdx.x * EPB + tid;
     double net = 0.0;
+    unsigned sg = 0;
 #pragma unroll
-    for (int f = 0; f < 6; ++f) net += fmax(0.0, s_out[le * 8 + f]);
-    const double r = fmax(0.0, fmin(1.0, qe / (net + 1.0e-10)));
-    if (fc.fct_elem && p == 0) fc.fct_elem[ke] = r;
-    if (fc.fct_node) fc.fct_node[(size_t)ke * Np + p] = r;
+    for (int f = 0; f < 6; ++f) {
+      const double o = s_out[tid * 8 + f];
+      net += fmax(0.0, o);
+      sg |= (unsigned)(signbit(o) != 0) << f;
+    }
+    const double r = fmax(0.0, fmin(1.0, J * s_red[tid] / (net + 1.0e-10)));
+    if (fc.fct_elem) fc.fct_elem[e] = r;
+    if (fc.sgn) fc.sgn[e] = sg;
+    s_out[tid * 8] = r;
+  }
+  if (fc.fct_node) {
+    __syncthreads();
+    if (valid) fc.fct_node[(size_t)ke * Np + p] = s_out[le * 8];
   }
 }
 
@@ -202,11 +245,15 @@ __device__ __forceinline__ double trc_post(const Ops& op, const TrcFilt& tf, dou
   }
   if (tmar) {
     const double J = op.Jac;
-    const double wd = valid ? J * (op.w[i] * op.w[j] * op.w[k]) * wgt : 0.0;
+    const double wd = valid ? op.w[i] * op.w[j] * op.w[k] * wgt : 0.0;
     const double qp = fmax(0.0, qn);
-    const double q0 = elem_sum<N1, EPB>(wd * qn, s_red, le, p);
-    const double q1 = elem_sum<N1, EPB>(wd * qp, s_red, le, p);
-    qn = q0 / (q1 + 1.0e-32) * qp;
+    double v[2] = {wd * qn, wd * qp};
+    elem_sums<N1, EPB, 2>(v, s_red, le, p);
+    __syncthreads();
+    const int tid = threadIdx.x;
+    if (tid < EPB) s_red[tid] = J * s_red[tid] / (J * s_red[EPB + tid] + 1.0e-32);
+    __syncthreads();
+    qn = s_red[le] * qp;
   }
   return qn;
 }
@@ -214,21 +261,27 @@ __device__ __forceinline__ double trc_post(const Ops& op, const TrcFilt& tf, dou
 // ---------------------------------------------------------------------------------------
 // cal_tend (FCT-limited del_flux, Div, Lift) and the low-storage tracer RK advance
 // ---------------------------------------------------------------------------------------
-template <int N1, int EPB>
+//
+// With the fused update's limiter (LIM) the face fluxes and the signs of their integrals come from k_trc_fct; otherwise
+// they are formed here, the integrals only for a nodal coefficient.  q^n dens^n and varTmp (q^n dens^n / 3 in
+// SSP-RK3) come from QTRC, which the last stage overwrites.  Metric factors are in each block's tables.
+//
+// What bounds it: the FP64 pipe (about 57 instructions per node; 16x16x8 elements at p = 7 122 us, 104 at the pipe's
+// rate).  20x20x5 elements at p = 3: 37-46 -> 20-27 us.
+template <int N1, int EPB, bool LIM>
 __global__ void __launch_bounds__(EPB* N1* N1* N1)
-    k_trc_stage(const Ops op, const double* __restrict__ dens_prof, const TrcIn in, const TrcStage st,
-                const TrcFilt tf, int Ne) {
+    k_trc_stage(const __grid_constant__ Ops op, const double* __restrict__ dens_prof, const TrcIn in, const TrcStage st,
+                const __grid_constant__ TrcFilt tf, int Ne) {
   constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
   extern __shared__ double sm[];
-  double* s_fl = sm;                       // [EPB][3][Np] volume fluxes MFLX_d q
-  double* s_nf = s_fl + EPB * 3 * Np;      // [EPB][6NF] numflux
-  double* s_qm = s_nf + EPB * 6 * NF;      // [EPB][6NF] q- MomFlx-
-  double* s_rm = s_qm + EPB * 6 * NF;      // [EPB][6NF] R-
-  double* s_rp = s_rm + EPB * 6 * NF;      // [EPB][6NF] R+
-  double* s_face = s_rp + EPB * 6 * NF;    // [EPB][6NF] weighted integrands; del_flux afterwards
+  double* s_d = sm;                        // [3][NF] -Escale D
+  double* s_l = s_d + 3 * NF;              // [6][N1] -Fscale Lift of face f
+  double* s_fl = s_l + 6 * N1;             // [EPB][3][Np] volume fluxes MFLX_d q
+  double* s_df = s_fl + EPB * 3 * Np;      // [EPB][6NF] numflux R, then del_flux / Fscale
+  double* s_face = s_df + EPB * 6 * NF;    // [EPB][6NF] weighted integrands (nodal coefficient)
   double* s_out = s_face + EPB * 6 * NF;   // [EPB][8]
-  double* s_red = s_out + EPB * 8;         // [EPB][Np]
-  double* s_b = s_red + EPB * Np;          // [EPB][Np] (filter)
+  double* s_red = s_out + EPB * 8;         // [EPB][2 (Np + 1)]
+  double* s_b = s_red + 2 * EPB * (Np + 1);  // [EPB][Np] (filter)
   const int tid = threadIdx.x, le = tid / Np, p = tid - le * Np;
   const long ke = (long)blockIdx.x * EPB + le;
   const bool valid = ke < Ne;
@@ -237,77 +290,88 @@ __global__ void __launch_bounds__(EPB* N1* N1* N1)
   const int ez = valid ? (int)(ke / nxy) : 0;
   const int ey = valid ? (int)((ke - (long)ez * nxy) / op.NeX) : 0;
   const int ex = valid ? (int)(ke - (long)ez * nxy - (long)ey * op.NeX) : 0;
-  const double J = op.Jac;
   const size_t g = (size_t)ke * Np + p;
   double* fl = s_fl + le * 3 * Np;
-  double* nfv = s_nf + le * 6 * NF;
-  double* qmv = s_qm + le * 6 * NF;
-  double* rmv = s_rm + le * 6 * NF;
-  double* rpv = s_rp + le * 6 * NF;
-  double* sf = s_face + le * 6 * NF;
-
-  const double q = valid ? __ldg(in.Q + g) : 0.0;
-  fl[p] = valid ? __ldg(in.mf[0] + g) * q : 0.0;
-  fl[Np + p] = valid ? __ldg(in.mf[1] + g) * q : 0.0;
-  fl[2 * Np + p] = valid ? __ldg(in.mf[2] + g) * q : 0.0;
+  double* df = s_df + le * 6 * NF;
+  for (int c = tid; c < NF; c += EPB * Np) {
+    s_d[c] = -op.E11 * op.D[c];
+    s_d[NF + c] = -op.E22 * op.D[c];
+    s_d[2 * NF + c] = -op.E33 * op.D[c];
+    if (c < N1) {
+      s_l[c] = -op.FSy * op.Lb[c];
+      s_l[N1 + c] = -op.FSx * op.Lt[c];
+      s_l[2 * N1 + c] = -op.FSy * op.Lt[c];
+      s_l[3 * N1 + c] = -op.FSx * op.Lb[c];
+      s_l[4 * N1 + c] = -op.FSz * op.Lb[c];
+      s_l[5 * N1 + c] = -op.FSz * op.Lt[c];
+    }
+  }
+  double q = 0.0;
   if (valid) {
-    const double own = st.fct_elem ? __ldg(st.fct_elem + ke) : 1.0;
+    q = __ldg(in.Q + g);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) fl[d * Np + p] = __ldg(in.mf[d] + g) * q;
+    const double own = LIM ? __ldg(st.fct_elem + ke) : 1.0;
+    const unsigned sg = LIM ? __ldg(st.sgn + ke) : 0u;
     for (int fi = p; fi < 6 * NF; fi += Np) {
       const int f = fi / NF, ab = fi - f * NF, a = ab % N1, b = ab / N1;
       int pM;
       size_t gP;
       long kn;
       face_exterior<N1>(op, f, a, b, ke, ex, ey, ez, nxy, pM, gP, kn);
-      const size_t gM = (size_t)ke * Np + pM;
-      const double mfM = normal_comp(f, in.mf[0], in.mf[1], in.mf[2], gM);
-      const double mfP = normal_comp(f, in.mf[0], in.mf[1], in.mf[2], gP, kn < 0);
       const size_t fa = (size_t)ke * 6 * NF + fi;
-      const double qM = __ldg(in.Q + gM);
-      const double nf = trc_numflux(qM, __ldg(in.Q + gP), mfM, mfP, __ldg(in.aM + fa), __ldg(in.aP + fa));
-      const double JF = J * (f >= 4 ? op.FSz : ((f & 1) ? op.FSx : op.FSy));
-      nfv[fi] = nf;
-      qmv[fi] = qM * mfM;
-      if (st.fct_node) {
-        rmv[fi] = __ldg(st.fct_node + gM);
-        rpv[fi] = __ldg(st.fct_node + gP);
+      if (LIM) {  // numflux 0.5 (R+ + R- - (R+ - R-) sign(1, outflux_f))
+        const double R = (sg >> f & 1) && kn >= 0 ? __ldg(st.fct_elem + kn) : own;
+        df[fi] = __ldg(st.nf + fa) * R;
       } else {
-        rmv[fi] = own;
-        rpv[fi] = st.fct_elem ? (kn >= 0 ? __ldg(st.fct_elem + kn) : own) : 1.0;
+        const size_t gM = (size_t)ke * Np + pM;
+        const double mfM = normal_comp(f, in.mf[0], in.mf[1], in.mf[2], gM);
+        const double mfP = normal_comp(f, in.mf[0], in.mf[1], in.mf[2], gP, kn < 0);
+        const double nf = trc_numflux(__ldg(in.Q + gM), __ldg(in.Q + gP), mfM, mfP, __ldg(in.aM + fa), __ldg(in.aP + fa));
+        df[fi] = nf;
+        if (st.fct_node) {
+          const double JF = op.Jac * (f >= 4 ? op.FSz : ((f & 1) ? op.FSx : op.FSy));
+          s_face[le * 6 * NF + fi] = __dmul_rn(__dmul_rn(op.w[a], op.w[b]), __dmul_rn(JF, nf));
+        }
       }
-      sf[fi] = __dmul_rn(__dmul_rn(op.w[a], op.w[b]), __dmul_rn(JF, nf));
     }
   }
   __syncthreads();
-  if (valid && p < 6) {
-    double s = 0.0;
-    for (int qq = 0; qq < NF; ++qq) s = __dadd_rn(s, sf[p * NF + qq]);
-    s_out[le * 8 + p] = s;
+  if (!LIM && st.fct_node) {
+    face_sums<N1, EPB>(s_face, s_out);
+    __syncthreads();
   }
-  __syncthreads();
-  if (valid) {  // del_flux = Fscale (numflux 0.5 (R+ + R- - (R+ - R-) sign(1, outflux_f)) - q- MomFlx-)
+  if (valid) {  // numflux R - q- MomFlx-
     for (int fi = p; fi < 6 * NF; fi += Np) {
-      const int f = fi / NF;
-      const double sg = signbit(s_out[le * 8 + f]) ? -1.0 : 1.0;
-      const double RM = rmv[fi], RP = rpv[fi];
-      const double fs = f >= 4 ? op.FSz : ((f & 1) ? op.FSx : op.FSy);
-      sf[fi] = fs * (nfv[fi] * (0.5 * (RP + RM - (RP - RM) * sg)) - qmv[fi]);
+      const int f = fi / NF, ab = fi - f * NF, a = ab % N1, b = ab / N1;
+      int pM;
+      size_t gP;
+      long kn;
+      face_exterior<N1>(op, f, a, b, ke, ex, ey, ez, nxy, pM, gP, kn);
+      double nf = df[fi];
+      if (!LIM && st.fct_node) nf *= __ldg(st.fct_node + (signbit(s_out[le * 8 + f]) ? gP : (size_t)ke * Np + pM));
+      const double own = fl[(f >= 4 ? 2 : (f & 1 ? 0 : 1)) * Np + pM];
+      df[fi] = (f == 1 || f == 2 || f == 5) ? nf - own : nf + own;
     }
   }
   __syncthreads();
 
   double t = 0.0;
   if (valid) {
-    double sx = 0.0, sy = 0.0, sz = 0.0;
+    if (in.rhoq) t = __ldg(in.rhoq + g);
 #pragma unroll
     for (int l = 0; l < N1; ++l) {
-      sx = fma(op.D[i * N1 + l], fl[l + N1 * j + NF * k], sx);
-      sy = fma(op.D[j * N1 + l], fl[Np + i + N1 * l + NF * k], sy);
-      sz = fma(op.D[k * N1 + l], fl[2 * Np + i + N1 * j + NF * l], sz);
+      t = fma(s_d[i * N1 + l], fl[p - i + l], t);
+      t = fma(s_d[NF + j * N1 + l], fl[Np + p + (l - j) * N1], t);
+      t = fma(s_d[2 * NF + k * N1 + l], fl[2 * Np + p + (l - k) * NF], t);
     }
-    const double lf = op.Lb[j] * sf[0 * NF + i + N1 * k] + op.Lt[i] * sf[1 * NF + j + N1 * k] +
-                      op.Lt[j] * sf[2 * NF + i + N1 * k] + op.Lb[i] * sf[3 * NF + j + N1 * k] +
-                      op.Lb[k] * sf[4 * NF + i + N1 * j] + op.Lt[k] * sf[5 * NF + i + N1 * j];
-    t = -(op.E11 * sx + op.E22 * sy + op.E33 * sz + lf) + (in.rhoq ? __ldg(in.rhoq + g) : 0.0);
+    const int xy = i + N1 * j, xz = i + N1 * k, yz = j + N1 * k;
+    t = fma(s_l[j], df[xz], t);
+    t = fma(s_l[N1 + i], df[NF + yz], t);
+    t = fma(s_l[2 * N1 + j], df[2 * NF + xz], t);
+    t = fma(s_l[3 * N1 + i], df[3 * NF + yz], t);
+    t = fma(s_l[4 * N1 + k], df[4 * NF + xy], t);
+    t = fma(s_l[5 * N1 + k], df[5 * NF + xy], t);
     if (st.tend) st.tend[g] = t;
   }
   if (!st.advance) return;  // uniform across the block
@@ -318,35 +382,18 @@ __global__ void __launch_bounds__(EPB* N1* N1* N1)
     const double dh = __ldg(dens_prof + ez * N1 + k);
     const double dd = __ldg(in.ddens + g), dd0 = __ldg(in.ddens0 + g);
     const double d0 = dh + dd0;
-    const double dssm1 = d0 + st.c_ssm1 * (dd - dd0);
-    if (st.last) {
-      qn = (st.vtmp[g] + st.sig_ss * q * dssm1 + st.gam_ss * t) / (dh + dd);
-    } else {
-      double v0;
-      if (st.first) {
-        v0 = q * d0;
-        st.var0[g] = v0;
-      } else {
-        v0 = st.var0[g];
-      }
-      if (st.acc) {
-        const double vt = (st.first ? 0.0 : st.vtmp[g]) + st.sig_Ns * q * dssm1 + st.gam_Ns * t;
-        st.vtmp[g] = vt;
-      } else if (st.first) {
-        st.vtmp[g] = 0.0;
-      }
-      const double dss = d0 + st.c_ss * (dd - dd0);
-      qn = ((1.0 - st.sig_ss) * v0 + st.sig_ss * q * dssm1 + st.gam_ss * t) / dss;
-      st.q_out[g] = qn;
-    }
-    wgt = dh + dd;
+    auto dens = [&](int h) { return h == 1 ? fma(0.5, dd - dd0, d0) : (h ? dh + dd : d0); };
+    qn = fma(st.sig_ss, q * dens(st.h_ssm1), st.gam_ss * t);
+    if (!st.first) qn = fma(st.last ? st.sig_N1 : 1.0 - st.sig_ss, st.qtrc[g] * d0, qn);
+    wgt = dens(st.last ? 2 : st.h_ss);
+    qn /= wgt;
+    if (!st.last) st.q_out[g] = qn;
   }
   if (!st.last) return;  // uniform across the block
   qn = trc_post<N1, EPB>(op, tf, qn, wgt, st.filter, st.tmar, s_fl, s_b, s_red, le, p, valid);
   if (valid) {
-    const double dh = __ldg(dens_prof + ez * N1 + k);
-    const double ddf = st.ddens_fin ? __ldg(st.ddens_fin + g) : __ldg(in.ddens + g);
-    st.qtrc_out[g] = (dh + __ldg(in.ddens + g)) / (dh + ddf) * qn;
+    if (st.ddens_fin) qn *= wgt / (__ldg(dens_prof + ez * N1 + k) + __ldg(st.ddens_fin + g));
+    st.qtrc[g] = qn;
   }
 }
 
@@ -359,7 +406,7 @@ __global__ void __launch_bounds__(EPB* N1* N1* N1)
   extern __shared__ double sm[];
   double* s_a = sm;
   double* s_b = s_a + EPB * Np;
-  double* s_red = s_b + EPB * Np;
+  double* s_red = s_b + EPB * Np;  // [EPB][2 (Np + 1)]
   const int tid = threadIdx.x, le = tid / Np, p = tid - le * Np;
   const long ke = (long)blockIdx.x * EPB + le;
   const bool valid = ke < Ne;
@@ -524,12 +571,12 @@ constexpr int trc_epb() { return N1 <= 4 ? (N1 <= 2 ? 16 : (N1 == 3 ? 8 : 4)) : 
 template <int N1>
 size_t fct_smem() {
   constexpr int EPB = trc_epb<N1>(), Np = N1 * N1 * N1, NF = N1 * N1;
-  return sizeof(double) * EPB * (6 * NF + 8 + Np);
+  return sizeof(double) * EPB * (6 * NF + 8 + Np + 1);
 }
 template <int N1>
 size_t stage_smem() {
   constexpr int EPB = trc_epb<N1>(), Np = N1 * N1 * N1, NF = N1 * N1;
-  return sizeof(double) * EPB * (3 * Np + 5 * 6 * NF + 8 + 2 * Np);
+  return sizeof(double) * (3 * NF + 6 * N1 + EPB * (3 * Np + 2 * 6 * NF + 8 + 2 * (Np + 1) + Np));
 }
 
 template <int N1>
@@ -538,7 +585,8 @@ int launch_fct_n(const Ops& op, const double* dp, const TrcIn& in, const TrcFct&
   const size_t sm = fct_smem<N1>();
   auto kfn = k_trc_fct<N1, EPB>;
   cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  kfn<<<(Ne + EPB - 1) / EPB, EPB * Np, sm, s>>>(op, dp, in, fc, Ne);
+  kfn<<<(Ne + EPB - 1) / EPB, EPB * Np, sm, s>>>(
+      op, dp, in, fc, make_double3(op.Jac * op.FSx, op.Jac * op.FSy, op.Jac * op.FSz), 1.0 / fc.dt, Ne);
   return (int)cudaGetLastError();
 }
 template <int N1>
@@ -546,7 +594,7 @@ int launch_stage_n(const Ops& op, const double* dp, const TrcIn& in, const TrcSt
                    cudaStream_t s) {
   constexpr int EPB = trc_epb<N1>(), Np = N1 * N1 * N1;
   const size_t sm = stage_smem<N1>();
-  auto kfn = k_trc_stage<N1, EPB>;
+  auto kfn = st.fct_elem ? k_trc_stage<N1, EPB, true> : k_trc_stage<N1, EPB, false>;
   cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   kfn<<<(Ne + EPB - 1) / EPB, EPB * Np, sm, s>>>(op, dp, in, st, tf, Ne);
   return (int)cudaGetLastError();
@@ -555,7 +603,7 @@ template <int N1>
 int launch_post_n(const Ops& op, const double* dp, double* Q, const double* dd, const TrcFilt& tf, int filter, int tmar,
                   int Ne, cudaStream_t s) {
   constexpr int EPB = trc_epb<N1>(), Np = N1 * N1 * N1;
-  const size_t sm = sizeof(double) * EPB * 3 * Np;
+  const size_t sm = sizeof(double) * EPB * (4 * Np + 2);
   k_trc_post<N1, EPB><<<(Ne + EPB - 1) / EPB, EPB * Np, sm, s>>>(op, dp, Q, dd, tf, filter, tmar, Ne);
   return (int)cudaGetLastError();
 }
@@ -726,7 +774,7 @@ int fedg_trc_fct_coef(fedg_ctx* c, const double* QTRC, const double* const mflx[
   if (int r = check_periodic(c, "fedg_trc_fct_coef")) return r;
   cudaSetDevice(c->d.device);
   const TrcIn in{QTRC, {mflx[0], mflx[1], mflx[2]}, alph_M, alph_P, RHOQ_tp, DDENS_TRC, DDENS0_TRC};
-  const TrcFct fc{rk_c_ssm1, dt, nullptr, fct_coef};
+  const TrcFct fc{rk_c_ssm1, dt, nullptr, fct_coef, nullptr, nullptr};
   const int r = tracked(c, FEDG_K_TRC_FCT, [&] { return launch_fct(c->op, c->d_prof, in, fc, c->Ne, c->stream); });
   return r ? api_cuda_fail((cudaError_t)r, "fedg_trc_fct_coef") : 0;
 }
@@ -784,10 +832,10 @@ int fedg_trc_update(fedg_ctx* c, double* QTRC, const double* const mflx[3], cons
   constexpr int ns = 3;
   const double sig[4][3] = {{0, 0, 0}, {1, 0, 0}, {0.75, 0.25, 0}, {1.0 / 3.0, 0, 2.0 / 3.0}};
   const double gam[4][3] = {{0, 0, 0}, {1, 0, 0}, {0, 0.25, 0}, {0, 0, 2.0 / 3.0}};
-  const double cn[3] = {0.0, 1.0, 0.5};
+  const int cn2[3] = {0, 2, 1};  // twice the stage's time fraction
   const size_t n = c->n;
   if (!c->trc_buf) {
-    const size_t nfp = (size_t)6 * c->N1 * c->N1 * c->Ne;  // the float-pair path's face fluxes, in place of two fields
+    const size_t nfp = (size_t)6 * c->N1 * c->N1 * c->Ne;  // the face fluxes (two fields' worth at least)
     if (cudaMalloc(&c->trc_buf, sizeof(double) * (2 * n + std::max(2 * n, nfp) + 2 * (size_t)c->Ne)) != cudaSuccess) {
       c->trc_buf = nullptr;
       return api_fail("fedg_trc_update: out of device memory (4 tracer fields of scratch)");
@@ -797,9 +845,9 @@ int fedg_trc_update(fedg_ctx* c, double* QTRC, const double* const mflx[3], cons
     return trc_update_pair(c, QTRC, mflx, alph_M, alph_P, DDENS_TRC, DDENS0_TRC, DDENS, RHOQ_tp, o, c->trc_buf);
   double* bufA = c->trc_buf;
   double* bufB = bufA + n;
-  double* var0 = bufB + n;
-  double* vtmp = var0 + n;
-  double* fct = vtmp + n;
+  double* nf = bufB + n;
+  double* fct = nf + std::max(2 * n, (size_t)6 * c->N1 * c->N1 * c->Ne);
+  unsigned* sgn = reinterpret_cast<unsigned*>(fct + c->Ne);
   const TrcFilt tf = o->filter ? make_filter(c, o->mf_etac_h, o->mf_alpha_h, o->mf_order_h, o->mf_etac_v,
                                              o->mf_alpha_v, o->mf_order_v)
                                : TrcFilt{};
@@ -810,7 +858,7 @@ int fedg_trc_update(fedg_ctx* c, double* QTRC, const double* const mflx[3], cons
       const TrcIn in{qs, {mflx[0], mflx[1], mflx[2]}, alph_M, alph_P, RHOQ_tp, DDENS_TRC, DDENS0_TRC};
       const double sig_ss = sig[s][s - 1], gam_ss = gam[s][s - 1];
       if (o->limiter) {
-        const TrcFct fc{cn[s - 1], o->dt * gam_ss / sig_ss, fct, nullptr};
+        const TrcFct fc{0.5 * cn2[s - 1], o->dt * gam_ss / sig_ss, fct, nullptr, nf, sgn};
         const int r = tracked(c, FEDG_K_TRC_FCT, [&] { return launch_fct(c->op, c->d_prof, in, fc, c->Ne, c->stream); });
         if (r) return api_cuda_fail((cudaError_t)r, "fedg_trc_update: FCT coefficient");
       }
@@ -820,21 +868,19 @@ int fedg_trc_update(fedg_ctx* c, double* QTRC, const double* const mflx[3], cons
       st.advance = 1;
       st.first = s == 1;
       st.last = s == ns;
-      const double sig_Ns = sig[ns][s - 1], gam_Ns = o->dt * gam[ns][s - 1];
-      st.acc = !st.last && (std::fabs(sig_Ns) > 1.0e-16 || std::fabs(gam_Ns) > 1.0e-16);
+      // varTmp collects the last stage's terms of the earlier stages: here sig(3,1) q^n dens^n alone
+      st.nf = nf;
+      st.sgn = sgn;
       st.sig_ss = sig_ss;
       st.gam_ss = o->dt * gam_ss;
-      st.sig_Ns = sig_Ns;
-      st.gam_Ns = gam_Ns;
-      st.c_ssm1 = cn[s - 1];
-      st.c_ss = s < ns ? cn[s] : 0.0;
+      st.sig_N1 = sig[ns][0];
+      st.h_ssm1 = cn2[s - 1];
+      st.h_ss = s < ns ? cn2[s] : 0;
       st.q_out = qo;
-      st.var0 = var0;
-      st.vtmp = vtmp;
       st.filter = o->filter != 0;
       st.tmar = o->limiter && o->tmar;
       st.ddens_fin = DDENS;
-      st.qtrc_out = QTRC;
+      st.qtrc = QTRC;
       const int r = tracked(c, FEDG_K_TRC_TEND, [&] { return launch_stage(c->op, c->d_prof, in, st, tf, c->Ne, c->stream); });
       if (r) return api_cuda_fail((cudaError_t)r, "fedg_trc_update: stage");
       qs = qo;
