@@ -26,51 +26,13 @@
 namespace fedg {
 namespace {
 
-__device__ __forceinline__ double sgn1(double x) { return signbit(x) ? -1.0 : 1.0; }  // Fortran sign(1, x)
-__device__ __forceinline__ double face_n(int f) { return (f == 1 || f == 2 || f == 5) ? 1.0 : -1.0; }
-__device__ __forceinline__ int face_dir(int f) { return f >= 4 ? 2 : ((f & 1) ? 0 : 1); }
-
-// exterior of a scalar at a lid (even routine): the wall-normal momentum is reflected
-__device__ __forceinline__ double even_ext(int var, int dir, double vM, double n) {
-  const bool refl = (var == VMX && dir == 0) || (var == VMY && dir == 1) || (var == VMZ && dir == 2);
-  if (!refl) return vM;
-  const double g = vM * n;
-  return vM - 2.0 * g * n;
-}
-// exterior normal gradient component at a lid (odd routine): the normal component is reflected for
-// DENS/RHOT (adiabatic) and for the tangential momenta (slip); kept for the wall-normal momentum
-__device__ __forceinline__ double odd_ext_n(int var, int dir, double gMn_comp, double n) {
-  const bool keep = (var == VMX && dir == 0) || (var == VMY && dir == 1) || (var == VMZ && dir == 2);
-  if (keep) return gMn_comp;
-  const double gn = gMn_comp * n;
-  return gMn_comp - 2.0 * gn * n;
-}
-
-template <int N1>
-__device__ __forceinline__ double lift(const Ops& op, const double* fv, int i, int j, int k) {
-  constexpr int NF = N1 * N1;
-  return op.Lb[j] * fv[0 * NF + i + N1 * k] + op.Lt[i] * fv[1 * NF + j + N1 * k] + op.Lt[j] * fv[2 * NF + i + N1 * k] +
-         op.Lb[i] * fv[3 * NF + j + N1 * k] + op.Lb[k] * fv[4 * NF + i + N1 * j] + op.Lt[k] * fv[5 * NF + i + N1 * j];
-}
-// Lift of the faces of one direction only (the others carry zeros)
-template <int N1>
-__device__ __forceinline__ double lift_dir(const Ops& op, const double* fv, int dir, int i, int j, int k) {
-  constexpr int NF = N1 * N1;
-  if (dir == 0) return op.Lt[i] * fv[1 * NF + j + N1 * k] + op.Lb[i] * fv[3 * NF + j + N1 * k];
-  if (dir == 1) return op.Lb[j] * fv[0 * NF + i + N1 * k] + op.Lt[j] * fv[2 * NF + i + N1 * k];
-  return op.Lb[k] * fv[4 * NF + i + N1 * j] + op.Lt[k] * fv[5 * NF + i + N1 * j];
-}
-template <int N1>
-__device__ __forceinline__ double dsum(const Ops& op, const double* u, int dir, int i, int j, int k) {
-  constexpr int NF = N1 * N1;
-  double s = 0.0;
-#pragma unroll
-  for (int l = 0; l < N1; ++l) {
-    const int p = dir == 0 ? l + N1 * j + NF * k : (dir == 1 ? i + N1 * l + NF * k : i + N1 * j + NF * l);
-    s = fma(op.D[(dir == 0 ? i : (dir == 1 ? j : k)) * N1 + l], u[p], s);
-  }
-  return s;
-}
+// Tables of a pass.  An interior face's flux is nonzero only on one of its two sides (the gradient takes the
+// lower neighbour, the divergence the upper), so an element computes three faces, with Lift lf, and a lid face (Lift
+// lo of the fourth) only where the reflection leaves a jump; the signs are in lf and lo.  E of each
+// direction holds the pass's coefficient; Escale and Fscale are the same 2/dx.
+struct NdOps {
+  double E[3], lf[FEDG_MAXN1], lo[FEDG_MAXN1];
+};
 
 struct ElemIdx {
   long ke;
@@ -95,149 +57,147 @@ __device__ __forceinline__ ElemIdx elem_idx(const Ops& op, int Ne) {
   e.ex = e.valid ? (int)(e.ke - (long)e.ez * e.nxy - (long)e.ey * op.NeX) : 0;
   return e;
 }
+// the exterior node of face node ab on the lower (up = 0) or upper face of direction dir, -1 at a lid, and its level
+template <int N1>
+__device__ __forceinline__ long nd_exterior(const Ops& op, const ElemIdx& e, int dir, int up, int ab, int& lev) {
+  constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
+  const int a = ab % N1, b = ab / N1, w = up ? 0 : N1 - 1;
+  long kn = e.ke;
+  if (dir == 0) kn += up ? (e.ex < op.NeX - 1 ? 1 : -(op.NeX - 1)) : (e.ex > 0 ? -1 : op.NeX - 1);
+  else if (dir == 1) kn += up ? (e.ey < op.NeY - 1 ? op.NeX : -(long)(op.NeY - 1) * op.NeX) : (e.ey > 0 ? -op.NeX : (long)(op.NeY - 1) * op.NeX);
+  else {
+    if (up ? e.ez == op.NeZ - 1 : e.ez == 0) return -1;
+    kn += up ? e.nxy : -e.nxy;
+  }
+  lev = dir == 2 ? (e.ez + (up ? 1 : -1)) * N1 + w : e.ez * N1 + b;
+  return kn * Np + (dir == 0 ? w + N1 * ab : (dir == 1 ? a + N1 * w + NF * b : ab + NF * w));
+}
+// the element's own node of face node ab
+template <int N1>
+__device__ __forceinline__ int nd_own(int dir, int up, int ab) {
+  constexpr int NF = N1 * N1;
+  const int a = ab % N1, b = ab / N1, w = up ? N1 - 1 : 0;
+  return dir == 0 ? w + N1 * ab : (dir == 1 ? a + N1 * w + NF * b : ab + NF * w);
+}
+// contraction along direction dir and the Lift of its faces; D: the block's copy of the operator
+template <int N1>
+__device__ __forceinline__ double nd_dir(const NdOps& nd, const double* D, const double* u, const double* df, int dir,
+                                         const ElemIdx& e, bool lid) {
+  constexpr int NF = N1 * N1;
+  const int row = dir == 0 ? e.i : (dir == 1 ? e.j : e.k), stp = dir == 0 ? 1 : (dir == 1 ? N1 : NF);
+  const int ab = dir == 0 ? e.j + N1 * e.k : (dir == 1 ? e.i + N1 * e.k : e.i + N1 * e.j);
+  double s = nd.lf[row] * df[dir * NF + ab];
+  if (dir == 2 && lid) s = fma(nd.lo[row], df[3 * NF + ab], s);
+  u += e.p - row * stp;
+#pragma unroll
+  for (int l = 0; l < N1; ++l) s = fma(D[row * N1 + l], u[l * stp], s);
+  return s;
+}
 
-__device__ __forceinline__ double fscale(const Ops& op, int f) { return f >= 4 ? op.FSz : ((f & 1) ? op.FSx : op.FSy); }
-
-// numdiff_cal_flx: G = (d/dx Vh, d/dy Vh, d/dz Vv) (each divided by the density when dens_div),
-// with the even routine's lid exterior of Vh (and of Vv when bc_v)
+// numdiff_cal_flx: G = (d/dx Vh, d/dy Vh, d/dz Vv) (each divided by the density when dens_div).  refl: at the
+// lids the even routine's exterior of Vv reflects it (the wall-normal momentum); otherwise no jump there.
+//
+// What bounds it: the FP64 pipe, about 47 instructions per node (one reciprocal for the node and one for each computed
+// face node).  16x16x8 elements at p = 7: 128 -> 82 us.
 template <int N1, int EPB>
 __global__ void __launch_bounds__(EPB* N1* N1* N1)
-    k_nd_grad(const Ops op, const double* __restrict__ dens_prof, const double* __restrict__ Vh,
-              const double* __restrict__ Vv, const double* __restrict__ ddens, int var, int dens_div, int bc_v,
-              double* __restrict__ Gx, double* __restrict__ Gy, double* __restrict__ Gz, int Ne) {
+    k_nd_grad(const __grid_constant__ Ops op, const __grid_constant__ NdOps nd, const double* __restrict__ dens_prof,
+              const double* __restrict__ Vh, const double* __restrict__ Vv, const double* __restrict__ ddens, int dens_div,
+              int refl, double* __restrict__ Gx, double* __restrict__ Gy, double* __restrict__ Gz, int Ne) {
   constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
   extern __shared__ double sm[];
   const ElemIdx e = elem_idx<N1, EPB>(op, Ne);
-  double* vh = sm + e.le * (2 * Np + 6 * NF);
-  double* vv = vh + Np;
-  double* df = vv + Np;
+  double* D = sm;
+  double* vh = sm + NF + e.le * (2 * Np + 4 * NF);
+  double* vv = Vh == Vv ? vh : vh + Np;
+  double* df = vh + 2 * Np;
   const size_t g = (size_t)e.ke * Np + e.p;
+  for (int c = threadIdx.x; c < NF; c += EPB * Np) D[c] = op.D[c];
+  const bool top = refl && e.ez == op.NeZ - 1;
   if (e.valid) {
-    const double dens = dens_div ? __ldg(ddens + g) + __ldg(dens_prof + e.ez * N1 + e.k) : 1.0;
-    vh[e.p] = dens_div ? __ldg(Vh + g) / dens : __ldg(Vh + g);
-    vv[e.p] = dens_div ? __ldg(Vv + g) / dens : __ldg(Vv + g);
-    for (int fi = e.p; fi < 6 * NF; fi += Np) {
-      const int f = fi / NF, ab = fi - f * NF, a = ab % N1, b = ab / N1;
-      int pM;
-      size_t gP;
-      long kn;
-      face_exterior<N1>(op, f, a, b, e.ke, e.ex, e.ey, e.ez, e.nxy, pM, gP, kn);
-      const size_t gM = (size_t)e.ke * Np + pM;
-      const int dir = face_dir(f);
-      const double n = face_n(f);
-      double wM = 1.0, wP = 1.0;
-      if (dens_div) {
-        const int levM = e.ez * N1 + pM / NF;
-        const int levP = (kn >= 0 ? (int)(kn / e.nxy) : e.ez) * N1 + (int)((gP % Np) / NF);
-        wP = 1.0 / (__ldg(ddens + gP) + __ldg(dens_prof + levP));
-        wM = 1.0 / (__ldg(ddens + gM) + __ldg(dens_prof + levM));
-      }
-      const bool lid = kn < 0;
-      const double src_M = dir == 2 ? __ldg(Vv + gM) : __ldg(Vh + gM);
-      double src_P = dir == 2 ? __ldg(Vv + gP) : __ldg(Vh + gP);
-      if (lid && (dir != 2 || bc_v)) src_P = even_ext(var, dir, src_M, n);
-      const double d = 0.5 * (src_P * wP - src_M * wM);
-      df[fi] = fscale(op, f) * (lid ? d * n : (1.0 - sgn1(n)) * d * n);
+    const double rd = dens_div ? 1.0 / (__ldg(ddens + g) + __ldg(dens_prof + e.ez * N1 + e.k)) : 1.0;
+    vh[e.p] = dens_div ? __ldg(Vh + g) * rd : __ldg(Vh + g);
+    if (vv != vh) vv[e.p] = dens_div ? __ldg(Vv + g) * rd : __ldg(Vv + g);
+    for (int fi = e.p; fi < 3 * NF; fi += Np) {
+      const int dir = fi / NF;
+      int lev;
+      const long gP = nd_exterior<N1>(op, e, dir, 0, fi - dir * NF, lev);
+      if (gP < 0) continue;
+      const double vP = __ldg((dir == 2 ? Vv : Vh) + gP);
+      df[fi] = dens_div ? vP / (__ldg(ddens + gP) + __ldg(dens_prof + lev)) : vP;
+    }
+  }
+  __syncthreads();
+  if (e.valid) {
+    for (int fi = e.p; fi < (top ? 4 : 3) * NF; fi += Np) {
+      const int f = fi / NF, dir = f < 2 ? f : 2;
+      const double own = (dir == 2 ? vv : vh)[nd_own<N1>(dir, f == 3, fi - f * NF)];
+      if (f == 3 || (f == 2 && e.ez == 0)) df[fi] = refl ? -own : 0.0;  // half of the reflected jump
+      else df[fi] -= own;
     }
   }
   __syncthreads();
   if (!e.valid) return;
-  Gx[g] = op.E11 * dsum<N1>(op, vh, 0, e.i, e.j, e.k) + lift_dir<N1>(op, df, 0, e.i, e.j, e.k);
-  Gy[g] = op.E22 * dsum<N1>(op, vh, 1, e.i, e.j, e.k) + lift_dir<N1>(op, df, 1, e.i, e.j, e.k);
-  Gz[g] = op.E33 * dsum<N1>(op, vv, 2, e.i, e.j, e.k) + lift_dir<N1>(op, df, 2, e.i, e.j, e.k);
+  Gx[g] = nd.E[0] * nd_dir<N1>(nd, D, vh, df, 0, e, false);
+  Gy[g] = nd.E[1] * nd_dir<N1>(nd, D, vh, df, 1, e, false);
+  Gz[g] = nd.E[2] * nd_dir<N1>(nd, D, vv, df, 2, e, top);
 }
 
-// numdiff_cal_laplacian with the odd routine's lid exterior of G: horizontal and vertical parts
-template <int N1, int EPB>
+// divergence of G (times the density when mul_dens).  At the lids the odd routine's exterior of G reflects it, but
+// for the wall-normal momentum (keep: no jump).  TEND: numdiff_tend and V += its sum (nd.E holds dt and the
+// coefficients); otherwise numdiff_cal_laplacian's horizontal and vertical parts.
+//
+// What bounds it: the FP64 pipe, about 38 instructions per node.  16x16x8 elements at p = 7: 102 -> 74 us.
+template <int N1, int EPB, bool TEND>
 __global__ void __launch_bounds__(EPB* N1* N1* N1)
-    k_nd_lap(const Ops op, const double* __restrict__ Gx, const double* __restrict__ Gy,
-             const double* __restrict__ Gz, int var, double* __restrict__ lh, double* __restrict__ lv, int Ne) {
+    k_nd_div(const __grid_constant__ Ops op, const __grid_constant__ NdOps nd, const double* __restrict__ dens_prof,
+             const double* __restrict__ Gx, const double* __restrict__ Gy, const double* __restrict__ Gz,
+             const double* ddens, int mul_dens, int keep, double* __restrict__ lh, double* __restrict__ lv, double* V, int Ne) {
   constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
   extern __shared__ double sm[];
   const ElemIdx e = elem_idx<N1, EPB>(op, Ne);
-  double* gx = sm + e.le * (3 * Np + 6 * NF);
-  double* gy = gx + Np;
-  double* gz = gy + Np;
-  double* df = gz + Np;
+  double* D = sm;
+  double* fl = sm + NF + e.le * (3 * Np + 4 * NF);
+  double* df = fl + 3 * Np;
   const size_t g = (size_t)e.ke * Np + e.p;
-  const double* G[3] = {Gx, Gy, Gz};
-  if (e.valid) {
-    gx[e.p] = __ldg(Gx + g);
-    gy[e.p] = __ldg(Gy + g);
-    gz[e.p] = __ldg(Gz + g);
-    for (int fi = e.p; fi < 6 * NF; fi += Np) {
-      const int f = fi / NF, ab = fi - f * NF, a = ab % N1, b = ab / N1;
-      int pM;
-      size_t gP;
-      long kn;
-      face_exterior<N1>(op, f, a, b, e.ke, e.ex, e.ey, e.ez, e.nxy, pM, gP, kn);
-      const size_t gM = (size_t)e.ke * Np + pM;
-      const int dir = face_dir(f);
-      const double n = face_n(f);
-      const double gMc = __ldg(G[dir] + gM);
-      const bool lid = kn < 0;
-      const double gPc = lid ? odd_ext_n(var, dir, gMc, n) : __ldg(G[dir] + gP);
-      df[fi] = fscale(op, f) * (lid ? 0.5 * (gPc - gMc) * n : 0.5 * (1.0 + sgn1(n)) * (gPc - gMc) * n);
-    }
-  }
-  __syncthreads();
-  if (!e.valid) return;
-  lh[g] = op.E11 * dsum<N1>(op, gx, 0, e.i, e.j, e.k) + op.E22 * dsum<N1>(op, gy, 1, e.i, e.j, e.k) +
-          (lift_dir<N1>(op, df, 1, e.i, e.j, e.k) + lift_dir<N1>(op, df, 0, e.i, e.j, e.k));
-  lv[g] = op.E33 * dsum<N1>(op, gz, 2, e.i, e.j, e.k) + lift_dir<N1>(op, df, 2, e.i, e.j, e.k);
-}
-
-// numdiff_tend with the odd routine's lid exterior of G, then V += dt tend
-template <int N1, int EPB>
-__global__ void __launch_bounds__(EPB* N1* N1* N1)
-    k_nd_tend(const Ops op, const double* __restrict__ dens_prof, const double* __restrict__ Gx,
-              const double* __restrict__ Gy, const double* __restrict__ Gz, const double* ddens, int var,
-              int mul_dens, double ch, double cv, double dt, double* V, int Ne) {
-  constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
-  extern __shared__ double sm[];
-  const ElemIdx e = elem_idx<N1, EPB>(op, Ne);
-  double* fx = sm + e.le * (3 * Np + 6 * NF);
-  double* fy = fx + Np;
-  double* fz = fy + Np;
-  double* df = fz + Np;
-  const size_t g = (size_t)e.ke * Np + e.p;
-  const double* G[3] = {Gx, Gy, Gz};
+  for (int c = threadIdx.x; c < NF; c += EPB * Np) D[c] = op.D[c];
+  const bool bot = !keep && e.ez == 0;
   if (e.valid) {
     // DDENS is read only when it weights the variable (for DDENS itself V aliases it)
     const double dens = mul_dens ? __ldg(dens_prof + e.ez * N1 + e.k) + __ldg(ddens + g) : 1.0;
-    const double h = mul_dens ? ch * dens : ch, v = mul_dens ? cv * dens : cv;
-    fx[e.p] = h * __ldg(Gx + g);
-    fy[e.p] = h * __ldg(Gy + g);
-    fz[e.p] = v * __ldg(Gz + g);
-    for (int fi = e.p; fi < 6 * NF; fi += Np) {
-      const int f = fi / NF, ab = fi - f * NF, a = ab % N1, b = ab / N1;
-      int pM;
-      size_t gP;
-      long kn;
-      face_exterior<N1>(op, f, a, b, e.ke, e.ex, e.ey, e.ez, e.nxy, pM, gP, kn);
-      const size_t gM = (size_t)e.ke * Np + pM;
-      const int dir = face_dir(f);
-      const double n = face_n(f);
-      const double gMc = __ldg(G[dir] + gM);
-      const bool lid = kn < 0;
-      const double gPc = lid ? odd_ext_n(var, dir, gMc, n) : __ldg(G[dir] + gP);
-      double wM = 0.5, wP = 0.5;
-      if (mul_dens) {
-        const int levM = e.ez * N1 + pM / NF;
-        const int levP = (kn >= 0 ? (int)(kn / e.nxy) : e.ez) * N1 + (int)((gP % Np) / NF);
-        wM = 0.5 * (__ldg(dens_prof + levM) + __ldg(ddens + gM));
-        wP = 0.5 * (__ldg(dens_prof + levP) + __ldg(ddens + gP));
-      }
-      const double c = dir == 2 ? cv : ch;
-      const double d = lid ? c * (wP * gPc - wM * gMc) * n : (1.0 + sgn1(n)) * c * (wP * gPc - wM * gMc) * n;
-      df[fi] = fscale(op, f) * d;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double x = __ldg((d == 0 ? Gx : (d == 1 ? Gy : Gz)) + g);
+      fl[d * Np + e.p] = mul_dens ? dens * x : x;
+    }
+    for (int fi = e.p; fi < 3 * NF; fi += Np) {
+      const int dir = fi / NF;
+      int lev;
+      const long gP = nd_exterior<N1>(op, e, dir, 1, fi - dir * NF, lev);
+      if (gP < 0) continue;
+      const double x = __ldg((dir == 0 ? Gx : (dir == 1 ? Gy : Gz)) + gP);
+      df[fi] = mul_dens ? (__ldg(dens_prof + lev) + __ldg(ddens + gP)) * x : x;
+    }
+  }
+  __syncthreads();
+  if (e.valid) {
+    for (int fi = e.p; fi < (bot ? 4 : 3) * NF; fi += Np) {
+      const int f = fi / NF, dir = f < 2 ? f : 2;
+      const double own = fl[dir * Np + nd_own<N1>(dir, f != 3, fi - f * NF)];
+      if (f == 3 || (f == 2 && e.ez == op.NeZ - 1)) df[fi] = keep ? 0.0 : -own;
+      else df[fi] -= own;
     }
   }
   __syncthreads();
   if (!e.valid) return;
-  const double t = op.E11 * dsum<N1>(op, fx, 0, e.i, e.j, e.k) + op.E22 * dsum<N1>(op, fy, 1, e.i, e.j, e.k) +
-                   op.E33 * dsum<N1>(op, fz, 2, e.i, e.j, e.k) + lift<N1>(op, df, e.i, e.j, e.k);
-  V[g] = V[g] + dt * t;
+  const double h = fma(nd.E[0], nd_dir<N1>(nd, D, fl, df, 0, e, false), nd.E[1] * nd_dir<N1>(nd, D, fl + Np, df, 1, e, false));
+  const double z = nd_dir<N1>(nd, D, fl + 2 * Np, df, 2, e, bot);
+  if (TEND) {
+    V[g] += fma(nd.E[2], z, h);
+  } else {
+    lh[g] = h;
+    lv[g] = nd.E[2] * z;
+  }
 }
 
 // sponge layer: tend -= c(z) (s MOMX, s MOMY, MOMZ), c per level
@@ -257,42 +217,51 @@ __global__ void k_sponge(const double* __restrict__ coef, double* __restrict__ t
 template <int N1>
 constexpr int nd_epb() { return N1 <= 4 ? (N1 <= 2 ? 16 : (N1 == 3 ? 8 : 4)) : 1; }
 
-template <int N1>
-int nd_pass_n(int pass, const Ops& op, const double* dp, const double* a, const double* b, const double* c,
-              const double* ddens, int var, int flag1, int flag2, double ch, double cv, double dt, double* o1,
-              double* o2, double* o3, int Ne, cudaStream_t s) {
-  constexpr int EPB = nd_epb<N1>(), Np = N1 * N1 * N1, NF = N1 * N1;
-  const int grid = (Ne + EPB - 1) / EPB;
-  if (pass == 0) {
-    const size_t sm = sizeof(double) * EPB * (2 * Np + 6 * NF);
-    auto kf = k_nd_grad<N1, EPB>;
-    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kf<<<grid, EPB * Np, sm, s>>>(op, dp, a, b, ddens, var, flag1, flag2, o1, o2, o3, Ne);
-  } else if (pass == 1) {
-    const size_t sm = sizeof(double) * EPB * (3 * Np + 6 * NF);
-    auto kf = k_nd_lap<N1, EPB>;
-    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kf<<<grid, EPB * Np, sm, s>>>(op, a, b, c, var, o1, o2, Ne);
-  } else {
-    const size_t sm = sizeof(double) * EPB * (3 * Np + 6 * NF);
-    auto kf = k_nd_tend<N1, EPB>;
-    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kf<<<grid, EPB * Np, sm, s>>>(op, dp, a, b, c, ddens, var, flag1, ch, cv, dt, o1, Ne);
+NdOps nd_ops(const Ops& d, double ch, double cv, bool lower) {
+  NdOps n;
+  std::memset(&n, 0, sizeof(n));
+  n.E[0] = ch * d.E11;
+  n.E[1] = ch * d.E22;
+  n.E[2] = cv * d.E33;
+  for (int i = 0; i < d.N1; ++i) {
+    n.lf[i] = lower ? -d.Lb[i] : d.Lt[i];
+    n.lo[i] = lower ? d.Lt[i] : -d.Lb[i];
   }
-  return (int)cudaGetLastError();
+  return n;
 }
 
-int nd_pass(int pass, const Ops& op, const double* dp, const double* a, const double* b, const double* c,
-            const double* ddens, int var, int flag1, int flag2, double ch, double cv, double dt, double* o1,
-            double* o2, double* o3, int Ne, cudaStream_t s) {
+struct NdPass {
+  int pass;  // 0 gradient, 1 Laplacian, 2 update
+  const double *a, *b;  // gradient: the fields of the horizontal and of the vertical derivative
+  const double* ddens;
+  int dens, wall;  // density division / weight; the lid's reflection (gradient), or none at it (divergence)
+  double *G[3], *lh, *lv, *V;
+};
+
+template <int N1>
+int nd_pass_n(const NdPass& P, const Ops& op, const NdOps& nd, const double* dp, int Ne, cudaStream_t s) {
+  constexpr int EPB = nd_epb<N1>(), Np = N1 * N1 * N1, NF = N1 * N1;
+  const size_t sm = sizeof(double) * (NF + EPB * ((P.pass == 0 ? 2 : 3) * Np + 4 * NF));
+  auto go = [&](auto kf, auto... args) {
+    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    kf<<<(Ne + EPB - 1) / EPB, EPB * Np, sm, s>>>(op, nd, dp, args..., Ne);
+    return (int)cudaGetLastError();
+  };
+  const double *gx = P.G[0], *gy = P.G[1], *gz = P.G[2];
+  if (P.pass == 0) return go(k_nd_grad<N1, EPB>, P.a, P.b, P.ddens, P.dens, P.wall, P.G[0], P.G[1], P.G[2]);
+  return P.pass == 1 ? go(k_nd_div<N1, EPB, false>, gx, gy, gz, P.ddens, P.dens, P.wall, P.lh, P.lv, P.V)
+                     : go(k_nd_div<N1, EPB, true>, gx, gy, gz, P.ddens, P.dens, P.wall, P.lh, P.lv, P.V);
+}
+
+int nd_pass(const NdPass& P, const Ops& op, const NdOps& nd, const double* dp, int Ne, cudaStream_t s) {
   switch (op.N1) {
-    case 2: return nd_pass_n<2>(pass, op, dp, a, b, c, ddens, var, flag1, flag2, ch, cv, dt, o1, o2, o3, Ne, s);
-    case 3: return nd_pass_n<3>(pass, op, dp, a, b, c, ddens, var, flag1, flag2, ch, cv, dt, o1, o2, o3, Ne, s);
-    case 4: return nd_pass_n<4>(pass, op, dp, a, b, c, ddens, var, flag1, flag2, ch, cv, dt, o1, o2, o3, Ne, s);
-    case 5: return nd_pass_n<5>(pass, op, dp, a, b, c, ddens, var, flag1, flag2, ch, cv, dt, o1, o2, o3, Ne, s);
-    case 6: return nd_pass_n<6>(pass, op, dp, a, b, c, ddens, var, flag1, flag2, ch, cv, dt, o1, o2, o3, Ne, s);
-    case 7: return nd_pass_n<7>(pass, op, dp, a, b, c, ddens, var, flag1, flag2, ch, cv, dt, o1, o2, o3, Ne, s);
-    case 8: return nd_pass_n<8>(pass, op, dp, a, b, c, ddens, var, flag1, flag2, ch, cv, dt, o1, o2, o3, Ne, s);
+    case 2: return nd_pass_n<2>(P, op, nd, dp, Ne, s);
+    case 3: return nd_pass_n<3>(P, op, nd, dp, Ne, s);
+    case 4: return nd_pass_n<4>(P, op, nd, dp, Ne, s);
+    case 5: return nd_pass_n<5>(P, op, nd, dp, Ne, s);
+    case 6: return nd_pass_n<6>(P, op, nd, dp, Ne, s);
+    case 7: return nd_pass_n<7>(P, op, nd, dp, Ne, s);
+    case 8: return nd_pass_n<8>(P, op, nd, dp, Ne, s);
   }
   return (int)cudaErrorInvalidValue;
 }
@@ -346,27 +315,23 @@ int fedg_numdiff_apply_prec(fedg_ctx* c, double* const q[5], int nlap, double co
   double* lv = lh + n;
   const double sgn = ((nlap + 1) % 2 == 0) ? 1.0 : -1.0;  // (-1)^mod(n+1, 2)
   const int order[5] = {VRT, VMZ, VMX, VMY, VD};         // apply_numfilter's order: DDENS changes last
+  const NdOps grad = nd_ops(c->op, 1.0, 1.0, true), lap = nd_ops(c->op, 1.0, 1.0, false),
+              upd = nd_ops(c->op, dt * (sgn * coef_h), dt * (sgn * coef_v), false);
   for (int vi = 0; vi < 5; ++vi) {
     const int var = order[vi];
-    const int dw = var != VD;
-    int r = tracked(c, FEDG_K_ND, [&] {
-      return nd_pass(0, c->op, c->d_prof, q[var], q[var], nullptr, q[VD], var, dw, 1, 0, 0, 0, Gx, Gy, Gz, c->Ne,
-                     c->stream);
-    });
+    const int dw = var != VD, wall = var == VMZ;
+    auto pass = [&](int kind, const double* a, const double* b, int dens, int wl, double* V) {
+      const NdPass P{kind, a, b, q[VD], dens, wl, {Gx, Gy, Gz}, lh, lv, V};
+      return tracked(c, FEDG_K_ND, [&] {
+        return nd_pass(P, c->op, kind == 0 ? grad : (kind == 1 ? lap : upd), c->d_prof, c->Ne, c->stream);
+      });
+    };
+    int r = pass(0, q[var], q[var], dw, wall, nullptr);
     for (int it = 1; it < nlap && !r; ++it) {
-      r = tracked(c, FEDG_K_ND, [&] {
-        return nd_pass(1, c->op, c->d_prof, Gx, Gy, Gz, nullptr, var, 0, 0, 0, 0, 0, lh, lv, nullptr, c->Ne, c->stream);
-      });
-      if (!r)
-        r = tracked(c, FEDG_K_ND, [&] {
-          return nd_pass(0, c->op, c->d_prof, lh, lv, nullptr, q[VD], var, 0, 0, 0, 0, 0, Gx, Gy, Gz, c->Ne, c->stream);
-        });
+      r = pass(1, nullptr, nullptr, 0, wall, nullptr);
+      if (!r) r = pass(0, lh, lv, 0, 0, nullptr);
     }
-    if (!r)
-      r = tracked(c, FEDG_K_ND, [&] {
-        return nd_pass(2, c->op, c->d_prof, Gx, Gy, Gz, q[VD], var, dw, 0, sgn * coef_h, sgn * coef_v, dt, q[var],
-                       nullptr, nullptr, c->Ne, c->stream);
-      });
+    if (!r) r = pass(2, nullptr, nullptr, dw, wall, q[var]);
     if (r) return api_cuda_fail((cudaError_t)r, "fedg_numdiff_apply");
   }
   return 0;
