@@ -27,8 +27,8 @@ namespace fedg {
 namespace {
 
 // Tables of a pass.  An interior face's flux is nonzero only on one of its two sides (the gradient takes the
-// lower neighbour, the divergence the upper), so an element computes three faces, with Lift lf, and a lid face (Lift
-// lo of the fourth) only where the reflection leaves a jump; the signs are in lf and lo.  E of each
+// lower neighbour, the divergence the upper), so an element computes three faces, with Lift lf, and at the lid on the
+// other side a fourth with Lift lo; the signs are in lf and lo.  E of each
 // direction holds the pass's coefficient; Escale and Fscale are the same 2/dx.
 struct NdOps {
   double E[3], lf[FEDG_MAXN1], lo[FEDG_MAXN1];
@@ -86,19 +86,19 @@ __device__ __forceinline__ double nd_dir(const NdOps& nd, const double* D, const
   constexpr int NF = N1 * N1;
   const int row = dir == 0 ? e.i : (dir == 1 ? e.j : e.k), stp = dir == 0 ? 1 : (dir == 1 ? N1 : NF);
   const int ab = dir == 0 ? e.j + N1 * e.k : (dir == 1 ? e.i + N1 * e.k : e.i + N1 * e.j);
-  double s = nd.lf[row] * df[dir * NF + ab];
-  if (dir == 2 && lid) s = fma(nd.lo[row], df[3 * NF + ab], s);
+  double s = 0.0;
   u += e.p - row * stp;
 #pragma unroll
   for (int l = 0; l < N1; ++l) s = fma(D[row * N1 + l], u[l * stp], s);
-  return s;
+  s = fma(nd.lf[row], df[dir * NF + ab], s);
+  return dir == 2 && lid ? fma(nd.lo[row], df[3 * NF + ab], s) : s;
 }
 
 // numdiff_cal_flx: G = (d/dx Vh, d/dy Vh, d/dz Vv) (each divided by the density when dens_div).  refl: at the
 // lids the even routine's exterior of Vv reflects it (the wall-normal momentum); otherwise no jump there.
 //
-// What bounds it: the FP64 pipe, about 47 instructions per node (one reciprocal for the node and one for each computed
-// face node).  16x16x8 elements at p = 7: 128 -> 82 us.
+// What bounds it: the FP64 pipe, about 47 instructions per node (one quotient for the node and a reciprocal for each
+// side of a computed face node).  16x16x8 elements at p = 7: 128 -> 88 us.
 template <int N1, int EPB>
 __global__ void __launch_bounds__(EPB* N1* N1* N1)
     k_nd_grad(const __grid_constant__ Ops op, const __grid_constant__ NdOps nd, const double* __restrict__ dens_prof,
@@ -113,27 +113,29 @@ __global__ void __launch_bounds__(EPB* N1* N1* N1)
   double* df = vh + 2 * Np;
   const size_t g = (size_t)e.ke * Np + e.p;
   for (int c = threadIdx.x; c < NF; c += EPB * Np) D[c] = op.D[c];
-  const bool top = refl && e.ez == op.NeZ - 1;
+  const bool top = e.ez == op.NeZ - 1;
   if (e.valid) {
-    const double rd = dens_div ? 1.0 / (__ldg(ddens + g) + __ldg(dens_prof + e.ez * N1 + e.k)) : 1.0;
-    vh[e.p] = dens_div ? __ldg(Vh + g) * rd : __ldg(Vh + g);
-    if (vv != vh) vv[e.p] = dens_div ? __ldg(Vv + g) * rd : __ldg(Vv + g);
-    for (int fi = e.p; fi < 3 * NF; fi += Np) {
-      const int dir = fi / NF;
-      int lev;
-      const long gP = nd_exterior<N1>(op, e, dir, 0, fi - dir * NF, lev);
-      if (gP < 0) continue;
-      const double vP = __ldg((dir == 2 ? Vv : Vh) + gP);
-      df[fi] = dens_div ? vP / (__ldg(ddens + gP) + __ldg(dens_prof + lev)) : vP;
-    }
-  }
-  __syncthreads();
-  if (e.valid) {
+    // quotients, not a reciprocal's products: dens * const gives back the constant, whose derivative vanishes
+    const double dens = dens_div ? __ldg(ddens + g) + __ldg(dens_prof + e.ez * N1 + e.k) : 1.0;
+    vh[e.p] = dens_div ? __ldg(Vh + g) / dens : __ldg(Vh + g);
+    if (vv != vh) vv[e.p] = dens_div ? __ldg(Vv + g) / dens : __ldg(Vv + g);
+    // jumps of the lower faces of x, y, z, then the upper lid's, where half counts.  Of a uniform flow nothing is left but
+    // the products' rounding, by one formula on every face as in FElib's flux.
     for (int fi = e.p; fi < (top ? 4 : 3) * NF; fi += Np) {
-      const int f = fi / NF, dir = f < 2 ? f : 2;
-      const double own = (dir == 2 ? vv : vh)[nd_own<N1>(dir, f == 3, fi - f * NF)];
-      if (f == 3 || (f == 2 && e.ez == 0)) df[fi] = refl ? -own : 0.0;  // half of the reflected jump
-      else df[fi] -= own;
+      const int f = fi / NF, dir = f < 2 ? f : 2, ab = fi - f * NF, pM = nd_own<N1>(dir, f == 3, ab);
+      const size_t gM = (size_t)e.ke * Np + pM;
+      const double* V = dir == 2 ? Vv : Vh;
+      double wM = 1.0, wP = 1.0;
+      if (dens_div) wM = 1.0 / (__ldg(ddens + gM) + __ldg(dens_prof + e.ez * N1 + pM / NF));
+      const double vM = __ldg(V + gM);
+      int lev;
+      const long gP = f == 3 ? -1 : nd_exterior<N1>(op, e, dir, 0, ab, lev);
+      if (gP < 0) {
+        df[fi] = 0.5 * fma(refl ? -vM : vM, wM, -(vM * wM));
+        continue;
+      }
+      if (dens_div) wP = 1.0 / (__ldg(ddens + gP) + __ldg(dens_prof + lev));
+      df[fi] = fma(__ldg(V + gP), wP, -(vM * wM));
     }
   }
   __syncthreads();
