@@ -48,27 +48,22 @@ PATH_PREC = {"pair": 2, "mixed": 1, "fp64": 0}
 PATH_TOL = {"pair": 1e-13, "mixed": 1e-10, "fp64": 1e-10}
 PATH_ITER = {"pair": 30, "mixed": 20, "fp64": 20}
 PATH_NAME = {"pair": "pair", "mixed": "fp32", "fp64": "plain_fp64"}
-# FP64 flops of the plain column solve per node and launch, counted on FElib's algorithm (dense
-# block LU with partial pivoting of the 3N1 x 3N1 element blocks, hevi_common_linalgebra.F90:2296-2445):
-# per element column (n = 24 at p = 7) 2n^3/3 for the factorisation plus 4 right-hand sides x 2n^2
-# for the substitutions, per node (/ N1); the MOMX/MOMY element solves (N1 x N1, 3 right-hand sides)
-# and two residual evaluations (Dz of three fluxes, VPOrdM1, Lift: ~100 flop per node each)
-def fp64_vi_flops_per_node(N1):
-    n = 3 * N1
-    return (2 * n ** 3 / 3 + 4 * 2 * n * n) / N1 + (2 * N1 ** 3 / 3 + 3 * 2 * N1 * N1) / N1 + 2 * 100
+# FP64 instructions per node of the plain column solve (FP32 sweeps, FP64 residuals) at p = 7, measured by ncu: the
+# share of the FP64 pipe's cycles times the time on 16x16x8 elements, about 330 for a launch with one solve and 90
+# for the first stage's evaluation of A; the mean of a step's three launches
+VI64_FP64_INST_PER_NODE = (90 + 330 + 330) / 3
 PATH_DTYPE = {"pair": "f32x2", "mixed": "f32+f32x2", "fp64": "f64"}
 # DRAM bytes per node of one launch of the dominant kernel, measured by ncu (dram__bytes_read.sum +
-# dram__bytes_write.sum on the 32x32x16-element slice, 8,388,608 nodes; the mean of the step's two
-# launches, one per implicit stage), per path
+# dram__bytes_write.sum on 32x32x8 elements of p = 7), per path
 NCU_BYTES_PER_NODE = {
-    "pair": {"vi_mixed": ((1126.824704e6 + 656.262912e6) + (1039.029504e6 + 647.403264e6)) / 2 / (32 * 32 * 16 * 512)},
+    "pair": {"vi_mixed": 934.146542e9 * 714.496e-6 / (32 * 32 * 8 * 512)},
 }
 
 
 # warp instructions per node of one launch of the dominant kernel, measured by ncu
-# (smsp__inst_executed.sum on the 32x32x16-element slice, the mean of the step's two launches), per path
+# (smsp__inst_executed.sum on 32x32x8 elements of p = 7), per path
 NCU_INST_PER_NODE = {
-    "pair": {"vi_mixed": (1.841753748e9 + 1.782838923e9) / 2 / (32 * 32 * 16 * 512)},
+    "pair": {"vi_mixed": 446.382478e6 / (32 * 32 * 8 * 512)},
 }
 
 
@@ -84,7 +79,7 @@ def issue_roofline(kname, path, nodes, avg_ms, sm_mhz, n_sm):
     peak = 4.0 * n_sm * mhz * 1e6
     return {"bound": "issue", "kernel": kname, "achieved": achieved, "peak": peak, "unit": "warp instructions/s",
             "frac": achieved / peak, "inst_per_node": ipn, "sm_mhz": mhz, "sms": n_sm,
-            "source": "ncu smsp__inst_executed.sum on the 32x32x16 slice, scaled by nodes; peak = 4 x SMs x SM clock"}
+            "source": "ncu smsp__inst_executed.sum on 32x32x8 elements, scaled by nodes; peak = 4 x SMs x SM clock"}
 
 
 def max_over_ranks(value, world, device):
@@ -630,7 +625,7 @@ def run_fedg(args):
     traffic = ncu_bytes_per_node[kname] * nodes / 1e9 if kname in ncu_bytes_per_node else None
     roof = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peaks.get("hbm_gbs", 6800.0),
             "unit": "GB/s", "frac": achieved / peaks.get("hbm_gbs", 6800.0), "traffic": traffic,
-            "traffic_unit": "GB per launch (ncu DRAM read+write of the same path on the 32x32x16 slice, scaled by nodes)",
+            "traffic_unit": "GB per launch (ncu DRAM read+write of the same path on a slice of the mesh, scaled by nodes)",
             "peak_source": peak_src, "avg_launch_ms": avg_ms, "algorithmic_bytes_per_node": bytes_per_node.get(kname)}
     n_sm = torch.cuda.get_device_properties(ctx.dev).multi_processor_count
     roof_issue = issue_roofline(kname, path, nodes, avg_ms, (clocks or {}).get("sm_mhz"), n_sm)
@@ -743,13 +738,13 @@ def run_fedg(args):
                  "kernels": {k: {"ms": v[0], "launches": v[1]} for k, v in p64.items() if v[1]}}
         vt, vn = p64.get("vi_fp64", (0.0, 0))
         if vn and fp64_tf > 0:
-            fpn = fp64_vi_flops_per_node(case.N1) * max(its64, 1.0)
+            fpn = 2.0 * VI64_FP64_INST_PER_NODE
             ach = fpn * nodes / (vt / vn * 1e-3) / 1e12
             plain["roofline_fp64_column_solve"] = {
                 "bound": "fp64", "kernel": "vi_fp64", "achieved_tflops": ach, "peak_tflops": fp64_tf,
                 "frac": ach / fp64_tf, "flop_per_node": fpn, "avg_launch_ms": vt / vn,
-                "flop_count": "FElib's dense block LU with partial pivoting, its substitutions and the residuals, "
-                              "per Newton solve; the kernel itself skips the DENS rows' structural zeros"}
+                "flop_count": "FP64 instructions of the refinement solve (ncu), each counted as an FMA; FElib's dense "
+                              "block LU would be about 2000 flop per node and solve"}
         ctx.update(q_mix, ncmp, **opts)
         acc = {"steps": ncmp, "rel_l2_vs_plain_fp64": _full_field_errors(np, q_mix, q_ref, dnorm2, dens_hyd, therm_hyd)}
         if other is not None:
