@@ -568,32 +568,42 @@ __global__ void k_trc_alph_dyn(const Ops op, const Prof pf, const MflxArgs<S> A,
 template <int N1>
 constexpr int trc_epb() { return N1 <= 4 ? (N1 <= 2 ? 16 : (N1 == 3 ? 8 : 4)) : 1; }
 
-template <int N1>
+template <int N1, int EPB>
 size_t fct_smem() {
-  constexpr int EPB = trc_epb<N1>(), Np = N1 * N1 * N1, NF = N1 * N1;
+  constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
   return sizeof(double) * EPB * (6 * NF + 8 + Np + 1);
 }
-template <int N1>
+template <int N1, int EPB>
 size_t stage_smem() {
-  constexpr int EPB = trc_epb<N1>(), Np = N1 * N1 * N1, NF = N1 * N1;
+  constexpr int Np = N1 * N1 * N1, NF = N1 * N1;
   return sizeof(double) * (3 * NF + 6 * N1 + EPB * (3 * Np + 2 * 6 * NF + 8 + 2 * (Np + 1) + Np));
 }
 
+// At p = 3 two elements per block while blocks of four would be one wave (four per SM): 500 blocks of four leave some
+// SMs a third more elements than others (20x20x5 elements, a step: 138 us with four, 131 with two); with many
+// waves four are better (48x48x20 elements, coefficient kernel 259 and 276 us).
 template <int N1>
+bool one_wave(int Ne) { return N1 == 4 && Ne <= 4 * 152 * trc_epb<N1>(); }
+
+template <int N1, int EPB = trc_epb<N1>()>
 int launch_fct_n(const Ops& op, const double* dp, const TrcIn& in, const TrcFct& fc, int Ne, cudaStream_t s) {
-  constexpr int EPB = trc_epb<N1>(), Np = N1 * N1 * N1;
-  const size_t sm = fct_smem<N1>();
+  if constexpr (N1 == 4 && EPB != 2)
+    if (one_wave<N1>(Ne)) return launch_fct_n<N1, 2>(op, dp, in, fc, Ne, s);
+  constexpr int Np = N1 * N1 * N1;
+  const size_t sm = fct_smem<N1, EPB>();
   auto kfn = k_trc_fct<N1, EPB>;
   cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   kfn<<<(Ne + EPB - 1) / EPB, EPB * Np, sm, s>>>(
       op, dp, in, fc, make_double3(op.Jac * op.FSx, op.Jac * op.FSy, op.Jac * op.FSz), 1.0 / fc.dt, Ne);
   return (int)cudaGetLastError();
 }
-template <int N1>
+template <int N1, int EPB = trc_epb<N1>()>
 int launch_stage_n(const Ops& op, const double* dp, const TrcIn& in, const TrcStage& st, const TrcFilt& tf, int Ne,
                    cudaStream_t s) {
-  constexpr int EPB = trc_epb<N1>(), Np = N1 * N1 * N1;
-  const size_t sm = stage_smem<N1>();
+  if constexpr (N1 == 4 && EPB != 2)
+    if (one_wave<N1>(Ne)) return launch_stage_n<N1, 2>(op, dp, in, st, tf, Ne, s);
+  constexpr int Np = N1 * N1 * N1;
+  const size_t sm = stage_smem<N1, EPB>();
   auto kfn = st.fct_elem ? k_trc_stage<N1, EPB, true> : k_trc_stage<N1, EPB, false>;
   cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   kfn<<<(Ne + EPB - 1) / EPB, EPB * Np, sm, s>>>(op, dp, in, st, tf, Ne);

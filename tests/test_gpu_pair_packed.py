@@ -55,3 +55,20 @@ def test_tracer_pair(porder, ne, limiter):
                    prec=fl.PREC_PAIR)
     got = Qd.cpu().numpy()
     assert np.linalg.norm(got - ref) < 1e-11 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("ne", [(16, 38, 4), (17, 13, 11)])
+def test_tracer_fp64_block_rule(ne):
+    """p = 3 at the largest mesh of the two-elements-per-block rule (2432 elements, a whole wave) and at the one
+    below it (2431, the last block half empty): one limited step against the oracle, FP64 on both sides."""
+    case = t1(ne, 3)
+    o, ctx, q, b, _ = setup_trc(case, seed=70, wobble=0.3)
+    Q = 1.0 + np.random.default_rng(71).random(o.shape)
+    aM, aP = o.trc_alphdens_advtest(q[0], q[1], q[2], q[3])
+    dt = 0.05 * case.dt
+    ref = o.trc_step(Q, q[1:4], aM, aP, q[0], q[0], dt, nsteps=1, limiter=True, tmar=True)
+    qd = [ctx.tensor(a) for a in q]
+    Qd = ctx.tensor(Q)
+    ctx.trc_update(Qd, qd[1:4], ctx.tensor(aM), ctx.tensor(aP), qd[0], qd[0], dt, nsteps=1, limiter=True, tmar=True)
+    got = Qd.cpu().numpy()
+    assert np.linalg.norm(got - ref) < 1e-12 * np.linalg.norm(ref)
