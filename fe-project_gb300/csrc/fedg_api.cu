@@ -231,7 +231,11 @@ struct RKPtrs {
   const double* tim[3][5];
 };
 
-__global__ void k_rk(RKPtrs P, int kind, int stage, int nst, RKC c, size_t n, int first_stage) {
+// PRES: kind 1 also forms DPRES of the new DRHOT; the FP64 arithmetic of its series hides behind the copies' memory
+// traffic (a launch of its own: 25 us for 2^20 nodes)
+template <bool PRES>
+__global__ void k_rk(RKPtrs P, int kind, int stage, int nst, RKC c, size_t n, int first_stage,
+                     const __grid_constant__ Ops op, const Prof pf, double* __restrict__ dp) {
   const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= n) return;
 #pragma unroll
@@ -244,7 +248,13 @@ __global__ void k_rk(RKPtrs P, int kind, int stage, int nst, RKC c, size_t n, in
         P.var0[v][g] = q;
         P.vtmp[v][g] = q;
       }
-      P.q[v][g] = q + c.c[0] * P.tim[stage - 1][v][g];
+      q = fma(c.c[0], P.tim[stage - 1][v][g], q);
+      P.q[v][g] = q;
+      if (PRES && v == VRT) {
+        const size_t ke = g / op.Np;
+        const int lev = (int)(ke / ((size_t)op.NeX * op.NeY)) * op.N1 + (int)(g - ke * op.Np) / (op.N1 * op.N1);
+        dp[g] = dpres_of(op, pf, lev, q);
+      }
     } else if (kind == 2) {
       double s = P.var0[v][g];
       P.vtmp[v][g] = P.vtmp[v][g] + c.c[6] * P.tex[stage - 1][v][g] + c.c[7] * P.tim[stage - 1][v][g];
@@ -607,7 +617,7 @@ double* fedg_tint_tend_im(fedg_tint* t, int stage, int var) {
 }
 double* fedg_tint_var0(fedg_tint* t, int var) { return (t && var >= 0 && var < 5) ? t->var0(var) : nullptr; }
 
-static int rk_launch(fedg_tint* t, double* const q[5], int kind, int stage, RKC cc, int first) {
+static int rk_launch(fedg_tint* t, double* const q[5], int kind, int stage, RKC cc, int first, double* dp = nullptr) {
   fedg_ctx* c = t->ctx;
   CK(cudaSetDevice(c->d.device));
   RKPtrs P;
@@ -624,7 +634,8 @@ static int rk_launch(fedg_tint* t, double* const q[5], int kind, int stage, RKC 
   }
   const int bs = 256;
   CK((cudaError_t)tracked(c, FEDG_K_RK, [&] {
-    k_rk<<<(unsigned)((c->n + bs - 1) / bs), bs, 0, c->stream>>>(P, kind, stage, t->nstage, cc, c->n, first);
+    auto kf = dp ? k_rk<true> : k_rk<false>;
+    kf<<<(unsigned)((c->n + bs - 1) / bs), bs, 0, c->stream>>>(P, kind, stage, t->nstage, cc, c->n, first, c->op, c->prof(), dp);
     return (int)cudaGetLastError();
   }));
   return 0;
@@ -636,12 +647,17 @@ int fedg_tint_store_var0(fedg_tint* t, double* const q[5]) {
   return rk_launch(t, q, 0, 1, cc, 0);
 }
 
+// StoreImplicit of an IMEX scheme, with DPRES of the new state into dp unless NULL
+static int store_implicit(fedg_tint* t, int stage, double* const q[5], double* dp) {
+  RKC cc{};
+  cc.c[0] = t->dt * t->a_im[stage - 1][stage - 1];
+  return rk_launch(t, q, 1, stage, cc, stage == 1, dp);
+}
+
 int fedg_tint_store_implicit(fedg_tint* t, int stage, double* const q[5]) {
   if (!t || !q || stage < 1 || stage > t->nstage) return fail("fedg_tint_store_implicit: bad argument");
   if (t->scheme != FEDG_IMEX_ARK232) return 0;  // rk_storeimpl: explicit schemes return at once
-  RKC cc{};
-  cc.c[0] = t->dt * t->a_im[stage - 1][stage - 1];
-  return rk_launch(t, q, 1, stage, cc, stage == 1);
+  return store_implicit(t, stage, q, nullptr);
 }
 
 int fedg_tint_advance(fedg_tint* t, int stage, double* const q[5]) {
@@ -698,7 +714,6 @@ static int update_impl(fedg_ctx* c, double* const q[5], int nsteps, const fedg_u
   double* gsc = nullptr;
   if (o->eqs == FEDG_HEVI && !(gsc = vi_scratch(c, &ngsc)))
     return fail(ngsc ? "fedg_update: out of device memory" : "fedg_update: the column does not fit in shared memory");
-  const double* base[16] = {};
   long long nsum = 0, ncnt = 0;
   int nfail = 0;
   double* const* tf = c->trc_flux;
@@ -732,14 +747,13 @@ static int update_impl(fedg_ctx* c, double* const q[5], int nsteps, const fedg_u
   for (int step = 0; step < nsteps && r >= 0; ++step) {
     if (tf[0] && cudaMemcpyAsync(tf[6], q[0], nb64, cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess)
       return fail("fedg_update: DDENS0_TRC copy");
-    if (o->eqs == FEDG_HEVI) r = fedg_tint_store_var0(t, q);
     for (int s = 1; s <= t->nstage && r >= 0; ++s) {
       if (o->eqs == FEDG_HEVI) {
         const double fac = fedg_tint_implicit_diagfac(t, s);
         F5c qc{{q[0], q[1], q[2], q[3], q[4]}};
         F5c z{{t->var0(0), t->var0(1), t->var0(2), t->var0(3), t->var0(4)}};
         F5 tim{{t->tim(s - 1, 0), t->tim(s - 1, 1), t->tim(s - 1, 2), t->tim(s - 1, 3), t->tim(s - 1, 4)}};
-        // stage 1: var0 is the state itself (StoreImplicit copies it at stage 1)
+        // stage 1: var0 is the state itself, which StoreImplicit copies after the solve (store_var0 would copy it twice)
         if (s == 1) z = qc;
         ViArgs a{fac, o->dt, o->tol, o->max_iter, 340.0};
         r = tracked(c, FEDG_K_VI, [&] {
@@ -749,11 +763,13 @@ static int update_impl(fedg_ctx* c, double* const q[5], int nsteps, const fedg_u
         if (fac != 0.0) {
           if ((r = count_status(c, c->d_status))) return r;
         }
-        r = fedg_tint_store_implicit(t, s, q);
+        r = store_implicit(t, s, q, dp);
         if (r) break;
       }
-      r = tracked(c, FEDG_K_PRES, [&] { return launch_drhot2pres(c->op, c->prof(), q[4], nullptr, dp, c->n, c->stream); });
-      if (r) return cuda_fail((cudaError_t)r, "fedg_update: drhot2pres");
+      if (o->eqs != FEDG_HEVI) {
+        r = tracked(c, FEDG_K_PRES, [&] { return launch_drhot2pres(c->op, c->prof(), q[4], nullptr, dp, c->n, c->stream); });
+        if (r) return cuda_fail((cudaError_t)r, "fedg_update: drhot2pres");
+      }
       // a slab exchanges the face layers of the stage state and DPRES (driver_nonhydro3d.F90:768-787)
       if (fedg::slab(c) && (r = fedg::halo_exchange_fp64(c, q, dp, s))) return r;
       F5c qc{{q[0], q[1], q[2], q[3], q[4]}};
@@ -782,7 +798,6 @@ static int update_impl(fedg_ctx* c, double* const q[5], int nsteps, const fedg_u
       return fail("fedg_update: DDENS_TRC copy");
     if (r >= 0 && c->d.mf_on) r = fedg_modalfilter(c, q);
   }
-  (void)base;
   if (r < 0) return r;
   if (o->eqs == FEDG_HEVI && (nfail = count_read(c, &nsum, &ncnt)) < 0) return nfail;
   if (iters_out) *iters_out = ncnt ? double(nsum) / double(ncnt) : 0.0;
