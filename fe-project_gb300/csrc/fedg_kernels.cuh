@@ -45,7 +45,8 @@ int launch_vi_fp64(const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, 
                    const ViArgs& a, double* gsc, size_t gsc_doubles, cudaStream_t s);
 
 // Its first pass, by iterative refinement (fedg_vi64.cu): columns it leaves get status VI_REDO and are
-// solved by block LU.  Returns -1 if the columns are too tall for its shared memory (nothing launched).
+// solved by block LU.  Returns -1, nothing launched, if the columns are too tall for its shared memory or max_iter < 1
+// allows no solve (block LU then reports every column above tol as not converged).
 constexpr int VI_REDO = -100;
 size_t vi64_scratch_doubles(const Ops& op);
 int launch_vi64(const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, const F5& tout, int* status, const ViArgs& a,
