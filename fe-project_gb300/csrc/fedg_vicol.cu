@@ -861,10 +861,12 @@ __global__ void __launch_bounds__(64, 6) k_vi_cols(const Ops op, const OpsX ox, 
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int grp = lane / N1, k = lane % N1;
   // ncol is a multiple of C: a warp's columns are all valid or none (no block barriers).  REDO: only the
-  // warps with a column marked VI_REDO by the series kernel, which the grid's warps look for in turn
+  // columns marked VI_REDO by the series kernel, whose warps the grid looks for in turn; the warp's other columns
+  // take part in its shuffles, but nothing of them is stored or counted
   for (int col0 = (blockIdx.x * 2 + wib) * C; col0 < ncol; col0 += gridDim.x * 2 * C) {
   const int col = col0 + grp;
-  if (REDO && !__any_sync(FULL, status[col] == VI_REDO)) continue;
+  const bool mine = !REDO || status[col] == VI_REDO;
+  if (REDO && !__any_sync(FULL, mine)) continue;
   const int NeZ = op.NeZ, L = op.L;
   const ColLayout lay(N1, NeZ);
   unsigned char* base = smraw + (size_t)(wib * C + grp) * lay.stride;
@@ -911,7 +913,7 @@ __global__ void __launch_bounds__(64, 6) k_vi_cols(const Ops op, const OpsX ox, 
   // contract asks for LU corrections again.  The warp runs an LU correction if any of its active
   // columns asks for one.
   int nsolve = 0, st = 0;
-  bool active = true, want_lu = true, last_lu = true;
+  bool active = mine, want_lu = true, last_lu = true;
   float err_prev = 0.f;
   while (true) {
     // the first residual comes from the stage's A(var0) when the iterate starts at var0; every
@@ -953,6 +955,7 @@ __global__ void __launch_bounds__(64, 6) k_vi_cols(const Ops op, const OpsX ox, 
         po[m] = *c.plo(m, en);
       }
     }
+    if (!mine) continue;
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
       const f2 pnew{c.P[3 * l + m], pc[m]};
@@ -1012,7 +1015,7 @@ __global__ void __launch_bounds__(64, 6) k_vi_cols(const Ops op, const OpsX ox, 
     const float lb0 = ox.Lb[0].x, lbN = ox.Lb[N].x, lt0 = ox.Lt[0].x, ltN = ox.Lt[N].x;
     const float iscu_c = 1.f / (float)args.cref;
     float* jdel = reinterpret_cast<float*>(c.del);  // 4 jumps of the current element
-    bool active = true;
+    bool active = mine;
     for (int it = 0; it < 4; ++it) {
       float err = 0.f;
       bool bad = false;
@@ -1120,6 +1123,7 @@ __global__ void __launch_bounds__(64, 6) k_vi_cols(const Ops op, const OpsX ox, 
         eo[0] = *c.plo(0, en);
         eo[1] = *c.plo(1, en);
       }
+      if (!mine) continue;
       const f2 dh = f2_of(__ldg(px.dh + l));
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
@@ -1145,10 +1149,10 @@ __global__ void __launch_bounds__(64, 6) k_vi_cols(const Ops op, const OpsX ox, 
     asm volatile("discard.global.L2 [%0], 128;" ::"l"(a) : "memory");
   }
 
-  if (k == 0 && status) status[col] = st;
-  const unsigned nfail = __reduce_add_sync(FULL, (k == 0 && st < 0) ? 1u : 0u);
-  const unsigned nsol = __reduce_add_sync(FULL, (k == 0 && st >= 0) ? (unsigned)st : 0u);
-  const unsigned nok = __reduce_add_sync(FULL, (k == 0 && st >= 0) ? 1u : 0u);
+  if (k == 0 && mine && status) status[col] = st;
+  const unsigned nfail = __reduce_add_sync(FULL, (k == 0 && mine && st < 0) ? 1u : 0u);
+  const unsigned nsol = __reduce_add_sync(FULL, (k == 0 && mine && st >= 0) ? (unsigned)st : 0u);
+  const unsigned nok = __reduce_add_sync(FULL, (k == 0 && mine && st >= 0) ? 1u : 0u);
   if (lane == 0) {
     if (nfail) atomicAdd(cnt, (unsigned long long)nfail);
     if (nok) {
