@@ -33,7 +33,7 @@ struct SweepCtx {
 };
 
 // One sweep x <- (1 - w) x + w (b - K x), from x = w b if first; returns the lane's largest weighted
-// change.  (A NaN can drop out of the change; the certifying residual looks at every node.)
+// change.  (A NaN can drop out of the change; the FP64 residual that follows the sweeps looks at every node.)
 template <int N1, int GL>
 __device__ __forceinline__ float sweep(const SweepCtx<N1, GL>& c, const u64x (&Dk)[N1], const u64x (&Tk)[N1],
                                        u64x facB, u64x facT, u64x w, u64x w1, float c1, float c2, bool first) {

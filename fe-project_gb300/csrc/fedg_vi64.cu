@@ -312,12 +312,14 @@ __global__ void __launch_bounds__(64, 6)
           if (__all_sync(FULL, doneA && doneB)) break;
           if (nsolve >= args.v.max_iter) { give_up = true; break; }
         }
-        // ---- J delta = b by refinement: rho is the residual's size over b's ----
+        // ---- J delta = b by refinement: rho is the residual's size over b's.  Solved once what the last sweeps
+        // left, or the residual itself, is below FP64's roundoff; anything else is left to block LU ----
         float rho = 1.f, rmax = bmax;
+        bool solved = false;
         for (int it = 0; it < 6; ++it) {
           // the sweeps leave rel of their right-hand side; the last ones need not go below FP64's roundoff
-          const float rel = fminf(1.0e-3f, fmaxf(1.0e-6f, __fdividef(1.0e-17f, rho)));
-          if (!sweeps<N1, GL>(c, sc, op, impl, rmax, rel, 0.f, args.c1, args.c2)) { give_up = true; break; }
+          const float rel = fminf(1.0e-3f, fmaxf(1.0e-6f, 1.0e-17f / rho));
+          if (!sweeps<N1, GL>(c, sc, op, impl, rmax, rel, 0.f, args.c1, args.c2)) break;
           for (int e = 0; e < NeZ; ++e) {
 #pragma unroll
             for (int v = 0; v < 3; ++v) {
@@ -327,8 +329,9 @@ __global__ void __launch_bounds__(64, 6)
             }
           }
           __syncwarp();
-          if (rho <= 1.0e-11f) break;  // what these sweeps left is below 1e-17 of b
+          if (rho <= 1.0e-11f) { solved = true; break; }  // what these sweeps left is below 1e-17 of b
           float rm = 0.f;
+          bad = false;
           pass64<N1, GL>(
               args, c,
               [&](int e, double2 (&q)[5]) {  // linearised level quantities of delta
@@ -347,15 +350,17 @@ __global__ void __launch_bounds__(64, 6)
                 for (int v = 0; v < 3; ++v) {
                   const u64x r = to_f((c.w(W_B, v, e) - own[v]) - s[v]);
                   if (c.act) c.B[v * L + l] = r;
-                  rm = fmaxf(rm, wt[v] * fmaxf(fabsf(unpk(r).x), fabsf(unpk(r).y)));
+                  const float2 f = unpk(r);
+                  bad = bad || !(fabsf(f.x) < 3.0e38f) || !(fabsf(f.y) < 3.0e38f);
+                  rm = fmaxf(rm, wt[v] * fmaxf(fabsf(f.x), fabsf(f.y)));
                 }
               });
           rmax = warp_max_bits(rm);
-          rho = bmax > 0.f ? __fdividef(rmax, bmax) : 0.f;
-          if (!(rho < 0.1f)) { give_up = true; break; }
-          if (rho < 1.0e-16f) break;
+          rho = bmax > 0.f ? rmax / bmax : 0.f;
+          if (__any_sync(FULL, bad) || !(rho < 0.1f)) break;
+          if (rho < 1.0e-16f) { solved = true; break; }
         }
-        if (give_up) break;
+        if (!solved) { give_up = true; break; }
         ++nsolve;
         for (int e = 0; e < NeZ; ++e) {
 #pragma unroll
