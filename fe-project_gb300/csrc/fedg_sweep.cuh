@@ -13,8 +13,13 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-__device__ __forceinline__ float warp_max_bits(float e) {  // e >= 0 or NaN (which wins)
-  return __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(e) & 0x7fffffffu));
+// over the GL lanes of a pair; e >= 0 or NaN (which wins)
+template <int GL>
+__device__ __forceinline__ float pair_max_bits(float e) {
+  unsigned v = __float_as_uint(e) & 0x7fffffffu;
+#pragma unroll
+  for (int o = GL / 2; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(FULL, v, o));
+  return __uint_as_float(v);
 }
 
 // One pair of columns: GL >= N1 lanes, lane k < N1 (act) owns node k of every element; the other lanes
@@ -32,11 +37,11 @@ struct SweepCtx {
   __device__ size_t pi(int v, int e) const { return (size_t)v * pn + pb + (size_t)e * ps; }
 };
 
-// One sweep x <- (1 - w) x + w (b - K x), from x = w b if first; returns the lane's largest weighted
+// One sweep x <- (1 - w) x + w (b - K x), from x = w b if first, stored if run; returns the lane's largest weighted
 // change.  (A NaN can drop out of the change; the FP64 residual that follows the sweeps looks at every node.)
 template <int N1, int GL>
 __device__ __forceinline__ float sweep(const SweepCtx<N1, GL>& c, const u64x (&Dk)[N1], const u64x (&Tk)[N1],
-                                       u64x facB, u64x facT, u64x w, u64x w1, float c1, float c2, bool first) {
+                                       u64x facB, u64x facT, u64x w, u64x w1, float c1, float c2, bool first, bool run) {
   constexpr int N = N1 - 1;
   constexpr u64x SG = 0x8000000080000000ull;
   const int L = c.L, NeZ = c.NeZ;
@@ -123,7 +128,7 @@ __device__ __forceinline__ float sweep(const SweepCtx<N1, GL>& c, const u64x (&D
     const u64x nr = xfma(w, xsub(be[0], y0), xmul(w1, xo[0]));
     const u64x nm = xfma(w, xsub(be[1], xadd(y1, z1)), xmul(w1, xo[1]));
     const u64x nh = xfma(w, xsub(be[2], y2), xmul(w1, xo[2]));
-    if (GL == N1 || c.act) {
+    if (run && (GL == N1 || c.act)) {
       c.X[l] = nr;
       c.X[L + l] = nm;
       c.X[2 * L + l] = nh;
@@ -137,28 +142,28 @@ __device__ __forceinline__ float sweep(const SweepCtx<N1, GL>& c, const u64x (&D
   return dmax;
 }
 
-
-// relaxation of a warp's sweeps: w from the wave speed of its first column's lowest face
+// relaxation of a pair's sweeps: w from the wave speed of its lowest face
 template <int N1>
 struct SweepCoef {
   u64x w, w1;
   float wr;
-  __device__ __forceinline__ SweepCoef(const Ops& op, double impl_fac, int k, u64x a0) {
+  __device__ __forceinline__ SweepCoef(const Ops& op, double impl_fac, u64x a0) {
     const float2 a = unpk(a0);
     const float ds = 0.5f * (float)impl_fac * (float)op.Lb[0] * (float)op.FSz * fmaxf(a.x, a.y);
-    wr = __shfl_sync(FULL, 1.f / (1.f + ds), 0);
+    wr = 1.f / (1.f + ds);
     w = pk1(wr);
     w1 = pk1(1.f - wr);
   }
 };
 
 // Sweeps from x = w b until the change that the next one would make (the last change times the observed
-// contraction) is below rel times the first change or below abs.  bmax: the warp's largest weighted |b|
-// (weights 1, c1, c2).  A contraction above 0.4 ends the sweeps: at FP32's floor (a small change already)
-// the result stands, otherwise false is returned and the columns are left to block LU.  Warp-uniform.
+// contraction) is below rel times the first change.  bmax: the pair's largest weighted |b| (weights 1, c1, c2).  A
+// contraction above 0.4 ends the sweeps: at FP32's floor (a small change already) the result stands, otherwise false is
+// returned and the pair is left to block LU.  Each pair stops by itself (run: it takes part at all), so its x does not
+// depend on the warp's other pairs; the result is uniform over its lanes.
 template <int N1, int GL>
 __device__ __forceinline__ bool sweeps(const SweepCtx<N1, GL>& c, const SweepCoef<N1>& sc, const Ops& op, double impl_fac,
-                                       float bmax, float rel, float abs, float c1, float c2) {
+                                       float bmax, float rel, float c1, float c2, bool run) {
   const int k = c.k;
   const float fi = (float)impl_fac;
   const float fdzs = (float)op.E33 * fi;
@@ -170,16 +175,20 @@ __device__ __forceinline__ bool sweeps(const SweepCtx<N1, GL>& c, const SweepCoe
   }
   const u64x facB = pk1(0.5f * fi * (float)op.Lb[k] * (float)op.FSz);
   const u64x facT = pk1(0.5f * fi * (float)op.Lt[k] * (float)op.FSz);
-  const float d0 = sc.wr * bmax, stop = fmaxf(rel * d0, abs);
+  const float d0 = sc.wr * bmax, stop = rel * d0;
   float prev = d0;
+  bool ok = false;
   for (int n = 0; n < 24; ++n) {
-    const float d = warp_max_bits(sweep<N1, GL>(c, Dk, Tk, facB, facT, sc.w, sc.w1, c1, c2, n == 0));
+    const float d = pair_max_bits<GL>(sweep<N1, GL>(c, Dk, Tk, facB, facT, sc.w, sc.w1, c1, c2, n == 0, run));
     const float r = __fdividef(d, prev);
-    if (d * r <= stop || (!(r <= 0.4f) && d <= 1.0e-4f * d0)) return true;
-    if (!(r <= 0.4f) && n >= 2) return false;
+    if (run) {
+      ok = d * r <= stop || (!(r <= 0.4f) && d <= 1.0e-4f * d0);
+      run = !(ok || (!(r <= 0.4f) && n >= 2));
+    }
+    if (!__any_sync(FULL, run)) break;
     prev = d;
   }
-  return false;
+  return ok;
 }
 
 }  // namespace

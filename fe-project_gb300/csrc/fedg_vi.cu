@@ -446,10 +446,11 @@ __global__ void __launch_bounds__(128) k_vi_fp64(const Ops op, const Prof pf, co
 
   for (int pair = slot; pair < npair; pair += gridDim.x * wpb) {
     const int col_h = 2 * pair + h;
-    const bool live = col_h < ncol;  // an odd column count leaves the last half-warp a copy to idle on
-    const int col = live ? col_h : ncol - 1;
-    // redo: only the columns that the refinement kernel marked (a warp's two are marked together)
-    if (redo && !__any_sync(0xffffffffu, status[col] == VI_REDO)) continue;
+    // an odd column count leaves the last half-warp a copy to idle on; redo: only the columns that the refinement
+    // kernel marked are solved and stored
+    const int col = min(col_h, ncol - 1);
+    const bool live = col_h < ncol && !(redo && status[col] != VI_REDO);
+    if (!__any_sync(0xffffffffu, live)) continue;
     const int ij = col % NF, exy = col / NF;
     c.gxy = (size_t)exy * Np + ij % N1 + N1 * (ij / N1);
 

@@ -11,13 +11,15 @@
 // linear system's error from 1e-6 over 1e-12 below 1e-16, where the next FP64 residual has nothing left
 // to see.  That costs about 250 FP64 operations per node with the nonlinear residual.  The pressure
 // deviation PRES_hyd ((1 + DRHOT/RHOT_hyd)^kappa - 1) is its binomial series up to 3 % (13 terms, to
-// roundoff, no cancellation of totals) and pow() beyond.  A warp whose sweeps do not contract, whose Newton
+// roundoff, no cancellation of totals) and pow() beyond.  A pair of columns whose sweeps do not contract, whose Newton
 // does not converge in max_iter solves or whose residual is not finite stores nothing but a mark in
 // `status`; k_vi_fp64, launched after this kernel, solves the marked columns from the start.
 //
 // MOMX/MOMY: Q - q* from the interface jumps, one Thomas sweep per component (see fedg_viseries.cu), in FP64.
 //
-// Layout: GL = 2, 4 or 8 lanes per pair of neighbouring columns, lane k < N1 owns node k of every element.
+// Layout: GL = 2, 4 or 8 lanes per pair of neighbouring columns of an element (the last of an odd number alone), lane
+// k < N1 owns node k of every element.  Relaxation, stopping rules and counts are the pair's own, so a column's result
+// does not depend on which columns share its warp: a decomposed mesh gives the bits of the whole one.
 // FP64 fields of the columns in flight (the iterate, b, delta, the Jacobian's level quantities) sit in a
 // global slice of the warp, 16 bytes per lane and entry, which a persistent grid keeps in L2; the FP32
 // vectors and the exchange of level quantities are in shared memory.
@@ -169,13 +171,13 @@ __device__ __forceinline__ void pass64(const S64Args& args, const Ctx64<N1, GL>&
 template <int N1, int GL>
 __global__ void __launch_bounds__(64, 6)
     k_vi64(const __grid_constant__ Ops op, const Prof pf, const F5c qin, const F5c z, const F5 tout, int* status,
-           const __grid_constant__ S64Args args, int ncol, double* gsc) {
-  constexpr int N = N1 - 1, G = 32 / GL, NF = N1 * N1, Np = NF * N1;
+           const __grid_constant__ S64Args args, double* gsc) {
+  constexpr int N = N1 - 1, G = 32 / GL, NF = N1 * N1, Np = NF * N1, PE = (NF + 1) / 2;  // pairs per element
   extern __shared__ __align__(16) unsigned char smraw[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const int slot = blockIdx.x * wpb + wib, nslot = gridDim.x * wpb;
   const int grp = lane / GL, kl = lane % GL;
-  const int NeZ = op.NeZ, L = op.L, ncp = (ncol + 1) / 2;
+  const int NeZ = op.NeZ, L = op.L, ncp = op.NeX * op.NeY * PE;
   const S64Layout lay(N1, GL, NeZ);
   unsigned char* base = smraw + (size_t)(wib * G + grp) * lay.stride;
   Ctx64<N1, GL> c;
@@ -193,10 +195,10 @@ __global__ void __launch_bounds__(64, 6)
   const int gv[3] = {VD, VMZ, VRT};
 
   for (int p0 = slot * G; p0 < ncp; p0 += nslot * G) {
-    const int cp = min(p0 + grp, ncp - 1), colA = 2 * cp, colB = min(colA + 1, ncol - 1);
-    const bool liveA = p0 + grp < ncp && c.act, liveB = liveA && colB != colA;
-    c.gA = (size_t)(colA / NF) * Np + colA % NF;
-    c.gB = (size_t)(colB / NF) * Np + colB % NF;
+    const int cp = min(p0 + grp, ncp - 1), exy = cp / PE, ij = 2 * (cp - exy * PE), colA = exy * NF + ij, colB = ij + 1 < NF ? colA + 1 : colA;
+    bool liveA = p0 + grp < ncp && c.act, liveB = liveA && colB != colA;
+    c.gA = (size_t)exy * Np + ij;
+    c.gB = c.gA + (colB - colA);
     c.gs = (size_t)op.NeX * op.NeY * Np;
     auto store = [&](int v, int e, double2 x) {
       const size_t o = (size_t)e * c.gs + (size_t)NF * k;
@@ -267,16 +269,17 @@ __global__ void __launch_bounds__(64, 6)
     };
 
     int stA = 0, stB = 0;
-    bool give_up = false;
     if (impl == 0.0) {
       pass64<N1, GL>(args, c, fill, [&](int e, const double2 (&)[3], const double2 (&s)[3]) {
 #pragma unroll
         for (int v = 0; v < 3; ++v) store(gv[v], e, neg2(s[v]));
       });
     } else {
-      // ---- DENS/MOMZ/RHOT Newton ----
-      const SweepCoef<N1> sc(op, impl, k, c.A[0]);
-      bool doneA = !(p0 + grp < ncp), doneB = doneA || colB == colA;
+      // ---- DENS/MOMZ/RHOT Newton; the flags are the pair's, uniform over its lanes ----
+      const SweepCoef<N1> sc(op, impl, c.A[0]);
+      const unsigned group = (GL == 32 ? FULL : ((1u << GL) - 1u)) << (lane & ~(GL - 1));
+      bool run = p0 + grp < ncp, give_up = false;  // run: still iterating
+      bool doneA = !run, doneB = doneA || colB == colA;
       int nsolve = 0;
       while (true) {
         float errA = 0.f, errB = 0.f, bmax = 0.f;
@@ -299,37 +302,48 @@ __global__ void __launch_bounds__(64, 6)
             bmax = fmaxf(bmax, wt[v] * fmaxf(fabsf(f.x), fabsf(f.y)));
           }
         });
-        bmax = warp_max_bits(bmax);
-        if (__any_sync(FULL, bad)) { give_up = true; break; }
+        bmax = pair_max_bits<GL>(bmax);
+        bad = (__ballot_sync(FULL, bad) & group) != 0;
         if (args.v.max_iter > 1) {
 #pragma unroll
           for (int o = GL / 2; o > 0; o >>= 1) {
             errA = fmaxf(errA, __shfl_xor_sync(FULL, errA, o));
             errB = fmaxf(errB, __shfl_xor_sync(FULL, errB, o));
           }
-          if (!doneA && (double)errA <= args.v.tol) { stA = nsolve; doneA = true; }
-          if (!doneB && (double)errB <= args.v.tol) { stB = nsolve; doneB = true; }
-          if (__all_sync(FULL, doneA && doneB)) break;
-          if (nsolve >= args.v.max_iter) { give_up = true; break; }
+          if (run && !bad) {
+            if (!doneA && (double)errA <= args.v.tol) { stA = nsolve; doneA = true; }
+            if (!doneB && (double)errB <= args.v.tol) { stB = nsolve; doneB = true; }
+            bad = !(doneA && doneB) && nsolve >= args.v.max_iter;
+          }
         }
+        if (run) {
+          give_up = bad;
+          run = !bad && !(doneA && doneB);
+        }
+        if (!__any_sync(FULL, run)) break;
         // ---- J delta = b by refinement: rho is the residual's size over b's.  Solved once what the last sweeps
         // left, or the residual itself, is below FP64's roundoff; anything else is left to block LU ----
         float rho = 1.f, rmax = bmax;
-        bool solved = false;
+        bool open = run, solved = false;  // open: still refining
         for (int it = 0; it < 6; ++it) {
           // the sweeps leave rel of their right-hand side; the last ones need not go below FP64's roundoff
           const float rel = fminf(1.0e-3f, fmaxf(1.0e-6f, 1.0e-17f / rho));
-          if (!sweeps<N1, GL>(c, sc, op, impl, rmax, rel, 0.f, args.c1, args.c2)) break;
-          for (int e = 0; e < NeZ; ++e) {
+          open = sweeps<N1, GL>(c, sc, op, impl, rmax, rel, args.c1, args.c2, open);
+          if (open) {
+            for (int e = 0; e < NeZ; ++e) {
 #pragma unroll
-            for (int v = 0; v < 3; ++v) {
-              const float2 x = unpk(c.X[v * L + e * N1 + k]);
-              double2& d = c.w(W_D, v, e);
-              d = it == 0 ? make_double2(x.x, x.y) : make_double2(d.x + x.x, d.y + x.y);
+              for (int v = 0; v < 3; ++v) {
+                const float2 x = unpk(c.X[v * L + e * N1 + k]);
+                double2& d = c.w(W_D, v, e);
+                d = it == 0 ? make_double2(x.x, x.y) : make_double2(d.x + x.x, d.y + x.y);
+              }
+            }
+            if (rho <= 1.0e-11f) {  // what these sweeps left is below 1e-17 of b
+              solved = true;
+              open = false;
             }
           }
-          __syncwarp();
-          if (rho <= 1.0e-11f) { solved = true; break; }  // what these sweeps left is below 1e-17 of b
+          if (!__any_sync(FULL, open)) break;
           float rm = 0.f;
           bad = false;
           pass64<N1, GL>(
@@ -355,19 +369,28 @@ __global__ void __launch_bounds__(64, 6)
                   rm = fmaxf(rm, wt[v] * fmaxf(fabsf(f.x), fabsf(f.y)));
                 }
               });
-          rmax = warp_max_bits(rm);
+          rmax = pair_max_bits<GL>(rm);
           rho = bmax > 0.f ? rmax / bmax : 0.f;
-          if (__any_sync(FULL, bad) || !(rho < 0.1f)) break;
-          if (rho < 1.0e-16f) { solved = true; break; }
+          bad = (__ballot_sync(FULL, bad) & group) != 0;
+          if (open) {
+            solved = !bad && rho < 1.0e-16f;
+            open = !bad && rho < 0.1f && !solved;
+          }
+          if (!__any_sync(FULL, open)) break;
         }
-        if (!solved) { give_up = true; break; }
-        ++nsolve;
-        for (int e = 0; e < NeZ; ++e) {
+        if (run) {
+          run = solved;
+          give_up = !solved;
+          ++nsolve;
+        }
+        if (run) {
+          for (int e = 0; e < NeZ; ++e) {
 #pragma unroll
-          for (int v = 0; v < 3; ++v) {
-            const double2 d = c.w(W_D, v, e);
-            double2& P = c.w(W_P, v, e);
-            P = make_double2(doneA ? P.x : P.x + d.x, doneB ? P.y : P.y + d.y);
+            for (int v = 0; v < 3; ++v) {
+              const double2 d = c.w(W_D, v, e);
+              double2& P = c.w(W_P, v, e);
+              P = make_double2(doneA ? P.x : P.x + d.x, doneB ? P.y : P.y + d.y);
+            }
           }
         }
         __syncwarp();
@@ -376,21 +399,18 @@ __global__ void __launch_bounds__(64, 6)
           break;
         }
       }
-      if (!give_up) {
-        for (int e = 0; e < NeZ; ++e) {
-#pragma unroll
-          for (int v = 0; v < 3; ++v)
-            store(gv[v], e, args.inv_impl * (c.w(W_P, v, e) - c.ldg2(qin.v[gv[v]], e, k)));
-        }
-      }
-    }
-    if (give_up) {  // warp-uniform: block LU for these columns, by the kernel that follows
-      if (c.act && k == 0 && liveA) {
-        status[colA] = VI_REDO;
-        if (liveB) status[colB] = VI_REDO;
+      if (give_up) {  // block LU for these columns, by the kernel that follows
+        if (k == 0 && liveA) status[colA] = VI_REDO;
+        if (k == 0 && liveB) status[colB] = VI_REDO;
+        liveA = liveB = false;
       }
       __syncwarp();
-      continue;
+      if (!__any_sync(FULL, liveA)) continue;
+      for (int e = 0; e < NeZ; ++e) {
+#pragma unroll
+        for (int v = 0; v < 3; ++v)
+          store(gv[v], e, args.inv_impl * (c.w(W_P, v, e) - c.ldg2(qin.v[gv[v]], e, k)));
+      }
     }
 
     // ---- MOMX/MOMY (eval_Ax_uv / solve_uv): beta_ek = cLb[k] A_e, tau_ek = cLt[k] A_{e+1}.  impl_fac = 0: A
@@ -479,7 +499,7 @@ int plan_n(const Ops& op, Plan64& p) {
   }
   if (p.wpb == 0) return 0;  // the columns are too tall: block LU alone
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kfn, 32 * p.wpb, p.smem)) != cudaSuccess) return (int)e;
-  const int ncp = (op.NeX * op.NeY * N1 * N1 + 1) / 2, per = G * p.wpb;
+  const int ncp = op.NeX * op.NeY * ((N1 * N1 + 1) / 2), per = G * p.wpb;
   p.grid = std::max(1, std::min((ncp + per - 1) / per, nb * nsm));
   p.scratch = (size_t)p.grid * p.wpb * s64_slice(op.NeZ);
   return 0;
@@ -488,7 +508,7 @@ int plan_n(const Ops& op, Plan64& p) {
 template <int N1>
 int launch_n(const Plan64& p, const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, const F5& tout, int* status,
              const S64Args& a, double* gsc, cudaStream_t s) {
-  k_vi64<N1, gl_of<N1>()><<<p.grid, 32 * p.wpb, p.smem, s>>>(op, pf, qin, z, tout, status, a, op.NeX * op.NeY * N1 * N1, gsc);
+  k_vi64<N1, gl_of<N1>()><<<p.grid, 32 * p.wpb, p.smem, s>>>(op, pf, qin, z, tout, status, a, gsc);
   return (int)cudaGetLastError();
 }
 

@@ -1,0 +1,55 @@
+"""FP64 column solve: a column's result is its own.
+
+* A strong change of one column's input leaves every other column's tendency bit for bit as it was, but for the column
+  that shares its lanes (columns 2m and 2m + 1 of an element).
+* The parts of a decomposed domain equal the whole domain bit for bit at the orders whose elements do not fill whole
+  warps of columns (test_gpu_slabs.py holds p = 7)."""
+import numpy as np
+import pytest
+
+from conftest import have_gpu
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not have_gpu(), reason="needs a CUDA GPU")]
+
+from fedg import cases  # noqa: E402
+from fedg import lib as fl  # noqa: E402
+from test_gpu_parity import perturbed, to_np  # noqa: E402
+from test_gpu_slabs import _full, _slabs  # noqa: E402
+
+
+@pytest.mark.parametrize("max_iter,tol", [(1, 0.0), (30, 1e-12)])
+@pytest.mark.parametrize("p", [1, 2, 3, 4, 5, 6, 7])
+def test_column_independent_of_the_others(p, max_iter, tol):
+    case = cases.replace(cases.C1().scaled(3, 1, 3, porder=p), eqs="HEVI")
+    q0, b = perturbed(case, 11, amp=0.1)
+    rng = np.random.default_rng(12)
+    q = [a + s * rng.standard_normal(a.shape) for a, s in zip(q0, (1e-5, 0.01, 0.01, 0.01, 0.003))]
+    ctx = fl.Context(case)
+    ctx.set_base_state(b["dens_hyd"], b["pres_hyd"], b["therm_hyd"])
+    NF, ij = (p + 1) ** 2, (p + 1) ** 2 - 1
+    mine = [ij, ij ^ 1] if (ij ^ 1) < NF else [ij]
+    big = [a.copy() for a in q]
+    for v in (0, 3, 4):
+        big[v].reshape(3, 3, p + 1, NF)[:, 1, :, ij] += 300.0 * (q[v] - q0[v]).reshape(3, 3, p + 1, NF)[:, 1, :, ij]
+    got = []
+    for x in (q, big):
+        t, nfail, _ = ctx.cal_vi([ctx.tensor(a) for a in x], [ctx.tensor(a) for a in q0], 1e-3, 1e-3, max_iter, tol, want_status=True)
+        assert nfail == 0
+        got.append([a.reshape(3, 3, p + 1, NF) for a in to_np(t)])
+    for a, r in zip(*got):
+        same = a == r
+        if a is not got[0][1] and a is not got[0][2]:  # MOMX and MOMY do not see the change
+            assert not same[:, 1, :, mine[0]].all()
+        same[:, 1, :, mine] = True
+        assert same.all()
+
+
+@pytest.mark.parametrize("p", [1, 2, 4, 5, 6])
+def test_parts_equal_one_domain(p):
+    case = cases.C2().scaled(4, 2, 3, porder=p)
+    q, b = cases.initial_state(case)
+    opts = dict(eqs=fl.HEVI, prec=fl.PREC_FP64, dt=0.04, max_iter=30, tol=1e-10)
+    want = _full(fl, case, b, q, opts, 3)
+    got = _slabs(fl, case, b, q, opts, 3, (2, 2))
+    for v in range(5):
+        assert np.array_equal(got[v], want[v]), (v, np.abs(got[v] - want[v]).max())
