@@ -39,6 +39,7 @@ struct S64Args {
   double cb[13];     // binomial coefficients C(kappa, n), n = 1 .. 13
   double inv_impl;   // 1 / impl_fac
   float c1, c2;      // weights of MOMZ and RHOT in the sweeps' change
+  float tol_lo, tol_hi;  // tol less and plus 1e-5 of it
 };
 
 // shared memory of one column pair (bytes): the FP32 vectors x and b, the sweeps' exchange slots, the
@@ -166,6 +167,26 @@ __device__ __forceinline__ void pass64(const S64Args& args, const Ctx64<N1, GL>&
     }
     __syncwarp();
   }
+}
+
+// max |b| / scale of a pair's two columns from its planes of b (kept out of line: it hardly ever runs)
+template <int GL>
+__device__ __noinline__ double2 scaled_max(const Prof& pf, double cref, const double2* b, int k, int N1, int NeZ) {
+  double2 x = Z22;
+  for (int e = 0; e < NeZ; ++e) {
+    const double dh = __ldg(pf.dens + e * N1 + k), scale[3] = {dh, dh * cref, __ldg(pf.rhyd + e * N1 + k)};
+#pragma unroll
+    for (int v = 0; v < 3; ++v) {
+      const double2 y = b[((size_t)v * NeZ + e) * 32];
+      x = make_double2(fmax(x.x, fabs(y.x) / scale[v]), fmax(x.y, fabs(y.y) / scale[v]));
+    }
+  }
+#pragma unroll
+  for (int o = GL / 2; o > 0; o >>= 1) {
+    const double2 y = shx(x, o);
+    x = make_double2(fmax(x.x, y.x), fmax(x.y, y.y));
+  }
+  return x;
 }
 
 template <int N1, int GL>
@@ -310,9 +331,19 @@ __global__ void __launch_bounds__(64, 6)
             errA = fmaxf(errA, __shfl_xor_sync(FULL, errA, o));
             errB = fmaxf(errB, __shfl_xor_sync(FULL, errB, o));
           }
+          // The test is in FP64.  errA and errB are right to 1e-6 (above FP32's smallest numbers), so they decide it
+          // outside 1e-5 of tol; the rest takes the FP64 residual that the pass left
+          auto above = [&](float x) { return x > 1.0e-30f && x > args.tol_hi; };
+          auto sure = [&](float x) { return above(x) || (args.tol_lo > 1.0e-30f && x < args.tol_lo); };
+          bool convA = !above(errA), convB = !above(errB);
+          if (__any_sync(FULL, run && !bad && !((doneA || sure(errA)) && (doneB || sure(errB))))) {
+            const double2 x = scaled_max<GL>(pf, args.v.cref, c.W + (size_t)3 * W_B * NeZ * 32 + lane, k, N1, NeZ);
+            convA = x.x <= args.v.tol;
+            convB = x.y <= args.v.tol;
+          }
           if (run && !bad) {
-            if (!doneA && (double)errA <= args.v.tol) { stA = nsolve; doneA = true; }
-            if (!doneB && (double)errB <= args.v.tol) { stB = nsolve; doneB = true; }
+            if (!doneA && convA) { stA = nsolve; doneA = true; }
+            if (!doneB && convB) { stB = nsolve; doneB = true; }
             bad = !(doneA && doneB) && nsolve >= args.v.max_iter;
           }
         }
@@ -560,6 +591,8 @@ int launch_vi64(const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, con
   // MOMZ against 340 m/s of density, RHOT against 300 K of it
   a.c1 = (float)(1.0 / v.cref);
   a.c2 = 1.f / 300.f;
+  a.tol_lo = (float)(v.tol * (1.0 - 1.0e-5));
+  a.tol_hi = (float)(v.tol * (1.0 + 1.0e-5));
   switch (N1) {
     case 2: return launch_n<2>(p, op, pf, qin, z, tout, status, a, gsc, s);
     case 3: return launch_n<3>(p, op, pf, qin, z, tout, status, a, gsc, s);

@@ -2,6 +2,8 @@
 
 * A strong change of one column's input leaves every other column's tendency bit for bit as it was, but for the column
   that shares its lanes (columns 2m and 2m + 1 of an element).
+* The convergence test is an FP64 one: first residuals within 1e-9 of the tolerance, on either side of it, are told apart.
+  From var0 = 0, a state of rest, the first residual is q* itself.
 * The parts of a decomposed domain equal the whole domain bit for bit at the orders whose elements do not fill whole
   warps of columns (test_gpu_slabs.py holds p = 7)."""
 import numpy as np
@@ -42,6 +44,26 @@ def test_column_independent_of_the_others(p, max_iter, tol):
             assert not same[:, 1, :, mine[0]].all()
         same[:, 1, :, mine] = True
         assert same.all()
+
+
+@pytest.mark.parametrize("p", [2, 3, 7])
+def test_tolerance_in_fp64(p):
+    tol = 1e-6
+    case = cases.replace(cases.C1().scaled(3, 3, 2, porder=p), eqs="HEVI")
+    _, b = cases.initial_state(case)
+    NF, rng = (p + 1) ** 2, np.random.default_rng(13)
+    ctx = fl.Context(case)
+    ctx.set_base_state(b["dens_hyd"], b["pres_hyd"], b["therm_hyd"])
+    zero = np.zeros_like(b["dens_hyd"])
+    q = [zero.copy() for _ in range(5)]
+    below = rng.random((9, NF)) < 0.5
+    dens, lev = (a.reshape(2, 9, p + 1, NF) for a in (b["dens_hyd"], q[0]))
+    for e in range(9):
+        for c in range(NF):
+            l, f = rng.integers(0, 2 * (p + 1)), 1.0 + 1e-9 * rng.uniform(0.5, 1.0)
+            lev[l // (p + 1), e, l % (p + 1), c] = tol * dens[l // (p + 1), e, l % (p + 1), c] * (1.0 / f if below[e, c] else f)
+    _, nfail, st = ctx.cal_vi([ctx.tensor(a) for a in q], [ctx.tensor(zero)] * 5, 1e-3, 1e-3, 30, tol, want_status=True)
+    assert nfail == 0 and np.array_equal(st.cpu().numpy().reshape(9, NF) == 0, below)
 
 
 @pytest.mark.parametrize("p", [1, 2, 4, 5, 6])
