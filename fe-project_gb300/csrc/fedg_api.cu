@@ -405,8 +405,10 @@ int fedg_set_base_state(fedg_ctx* c, const double* DENS_hyd, const double* PRES_
     return fail("fedg_set_base_state: base state is not horizontally homogeneous dry air with DPhyd = 0 and constant "
                 "CORIOLIS (" + std::to_string(c->h_cnt[0]) + " mismatching entries)");
   const double p00 = c->op.pres00, rd = c->op.rdry;
+  c->op.cs_max = 0.0;
   for (int l = 0; l < L; ++l) {
     const double pres = hp[L + l], therm = hp[2 * L + l];
+    c->op.cs_max = std::max(c->op.cs_max, std::sqrt(c->op.kap * pres / hp[l]));
     // RHOT_hyd recomputed from PRES_hyd as cal_vi does (hevi_common_2.F90:236-237)
     hp[3 * L + l] = p00 / rd * std::pow(pres / p00, c->op.rgamm);
     hp[4 * L + l] = 1.0 / hp[3 * L + l];

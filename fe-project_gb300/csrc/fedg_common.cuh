@@ -28,6 +28,7 @@ struct Ops {
   double coriolis_f;
   double pb[13];         // binomial coefficients (kap over n), n = 1..13, of the pressure's series
   int pb_on;             // 0: kap outside [1, 2], the series is not used
+  double cs_max;         // largest sound speed of the base state
   int NeX, NeY, NeZ;
   int N1, Np, L;  // L = NeZ*N1 levels
   // part of a decomposed domain: the exterior face layers of the x-, x+, y-, y+ boundaries (receive

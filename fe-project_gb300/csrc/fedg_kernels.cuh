@@ -45,9 +45,20 @@ int launch_vi_fp64(const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, 
                    const ViArgs& a, double* gsc, size_t gsc_doubles, cudaStream_t s);
 
 // Its first pass, by iterative refinement (fedg_vi64.cu): columns it leaves get status VI_REDO and are
-// solved by block LU.  Returns -1, nothing launched, if the columns are too tall for its shared memory or max_iter < 1
-// allows no solve (block LU then reports every column above tol as not converged).
+// solved by block LU.  Returns -1, nothing launched, if the columns are too tall for its shared memory, the base state's
+// Courant number is above vi_courant_max, or max_iter < 1 allows no solve (block LU then reports every column above
+// tol as not converged).
 constexpr int VI_REDO = -100;
+// The sweeps of both first passes (fedg_sweep.cuh, fedg_viseries.cu) contract by a factor that depends on the order and on
+// the face dissipation's diagonal entry d = (impl_fac/2) Lift(0, bottom) Fscale_z c, c the base state's largest sound
+// speed.  Above vi_courant_max, d of the spectral radius 0.58 (of (1 - w) I - w K, computed for columns of 1 to 16
+// elements without gravity), the first pass is not launched: few columns would come out of it.  First pass and block
+// LU, a step of 24x24x16 elements in float pairs at p = 7 in ms: d = 0.65 4.5 and 6.8, d = 0.9 5.7 and 6.8; 16x16x8 in
+// FP64 d = 0.65 5.6 and 18.0; p = 3 in float pairs d = 0.65 0.59 and 0.64, d = 0.81 0.87 and 0.64.
+inline double vi_courant(const Ops& op, double impl_fac) { return 0.5 * impl_fac * op.Lb[0] * op.FSz * op.cs_max; }
+inline double vi_courant_max(int N1) {
+  return N1 == 2 ? 0.40 : N1 == 3 ? 0.53 : N1 == 4 ? 0.65 : N1 == 5 ? 0.72 : N1 == 6 ? 0.78 : N1 == 7 ? 0.83 : 0.90;
+}
 size_t vi64_scratch_doubles(const Ops& op);
 int launch_vi64(const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, const F5& tout, int* status, const ViArgs& a,
                 double* gsc, size_t gsc_doubles, cudaStream_t s);

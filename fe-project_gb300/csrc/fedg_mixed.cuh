@@ -137,7 +137,8 @@ int launch_vi_cols(int N1, const Ops& op, const OpsX& ox, const ProfX& px, const
 // Float-pair column solve by a fixed-point series, a warp per two columns (fedg_viseries.cu): the first
 // pass of the solve from var0; columns it leaves get status VI_REDO and are solved by launch_vi_cols
 // with redo = true.  gsc: as for launch_vi_cols.  hyd: DENS_hyd and RHOT_hyd of the lowest level, smallest
-// DENS_hyd.  Returns -1 if the columns are too tall for its shared memory (nothing launched).
+// DENS_hyd.  Returns -1, nothing launched, if the columns are too tall for its shared memory or the base state's Courant
+// number is above vi_courant_max.
 int launch_vi_series(int N1, const Ops& op, const OpsX& ox, const ProfX& px, const X5& qin, const F5c& z, const A3& a0,
                      void* const* qsf, void* const* tout, float* gsc, int* status, unsigned long long* cnt,
                      const MixViArgs& a, const float hyd[3], cudaStream_t s);

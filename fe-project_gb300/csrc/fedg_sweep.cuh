@@ -157,10 +157,12 @@ struct SweepCoef {
 };
 
 // Sweeps from x = w b until the change that the next one would make (the last change times the observed
-// contraction) is below rel times the first change.  bmax: the pair's largest weighted |b| (weights 1, c1, c2).  A
-// contraction above 0.4 ends the sweeps: at FP32's floor (a small change already) the result stands, otherwise false is
-// returned and the pair is left to block LU.  Each pair stops by itself (run: it takes part at all), so its x does not
-// depend on the warp's other pairs; the result is uniform over its lanes.
+// contraction) is below rel times the first change.  bmax: the pair's largest weighted |b| (weights 1, c1, c2).  The
+// change falls in beats (K's spectrum is complex), so it is held against a geometric envelope, not step to step: above
+// 4 SWEEP_RATE^n of the first change the sweeps end with false and the pair is left to block LU.  At FP32's floor (a
+// small change that falls no more) the result stands.  Each pair stops by itself (run: it takes part at all), so its x
+// does not depend on the warp's other pairs; the result is uniform over its lanes.
+constexpr float SWEEP_RATE = 0.65f;
 template <int N1, int GL>
 __device__ __forceinline__ bool sweeps(const SweepCtx<N1, GL>& c, const SweepCoef<N1>& sc, const Ops& op, double impl_fac,
                                        float bmax, float rel, float c1, float c2, bool run) {
@@ -176,14 +178,15 @@ __device__ __forceinline__ bool sweeps(const SweepCtx<N1, GL>& c, const SweepCoe
   const u64x facB = pk1(0.5f * fi * (float)op.Lb[k] * (float)op.FSz);
   const u64x facT = pk1(0.5f * fi * (float)op.Lt[k] * (float)op.FSz);
   const float d0 = sc.wr * bmax, stop = rel * d0;
-  float prev = d0;
+  float prev = d0, env = 4.f * d0;
   bool ok = false;
-  for (int n = 0; n < 24; ++n) {
+  for (int n = 0; n < 32; ++n) {
     const float d = pair_max_bits<GL>(sweep<N1, GL>(c, Dk, Tk, facB, facT, sc.w, sc.w1, c1, c2, n == 0, run));
     const float r = __fdividef(d, prev);
     if (run) {
-      ok = d * r <= stop || (!(r <= 0.4f) && d <= 1.0e-4f * d0);
-      run = !(ok || (!(r <= 0.4f) && n >= 2));
+      env *= SWEEP_RATE;
+      ok = d * r <= stop || (!(r <= 0.8f) && d <= 1.0e-4f * d0);
+      run = !ok && d <= env;
     }
     if (!__any_sync(FULL, run)) break;
     prev = d;

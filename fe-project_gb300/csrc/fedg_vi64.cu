@@ -567,7 +567,7 @@ int launch_vi64(const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, con
                 double* gsc, size_t gsc_doubles, cudaStream_t s) {
   Plan64 p;
   if (const int r = plan(op, p)) return r;
-  if (p.wpb == 0 || (v.impl_fac != 0.0 && v.max_iter < 1)) return -1;
+  if (p.wpb == 0 || (v.impl_fac != 0.0 && v.max_iter < 1) || vi_courant(op, v.impl_fac) > vi_courant_max(op.N1)) return -1;
   if (!gsc || gsc_doubles < p.scratch) return (int)cudaErrorInvalidValue;
   S64Args a;
   a.v = v;

@@ -43,6 +43,7 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr u64x SG = 0x8000000080000000ull;  // both sign bits
+constexpr float SWEEP_RATE = 0.55f;  // of the sweeps' envelope
 
 // shared memory of one pair (bytes)
 struct SLayout {
@@ -444,8 +445,8 @@ __global__ void __launch_bounds__(128, GLB ? 3 : 4)
       // Sweeps from x = w b until the change that the next one would make (the last change times the
       // observed contraction) is below 2e-6 of the first one, which FP32 resolves to 1e-7 (a later
       // correction goes on from the pair residual), or 2 % of the tolerance, so that what is accepted lies
-      // well inside, as after the LU kernel's corrections.  A contraction above 0.4 is left to the LU
-      // kernel, unless it is FP32's floor.
+      // well inside, as after the LU kernel's corrections.  The change falls in beats (K's spectrum is complex), so it
+      // is held against a geometric envelope: what falls slower is left to the LU kernel, unless it is FP32's floor.
       int c = 0;
       bool ok = false;
       {
@@ -456,13 +457,14 @@ __global__ void __launch_bounds__(128, GLB ? 3 : 4)
         }
         __syncwarp();
         const float d0 = wr * warp_max_bits(bmax), stop = fmaxf(2.0e-6f * d0, ctol);
-        float prev = d0;
+        float prev = d0, env = 4.f * d0;
         for (int it = 0; it < 24; ++it) {
           const float d = warp_max_bits(sweep<N1>(s, K, c, w, w1, args.c1, args.c2));
           c = 1 - c;
           const float r = __fdividef(d, prev);
-          if (d * r <= stop || (!(r <= 0.4f) && d <= 1.0e-4f * d0)) { ok = true; break; }
-          if (!(r <= 0.4f) && it >= 2) break;
+          env *= SWEEP_RATE;
+          if (d * r <= stop || (!(r <= 0.8f) && d <= 1.0e-4f * d0)) { ok = true; break; }
+          if (!(d <= env)) break;
           prev = d;
         }
       }
@@ -605,6 +607,7 @@ __global__ void __launch_bounds__(128, GLB ? 3 : 4)
 template <int N1, bool GLB>
 int launch_n(const Ops& op, const OpsX& ox, const ProfX& px, const X5& qin, const F5c& z, const A3& a0,
              void* const* qsf, void* const* tout, float* gsc, int* status, unsigned long long* cnt, const SerArgs& a, cudaStream_t s) {
+  if (vi_courant(op, a.v.impl_fac) > vi_courant_max(N1)) return -1;
   const SLayout lay(N1, op.NeZ, GLB);
   int wpb = 4;  // neighbouring pairs share 32-byte sectors; fewer where four would leave an SM one block
   while (wpb > 1 && (size_t)lay.stride * wpb > 113 * 1024) wpb /= 2;
