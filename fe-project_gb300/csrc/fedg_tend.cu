@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(EPB* N1* N1* N1, EPB* N1* N1* N1 > 256 ? 2 : 1
   // --- the stage: q_new = A q0 + B q + C t, the last stage's filter, DPRES of q_new ---
   if (valid) {
 #pragma unroll
-    for (int v = 0; v < 5; ++v) out[v] = rk_low(x.A, __ldg(x.q0.v[v] + g), x.B, st[v * Np + p], x.C, out[v]);
+    for (int v = 0; v < 5; ++v) out[v] = rk_low(x.A, x.q0.v[v][g], x.B, st[v * Np + p], x.C, out[v]);
   }
   if (x.filter) {
     double* a = fl;
