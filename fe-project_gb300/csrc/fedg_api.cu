@@ -323,7 +323,8 @@ int fedg_ctx_create(const fedg_mesh_desc* d, fedg_ctx** out) {
   op.NeX = d->NeX; op.NeY = d->NeY; op.NeZ = d->NeZ;
   op.N1 = c->N1; op.Np = c->Np; op.L = c->L;
   cudaError_t e;
-  if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
+  if ((e = cudaDeviceGetAttribute(&op.nsm, cudaDevAttrMultiProcessorCount, d->device)) != cudaSuccess ||
+      (e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
       (e = cudaMalloc(&c->d_prof, sizeof(double) * 8 * c->L)) != cudaSuccess ||
       (e = cudaMalloc(&c->d_status, sizeof(int) * c->ncol)) != cudaSuccess ||
       (e = cudaMalloc(&c->d_cnt, sizeof(unsigned long long) * 4)) != cudaSuccess ||

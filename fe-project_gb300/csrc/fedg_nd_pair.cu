@@ -344,7 +344,7 @@ int nd_pass_n(const NdPass& P, const NdOpsP& op, const double* dp, int Ne, cudaS
                      : go(k_nd_div_p<N1, PPB, NPT, true>, gx, gy, gz, P.ddens, P.dens, P.wall, P.lh, P.lv, P.V);
 }
 
-int nd_pass_p(int N1, const NdPass& P, const NdOpsP& op, const double* dp, int Ne, cudaStream_t s) {
+int nd_pass_p(int N1, int nsm, const NdPass& P, const NdOpsP& op, const double* dp, int Ne, cudaStream_t s) {
   switch (N1) {
     case 2: return nd_pass_n<2, 1>(P, op, dp, Ne, s);
     case 3: return nd_pass_n<3, 1>(P, op, dp, Ne, s);
@@ -356,7 +356,7 @@ int nd_pass_p(int N1, const NdPass& P, const NdOpsP& op, const double* dp, int N
       // Two nodes per thread once the pairs are more than the SMs hold as three blocks of 512 threads.  Gradient +
       // divergence in us, one / two nodes: 20 pairs 16.8 / 21.5, 320 pairs 28.6 / 30.4, 640 pairs
       // 44.5 / 40.8, 1280 pairs 73 / 64.  At p = 3 one node is as good at 10,240 pairs (59) and better at 162 (13 / 20).
-      return (Ne + 1) / 2 > 3 * 152 ? nd_pass_n<8, 2>(P, op, dp, Ne, s) : nd_pass_n<8, 1>(P, op, dp, Ne, s);
+      return (Ne + 1) / 2 > 3 * nsm ? nd_pass_n<8, 2>(P, op, dp, Ne, s) : nd_pass_n<8, 1>(P, op, dp, Ne, s);
   }
   return (int)cudaErrorInvalidValue;
 }
@@ -379,7 +379,7 @@ int numdiff_apply_pair(fedg_ctx* c, double* const q[5], int nlap, double coef_h,
     auto pass = [&](int kind, Src a, Src b, int dens, int wl, double* V) {
       const NdPass P{kind, a, b, q[VD], dens, wl, {Gx, Gy, Gz}, lh, lv, V};
       return tracked(c, FEDG_K_ND, [&] {
-        return nd_pass_p(c->N1, P, kind == 0 ? grad : (kind == 1 ? lap : upd), c->d_prof, c->Ne, c->stream);
+        return nd_pass_p(c->N1, c->op.nsm, P, kind == 0 ? grad : (kind == 1 ? lap : upd), c->d_prof, c->Ne, c->stream);
       });
     };
     const Src qv{q[var], nullptr}, L0{nullptr, lh}, L1{nullptr, lv};

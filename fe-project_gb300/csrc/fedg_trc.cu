@@ -583,12 +583,12 @@ size_t stage_smem() {
 // SMs a third more elements than others (20x20x5 elements, a step: 138 us with four, 131 with two); with many
 // waves four are better (48x48x20 elements, coefficient kernel 259 and 276 us).
 template <int N1>
-bool one_wave(int Ne) { return N1 == 4 && Ne <= 4 * 152 * trc_epb<N1>(); }
+bool one_wave(const Ops& op, int Ne) { return N1 == 4 && Ne <= 4 * op.nsm * trc_epb<N1>(); }
 
 template <int N1, int EPB = trc_epb<N1>()>
 int launch_fct_n(const Ops& op, const double* dp, const TrcIn& in, const TrcFct& fc, int Ne, cudaStream_t s) {
   if constexpr (N1 == 4 && EPB != 2)
-    if (one_wave<N1>(Ne)) return launch_fct_n<N1, 2>(op, dp, in, fc, Ne, s);
+    if (one_wave<N1>(op, Ne)) return launch_fct_n<N1, 2>(op, dp, in, fc, Ne, s);
   constexpr int Np = N1 * N1 * N1;
   const size_t sm = fct_smem<N1, EPB>();
   auto kfn = k_trc_fct<N1, EPB>;
@@ -601,7 +601,7 @@ template <int N1, int EPB = trc_epb<N1>()>
 int launch_stage_n(const Ops& op, const double* dp, const TrcIn& in, const TrcStage& st, const TrcFilt& tf, int Ne,
                    cudaStream_t s) {
   if constexpr (N1 == 4 && EPB != 2)
-    if (one_wave<N1>(Ne)) return launch_stage_n<N1, 2>(op, dp, in, st, tf, Ne, s);
+    if (one_wave<N1>(op, Ne)) return launch_stage_n<N1, 2>(op, dp, in, st, tf, Ne, s);
   constexpr int Np = N1 * N1 * N1;
   const size_t sm = stage_smem<N1, EPB>();
   auto kfn = st.fct_elem ? k_trc_stage<N1, EPB, true> : k_trc_stage<N1, EPB, false>;

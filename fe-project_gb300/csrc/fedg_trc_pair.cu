@@ -478,13 +478,13 @@ int launch_pair_n(bool fct, const TrcOpsP& op, const double* dp, const InP& in, 
                  : go(k_trc_stage_p<N1, PPB, NPS, FEW, false, false>, Np / NPS, sm);
 }
 
-int launch_pair(int N1, bool fct, const TrcOpsP& op, const double* dp, const InP& in, const StageP& st, int Ne,
+int launch_pair(int N1, int nsm, bool fct, const TrcOpsP& op, const double* dp, const InP& in, const StageP& st, int Ne,
                 cudaStream_t s) {
   // FEW: at most a block per SM, which gets the registers of one: coefficient kernel of 20 pairs at p = 7 8.0 us
   // against 9.0, of 162 pairs at p = 3 9.6 against 12.4.  More at p = 7: two nodes per thread in the stage (three
   // stages of 1280 pairs 151 us, one node 181; 320 pairs 71 either way); in the coefficient kernel only
   // from some thousand pairs on (1280 pairs: one node 30 us, two 33; 8192 pairs: 161, 150).
-  const bool few = (Ne + 1) / 2 <= 152 * (N1 == 4 ? ppb_t<4>() : 1);
+  const bool few = (Ne + 1) / 2 <= nsm * (N1 == 4 ? ppb_t<4>() : 1);
 #define FEDG_T(n, f, g, w) launch_pair_n<n, f, g, w>(fct, op, dp, in, st, Ne, s)
   switch (N1) {
     case 2: return FEDG_T(2, 1, 1, false);
@@ -573,9 +573,9 @@ int trc_update_pair(fedg_ctx* c, double* QTRC, const double* const mflx[3], cons
       st.qtrc = QTRC;
       int r = 0;
       if (o->limiter)
-        r = tracked(c, FEDG_K_TRC_FCT, [&] { return launch_pair(N1, true, op, c->d_prof, in, st, c->Ne, c->stream); });
+        r = tracked(c, FEDG_K_TRC_FCT, [&] { return launch_pair(N1, d.nsm, true, op, c->d_prof, in, st, c->Ne, c->stream); });
       if (!r)
-        r = tracked(c, FEDG_K_TRC_TEND, [&] { return launch_pair(N1, false, op, c->d_prof, in, st, c->Ne, c->stream); });
+        r = tracked(c, FEDG_K_TRC_TEND, [&] { return launch_pair(N1, d.nsm, false, op, c->d_prof, in, st, c->Ne, c->stream); });
       if (r) return api_cuda_fail((cudaError_t)r, "fedg_trc_update (pair)");
       qsp = st.q_out;
     }
