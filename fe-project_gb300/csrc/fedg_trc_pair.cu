@@ -483,7 +483,8 @@ int launch_pair(int N1, int nsm, bool fct, const TrcOpsP& op, const double* dp, 
   // FEW: at most a block per SM, which gets the registers of one: coefficient kernel of 20 pairs at p = 7 8.0 us
   // against 9.0, of 162 pairs at p = 3 9.6 against 12.4.  More at p = 7: two nodes per thread in the stage (three
   // stages of 1280 pairs 151 us, one node 181; 320 pairs 71 either way); in the coefficient kernel only
-  // from some thousand pairs on (1280 pairs: one node 30 us, two 33; 8192 pairs: 161, 150).
+  // from some thousand pairs on (a whole step with one node / two: 1280 pairs 257 / 266 us, 3072 542 / 542,
+  // 4224 708 / 697, 8192 1284 / 1252).
   const bool few = (Ne + 1) / 2 <= nsm * (N1 == 4 ? ppb_t<4>() : 1);
 #define FEDG_T(n, f, g, w) launch_pair_n<n, f, g, w>(fct, op, dp, in, st, Ne, s)
   switch (N1) {
