@@ -322,6 +322,7 @@ int fedg_ctx_create(const fedg_mesh_desc* d, fedg_ctx** out) {
   op.pb_on = op.kap >= 1.0 && op.kap <= 2.0;
   op.NeX = d->NeX; op.NeY = d->NeY; op.NeZ = d->NeZ;
   op.N1 = c->N1; op.Np = c->Np; op.L = c->L;
+  op.part = d->periodic_x == FEDG_HALO || d->periodic_y == FEDG_HALO;
   cudaError_t e;
   if ((e = cudaDeviceGetAttribute(&op.nsm, cudaDevAttrMultiProcessorCount, d->device)) != cudaSuccess ||
       (e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||

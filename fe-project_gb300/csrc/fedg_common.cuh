@@ -32,6 +32,7 @@ struct Ops {
   int NeX, NeY, NeZ;
   int N1, Np, L;  // L = NeZ*N1 levels
   int nsm;        // SMs of the device (launch rules)
+  int part;       // 1: one part of a decomposed domain
   // part of a decomposed domain: the exterior face layers of the x-, x+, y-, y+ boundaries (receive
   // buffers of the halo exchange, [6 fields][NeY*NeZ or NeX*NeZ][N1*N1] doubles); NULL where the
   // mesh is periodic in that direction

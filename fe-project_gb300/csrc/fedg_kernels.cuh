@@ -45,9 +45,8 @@ int launch_vi_fp64(const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, 
                    const ViArgs& a, double* gsc, size_t gsc_doubles, cudaStream_t s);
 
 // Its first pass, by iterative refinement (fedg_vi64.cu): columns it leaves get status VI_REDO and are
-// solved by block LU.  Returns -1, nothing launched, if the columns are too tall for its shared memory, the base state's
-// Courant number is above vi_courant_max, or max_iter < 1 allows no solve (block LU then reports every column above
-// tol as not converged).
+// solved by block LU.  Returns -1, nothing launched, if the columns are too tall for its shared memory or block LU serves
+// the call better alone.
 constexpr int VI_REDO = -100;
 // The sweeps of both first passes (fedg_sweep.cuh, fedg_viseries.cu) contract by a factor that depends on the order and on
 // the face dissipation's diagonal entry d = (impl_fac/2) Lift(0, bottom) Fscale_z c, c the base state's largest sound

@@ -558,6 +558,18 @@ int plan(const Ops& op, Plan64& p) {
 
 }  // namespace
 
+// Calls that block LU serves better: no solve allowed; sweeps that do not contract; and at p <= 3 the meshes whose
+// pairs of columns give each scheduler at most one of LU's warps (four per SM).  There this kernel's few warps are
+// held by the length of their chain, while LU's take the time of one.  Step in us, refinement / LU: p = 3, NeZ = 8, 512
+// pairs of columns 797 / 660, 800 pairs 816 / 911, 2048 938 / 1776; p = 2, 288 pairs 1016 / 813, 648 873 / 880, 1152 838 /
+// 896; p = 1, 128 pairs 910 / 574, 2048 1105 / 1196; p = 4, 200 pairs 747 / 774.  Not for a part of a decomposed
+// domain, which has to take what the whole domain takes (bit-equal down to that size).
+static bool block_lu_alone(const Ops& op, const ViArgs& v) {
+  const int pairs = (op.NeX * op.NeY * op.N1 * op.N1 + 1) / 2;
+  return v.max_iter < 1 || vi_courant(op, v.impl_fac) > vi_courant_max(op.N1) ||
+         (op.N1 <= 4 && pairs <= 4 * op.nsm && !op.part);
+}
+
 size_t vi64_scratch_doubles(const Ops& op) {
   Plan64 p;
   return plan(op, p) ? 0 : p.scratch;
@@ -567,7 +579,7 @@ int launch_vi64(const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, con
                 double* gsc, size_t gsc_doubles, cudaStream_t s) {
   Plan64 p;
   if (const int r = plan(op, p)) return r;
-  if (p.wpb == 0 || (v.impl_fac != 0.0 && v.max_iter < 1) || vi_courant(op, v.impl_fac) > vi_courant_max(op.N1)) return -1;
+  if (p.wpb == 0 || (v.impl_fac != 0.0 && block_lu_alone(op, v))) return -1;
   if (!gsc || gsc_doubles < p.scratch) return (int)cudaErrorInvalidValue;
   S64Args a;
   a.v = v;
