@@ -177,14 +177,17 @@ struct FctTab {
 };
 
 // FCT coefficient of the lowest mode, the face fluxes and the signs of their integrals
-template <int N1, int PPB, int NPT, bool FEW>
-__global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, two_minb(PPB * N1 * N1 * N1 / NPT, FEW ? 512 : 1536))
+// how many elements: MANY; FEW, at most a block per SM; SOLO, so few that a block takes one element, not two
+enum TrcMesh { MANY, FEW, SOLO };
+
+template <int N1, int PPB, int NPT, TrcMesh MESH>
+__global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, two_minb(PPB * N1 * N1 * N1 / NPT, MESH != MANY ? 512 : 1536))
     k_trc_fct_p(const __grid_constant__ TrcOpsP op, const double* __restrict__ dens_prof, const InP in, const StageP sp, int Ne) {
   constexpr int Np = N1 * N1 * N1, NF = N1 * N1, NT = Np / NPT, KH = N1 / NPT;
   extern __shared__ p2m smp[];
   FctTab<N1>& T = *reinterpret_cast<FctTab<N1>*>(smp);
   int pair;
-  const TwoIdx x = two_idx<N1, PPB, NT>(op, Ne, pair);
+  const TwoIdx x = two_idx<N1, PPB, NT, MESH == SOLO>(op, Ne, pair);
   p2m* sf = smp + sizeof(FctTab<N1>) / sizeof(p2m) + pair * (6 * NF + 8);
   p2m* out = sf + 6 * NF;
   p2m* red = smp + sizeof(FctTab<N1>) / sizeof(p2m) + PPB * (6 * NF + 8) + pair * (NT + 1);
@@ -283,8 +286,8 @@ __device__ __forceinline__ void contract(p2acc (&s)[NPT], const p2m* D, const p2
 }
 
 // tendency and Runge-Kutta stage; LIM: with the coefficient kernel's outputs
-template <int N1, int PPB, int NPT, bool FEW, bool LIM, bool LAST>
-__global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, two_minb(PPB * N1 * N1 * N1 / NPT, FEW ? 512 : 1280))
+template <int N1, int PPB, int NPT, TrcMesh MESH, bool LIM, bool LAST>
+__global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, two_minb(PPB * N1 * N1 * N1 / NPT, MESH != MANY ? 512 : 1280))
     k_trc_stage_p(const __grid_constant__ TrcOpsP op, const double* __restrict__ dens_prof, const InP in, const StageP sp, int Ne) {
   constexpr int Np = N1 * N1 * N1, NF = N1 * N1, NT = Np / NPT, KH = N1 / NPT;
   extern __shared__ p2m smp[];
@@ -292,7 +295,7 @@ __global__ void __launch_bounds__(PPB* N1* N1* N1 / NPT, two_minb(PPB * N1 * N1 
   LastTab<N1>& TL = *reinterpret_cast<LastTab<N1>*>(smp + sizeof(StageTab<N1>) / sizeof(p2m));
   constexpr int NTAB = (sizeof(StageTab<N1>) + (LAST ? sizeof(LastTab<N1>) : 0)) / sizeof(p2m);
   int pair;
-  const TwoIdx x = two_idx<N1, PPB, NT>(op, Ne, pair);
+  const TwoIdx x = two_idx<N1, PPB, NT, MESH == SOLO>(op, Ne, pair);
   p2m* fl = smp + NTAB + pair * (3 * Np + 6 * NF);
   p2m* df = fl + 3 * Np;
   for (int c = threadIdx.x; c < NF; c += PPB * NT) {
@@ -459,23 +462,23 @@ float2 hsplit(double x) {
 template <int N1>
 constexpr int ppb_t() { return N1 <= 4 ? (N1 == 2 ? 16 : (N1 == 3 ? 4 : 2)) : 1; }
 
-template <int N1, int NPF, int NPS, bool FEW>
+template <int N1, int NPF, int NPS, TrcMesh MESH>
 int launch_pair_n(bool fct, const TrcOpsP& op, const double* dp, const InP& in, const StageP& st, int Ne, cudaStream_t s) {
   constexpr int PPB = ppb_t<N1>(), Np = N1 * N1 * N1, NF = N1 * N1;
-  const int grid = ((Ne + 1) / 2 + PPB - 1) / PPB;
+  const int grid = ((MESH == SOLO ? Ne : (Ne + 1) / 2) + PPB - 1) / PPB;
   auto go = [&](auto kf, int nt, size_t sm) {
     cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     kf<<<grid, PPB * nt, sm, s>>>(op, dp, in, st, Ne);
     return (int)cudaGetLastError();
   };
-  if (fct) return go(k_trc_fct_p<N1, PPB, NPF, FEW>, Np / NPF, sizeof(FctTab<N1>) + sizeof(p2m) * PPB * (6 * NF + 8 + Np / NPF + 1));
+  if (fct) return go(k_trc_fct_p<N1, PPB, NPF, MESH>, Np / NPF, sizeof(FctTab<N1>) + sizeof(p2m) * PPB * (6 * NF + 8 + Np / NPF + 1));
   const size_t sm = sizeof(StageTab<N1>) + (st.last ? sizeof(LastTab<N1>) : 0) + sizeof(p2m) * PPB * (3 * Np + 6 * NF);
   static_assert(3 * Np + 6 * NF >= 2 * (Np + 1), "the sums' workspace");
   if (st.fct)
-    return st.last ? go(k_trc_stage_p<N1, PPB, NPS, FEW, true, true>, Np / NPS, sm)
-                   : go(k_trc_stage_p<N1, PPB, NPS, FEW, true, false>, Np / NPS, sm);
-  return st.last ? go(k_trc_stage_p<N1, PPB, NPS, FEW, false, true>, Np / NPS, sm)
-                 : go(k_trc_stage_p<N1, PPB, NPS, FEW, false, false>, Np / NPS, sm);
+    return st.last ? go(k_trc_stage_p<N1, PPB, NPS, MESH, true, true>, Np / NPS, sm)
+                   : go(k_trc_stage_p<N1, PPB, NPS, MESH, true, false>, Np / NPS, sm);
+  return st.last ? go(k_trc_stage_p<N1, PPB, NPS, MESH, false, true>, Np / NPS, sm)
+                 : go(k_trc_stage_p<N1, PPB, NPS, MESH, false, false>, Np / NPS, sm);
 }
 
 int launch_pair(int N1, int nsm, bool fct, const TrcOpsP& op, const double* dp, const InP& in, const StageP& st, int Ne,
@@ -484,17 +487,21 @@ int launch_pair(int N1, int nsm, bool fct, const TrcOpsP& op, const double* dp, 
   // against 9.0, of 162 pairs at p = 3 9.6 against 12.4.  More at p = 7: two nodes per thread in the stage (three
   // stages of 1280 pairs 151 us, one node 181; 320 pairs 71 either way); in the coefficient kernel only
   // from some thousand pairs on (a whole step with one node / two: 1280 pairs 257 / 266 us, 3072 542 / 542,
-  // 4224 708 / 697, 8192 1284 / 1252).
+  // 4224 708 / 697, 8192 1284 / 1252).  SOLO: half the FP64 sums per SM; a step of 64 elements at p = 7 76.1 us with
+  // pairs, 73.4 with single elements, of 125 and 150 the same either way.
   const bool few = (Ne + 1) / 2 <= nsm * (N1 == 4 ? ppb_t<4>() : 1);
 #define FEDG_T(n, f, g, w) launch_pair_n<n, f, g, w>(fct, op, dp, in, st, Ne, s)
   switch (N1) {
-    case 2: return FEDG_T(2, 1, 1, false);
-    case 3: return FEDG_T(3, 1, 1, false);
-    case 4: return few ? FEDG_T(4, 1, 1, true) : FEDG_T(4, 1, 1, false);
-    case 5: return FEDG_T(5, 1, 1, false);
-    case 6: return FEDG_T(6, 1, 1, false);
-    case 7: return FEDG_T(7, 1, 1, false);
-    case 8: return few ? FEDG_T(8, 1, 1, true) : ((Ne + 1) / 2 <= 4096 ? FEDG_T(8, 1, 2, false) : FEDG_T(8, 2, 2, false));
+    case 2: return FEDG_T(2, 1, 1, MANY);
+    case 3: return FEDG_T(3, 1, 1, MANY);
+    case 4: return few ? FEDG_T(4, 1, 1, FEW) : FEDG_T(4, 1, 1, MANY);
+    case 5: return FEDG_T(5, 1, 1, MANY);
+    case 6: return FEDG_T(6, 1, 1, MANY);
+    case 7: return FEDG_T(7, 1, 1, MANY);
+    case 8:
+      if (2 * Ne <= nsm) return FEDG_T(8, 1, 1, SOLO);
+      if (few) return FEDG_T(8, 1, 1, FEW);
+      return (Ne + 1) / 2 <= 4096 ? FEDG_T(8, 1, 2, MANY) : FEDG_T(8, 2, 2, MANY);
   }
 #undef FEDG_T
   return (int)cudaErrorInvalidValue;

@@ -19,20 +19,21 @@ __device__ __forceinline__ int two_at(int i, int row) {
 // blocks per SM that make up `total` threads
 constexpr int two_minb(int threads, int total) { return total / ((threads + 31) / 32 * 32); }
 
-// the thread's (first) node in elements e[0] and e[1] (e[1] = e[0] where the last element has no partner)
+// the thread's (first) node in elements e[0] and e[1] (e[1] = e[0] where the last element has no partner, or with SOLO
+// none has one)
 struct TwoIdx {
   int e[2], ex[2], ey[2], ez[2], nxy, p, i, j, k;
   bool valid, both;
 };
-template <int N1, int PPB, int NT, class Mesh>
+template <int N1, int PPB, int NT, bool SOLO = false, class Mesh>
 __device__ __forceinline__ TwoIdx two_idx(const Mesh& op, int Ne, int& pair) {
   constexpr int NF = N1 * N1;
   TwoIdx x;
   pair = threadIdx.x / NT;
   x.p = threadIdx.x - pair * NT;
-  const int e0 = 2 * (blockIdx.x * PPB + pair);
+  const int e0 = (SOLO ? 1 : 2) * (blockIdx.x * PPB + pair);
   x.valid = e0 < Ne;
-  x.both = e0 + 1 < Ne;
+  x.both = !SOLO && e0 + 1 < Ne;
   x.nxy = op.NeX * op.NeY;
   x.i = x.p % N1;
   x.j = (x.p / N1) % N1;

@@ -29,6 +29,7 @@ def tracer_step(ctx, Q, q, aM, aP, dt, limiter, prec):
 @pytest.mark.parametrize("p,ne,prec,tol", [
     (3, (19, 13, 10), fl.PREC_FP64, 1e-12),  # four elements per block (2470, the last one half empty)
     (3, (9, 7, 11), fl.PREC_PAIR, 1e-11),    # more than a block per SM (693)
+    (7, (7, 5, 3), fl.PREC_PAIR, 1e-11),     # two elements per block, at most a block per SM (105)
     (7, (7, 9, 5), fl.PREC_PAIR, 1e-11),     # two nodes per thread in the stage (315)
 ])
 @pytest.mark.parametrize("limiter", [True, False])
