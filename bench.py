@@ -48,22 +48,29 @@ PATH_PREC = {"pair": 2, "mixed": 1, "fp64": 0}
 PATH_TOL = {"pair": 1e-13, "mixed": 1e-10, "fp64": 1e-10}
 PATH_ITER = {"pair": 30, "mixed": 20, "fp64": 20}
 PATH_NAME = {"pair": "pair", "mixed": "fp32", "fp64": "plain_fp64"}
-# FP64 instructions per node of the plain column solve (FP32 sweeps, FP64 residuals) at p = 7, measured by ncu: the
-# share of the FP64 pipe's cycles times the time on 16x16x8 elements, about 330 for a launch with one solve and 90
-# for the first stage's evaluation of A; the mean of a step's three launches
-VI64_FP64_INST_PER_NODE = (90 + 330 + 330) / 3
+# FP64 instructions per node of the plain column solve (FP32 sweeps, FP64 residuals) at p = 7, measured by ncu
+# (32 x sm__inst_executed_pipe_fp64.sum on 16x16x8 elements) for the first stage's evaluation of A and for the two
+# solves; the mean of a step's three launches
+VI64_FP64_INST_PER_NODE = 32 * (2.955264e6 + 11.35616e6 + 11.35616e6) / 3 / (16 * 16 * 8 * 512)
 PATH_DTYPE = {"pair": "f32x2", "mixed": "f32+f32x2", "fp64": "f64"}
-# DRAM bytes per node of one launch of the dominant kernel, measured by ncu (dram__bytes_read.sum +
-# dram__bytes_write.sum on 32x32x8 elements of p = 7), per path
+# DRAM bytes per node of one launch, measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum on 32x32x16
+# elements of p = 7, where the launch rules take the same kernels as on the full mesh; the mean of a step's three stage
+# kernels and two column solves), per path
 NCU_BYTES_PER_NODE = {
-    "pair": {"vi_mixed": 934.146542e9 * 714.496e-6 / (32 * 32 * 8 * 512)},
+    "pair": {"stage_mixed": (742.755e6 + 1153.062e6 + 1751.156e6 + 640.495e6 + 1414.554e6 + 636.478e6) / 3 / (32 * 32 * 16 * 512),
+             "vi_mixed": (755.250e6 + 673.302e6 + 755.697e6 + 673.843e6) / 2 / (32 * 32 * 16 * 512)},
 }
 
 
-# warp instructions per node of one launch of the dominant kernel, measured by ncu
-# (smsp__inst_executed.sum on 32x32x8 elements of p = 7), per path
+# warp instructions per node of one launch of the latency-bound kernel, measured by ncu (smsp__inst_executed.sum, the same
+# launches), per path
 NCU_INST_PER_NODE = {
-    "pair": {"vi_mixed": 446.382478e6 / (32 * 32 * 8 * 512)},
+    "pair": {"vi_mixed": (698.956399e6 + 700.108438e6) / 2 / (32 * 32 * 16 * 512)},
+}
+# what limits a kernel that HBM does not, from ncu on the same launches, per path
+NCU_LIMIT = {
+    "pair": {"stage_mixed": "FP32 pipe 55-62 % busy, issue slots 47-52 %, then load latency and barriers",
+             "vi_mixed": "load/store path 69 % busy, issue slots 41 %, FP32 pipe 39 %, load latency"},
 }
 
 
@@ -79,7 +86,7 @@ def issue_roofline(kname, path, nodes, avg_ms, sm_mhz, n_sm):
     peak = 4.0 * n_sm * mhz * 1e6
     return {"bound": "issue", "kernel": kname, "achieved": achieved, "peak": peak, "unit": "warp instructions/s",
             "frac": achieved / peak, "inst_per_node": ipn, "sm_mhz": mhz, "sms": n_sm,
-            "source": "ncu smsp__inst_executed.sum on 32x32x8 elements, scaled by nodes; peak = 4 x SMs x SM clock"}
+            "source": "ncu smsp__inst_executed.sum of the same kernels on 32x32x16 elements, scaled by nodes; peak = 4 x SMs x SM clock"}
 
 
 def max_over_ranks(value, world, device):
@@ -609,8 +616,8 @@ def run_fedg(args):
         # fused stage kernels, mean of the three (FP32 deviation state in, FP64 q^n / q* ):
         # S1 q^n(f32) + q^n(f64) in -> q*_2, S3, SF out; S2 Q_2(f32), t_im, q^n, S3, SF in -> q*_3, SF out;
         # S3 Q_3(f32), t_im, q^n, SF in -> q^n+1 (f64) + its f32 copy out; S1 also writes A(q^n) of
-        # DENS, MOMZ, RHOT (3 pairs) for the column solve's first residual
-        "stage_mixed": (20 + 40 + 40 + 20 + 20 + 20 + 20 + 40 + 20 + 20 + 40 + 20 + 20 + 40 + 20 + 40 + 20 + 24) / 3,
+        # DENS, MOMZ, RHOT (3 pairs) for the column solve's first residual.  In the pair mode every stream is 8 bytes a value
+        "stage_mixed": ((5 * 40 + 24) + 7 * 40 + 6 * 40) / 3 if prec == fl.PREC_PAIR else (20 + 40 + 40 + 20 + 20 + 20 + 20 + 40 + 20 + 20 + 40 + 20 + 20 + 40 + 20 + 40 + 20 + 24) / 3,
         # column solve: q* (float pairs) and var0 (FP64) in -> Q and t_im out, FP32 in the FP32 mode and
         # float pairs in the pair mode; plus the three guess fields (FP32) when the guess is on, else
         # the stage-1 kernel's A(var0) of DENS, MOMZ, RHOT (pairs) for the first residual
@@ -620,13 +627,13 @@ def run_fedg(args):
     avg_ms = ktime / max(klaunch, 1)
     achieved = bytes_per_node.get(kname, 0) * nodes / (avg_ms * 1e-3) / 1e9 if avg_ms > 0 else 0.0
     # DRAM bytes per node of one launch measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum
-    # of the kernel on the 32x32x16-element slice), scaled to this workload's node count
+    # of the kernel on 32x32x16 elements), scaled to this workload's node count
     ncu_bytes_per_node = NCU_BYTES_PER_NODE.get(path, {})
     traffic = ncu_bytes_per_node[kname] * nodes / 1e9 if kname in ncu_bytes_per_node else None
     roof = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peaks.get("hbm_gbs", 6800.0),
             "unit": "GB/s", "frac": achieved / peaks.get("hbm_gbs", 6800.0), "traffic": traffic,
-            "traffic_unit": "GB per launch (ncu DRAM read+write of the same path on a slice of the mesh, scaled by nodes)",
-            "peak_source": peak_src, "avg_launch_ms": avg_ms, "algorithmic_bytes_per_node": bytes_per_node.get(kname)}
+            "traffic_unit": "GB per launch (ncu DRAM read+write of the same kernels on 32x32x16 elements, scaled by nodes)",
+            "limited_by": NCU_LIMIT.get(path, {}).get(kname), "peak_source": peak_src, "avg_launch_ms": avg_ms, "algorithmic_bytes_per_node": bytes_per_node.get(kname)}
     n_sm = torch.cuda.get_device_properties(ctx.dev).multi_processor_count
     roof_issue = issue_roofline(kname, path, nodes, avg_ms, (clocks or {}).get("sm_mhz"), n_sm)
     fp64_tf = fp64_dgemm_tflops(torch, ctx.dev) if rank == 0 else 0.0
@@ -743,8 +750,9 @@ def run_fedg(args):
             plain["roofline_fp64_column_solve"] = {
                 "bound": "fp64", "kernel": "vi_fp64", "achieved_tflops": ach, "peak_tflops": fp64_tf,
                 "frac": ach / fp64_tf, "flop_per_node": fpn, "avg_launch_ms": vt / vn,
-                "flop_count": "FP64 instructions of the refinement solve (ncu), each counted as an FMA; FElib's dense "
-                              "block LU would be about 2000 flop per node and solve"}
+                "flop_count": "the FP64 pipe's instructions (ncu), each counted as an FMA: the fraction is the pipe's "
+                              "use, not achieved flops; FElib's dense block LU would be about 2000 flop per node "
+                              "and solve"}
         ctx.update(q_mix, ncmp, **opts)
         acc = {"steps": ncmp, "rel_l2_vs_plain_fp64": _full_field_errors(np, q_mix, q_ref, dnorm2, dens_hyd, therm_hyd)}
         if other is not None:

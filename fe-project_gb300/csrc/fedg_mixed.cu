@@ -659,7 +659,7 @@ struct MixedState {
   // float-pair mode (FEDG_PREC_PAIR), allocated on first use: S3 | SF | TI | QSF | QNF as pairs
   float2* pbuf = nullptr;
   void** d_pptrs = nullptr;  // device arrays of pointers: TI[5], QSF[5] (pairs)
-  float2* prof5 = nullptr;   // [5][L] DENS_hyd, PRES_hyd, THERM_hyd, 1/THERM_hyd, THERM_hyd/DENS_hyd
+  float2* prof4 = nullptr;   // [4][L] DENS_hyd, PRES_hyd, 1/THERM_hyd, THERM_hyd/DENS_hyd
   // sponge-layer coefficient per level, pairs then FP32 ([L] each), for the (tau, height) in sl_key
   float2* sl2 = nullptr;
   double sl_key[2] = {0.0, 0.0};
@@ -700,7 +700,7 @@ void mixed_free(MixedState* m) {
   cudaFree(m->a0buf);
   cudaFree(m->pbuf);
   cudaFree(m->d_pptrs);
-  cudaFree(m->prof5);
+  cudaFree(m->prof4);
   cudaFree(m->sl2);
   delete m;
 }
@@ -811,9 +811,9 @@ static int pair_setup(fedg_ctx* c, MixedState* m) {
   cudaError_t e;
   if ((e = cudaMalloc(&m->pbuf, sizeof(float2) * 25 * c->n)) != cudaSuccess ||
       (e = cudaMalloc(&m->d_pptrs, sizeof(void*) * 10)) != cudaSuccess ||
-      (e = cudaMalloc(&m->prof5, sizeof(float2) * 5 * L)) != cudaSuccess) {
-    cudaFree(m->pbuf); cudaFree(m->d_pptrs); cudaFree(m->prof5);
-    m->pbuf = nullptr; m->d_pptrs = nullptr; m->prof5 = nullptr;
+      (e = cudaMalloc(&m->prof4, sizeof(float2) * 4 * L)) != cudaSuccess) {
+    cudaFree(m->pbuf); cudaFree(m->d_pptrs); cudaFree(m->prof4);
+    m->pbuf = nullptr; m->d_pptrs = nullptr; m->prof4 = nullptr;
     return api_cuda_fail(e, "fedg_update(pair): allocation");
   }
   const Ops& o = c->op;
@@ -837,18 +837,17 @@ static int pair_setup(fedg_ctx* c, MixedState* m) {
   std::vector<double> hp(4 * L);
   e = cudaMemcpy(hp.data(), c->d_prof, sizeof(double) * 4 * L, cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return api_cuda_fail(e, "fedg_update(pair): profile copy");
-  std::vector<float2> p5(5 * L);
+  std::vector<float2> p4(4 * L);
   for (int l = 0; l < L; ++l) {
-    p5[l] = split_host(hp[l]);
-    p5[L + l] = split_host(hp[L + l]);
-    p5[2 * L + l] = split_host(hp[2 * L + l]);
-    p5[3 * L + l] = split_host(1.0 / hp[2 * L + l]);
-    p5[4 * L + l] = split_host(hp[2 * L + l] / hp[l]);
+    p4[l] = split_host(hp[l]);
+    p4[L + l] = split_host(hp[L + l]);
+    p4[2 * L + l] = split_host(1.0 / hp[2 * L + l]);
+    p4[3 * L + l] = split_host(hp[2 * L + l] / hp[l]);
   }
   void* hptr[10];
   for (int v = 0; v < 5; ++v) hptr[v] = m->TIp(v);
   for (int v = 0; v < 5; ++v) hptr[5 + v] = m->QSFp(v);
-  if ((e = cudaMemcpy(m->prof5, p5.data(), sizeof(float2) * 5 * L, cudaMemcpyHostToDevice)) != cudaSuccess ||
+  if ((e = cudaMemcpy(m->prof4, p4.data(), sizeof(float2) * 4 * L, cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(m->d_pptrs, hptr, sizeof(void*) * 10, cudaMemcpyHostToDevice)) != cudaSuccess)
     return api_cuda_fail(e, "fedg_update(pair): upload");
   return 0;
@@ -967,8 +966,7 @@ static int pair_update_heve(fedg_ctx* c, double* const q[5], int nsteps, const f
   pc.ssp[1] = split_host(0.25);
   pc.ssp[2] = split_host(1.0 / 3.0);
   pc.ssp[3] = split_host(2.0 / 3.0);
-  ProfP pfp{m->prof5, m->prof5 + c->L, m->prof5 + 2 * c->L, m->prof5 + 3 * c->L, m->prof5 + 4 * c->L,
-            m->prof + c->L};
+  ProfP pfp{m->prof4, m->prof4 + c->L, m->prof4 + 2 * c->L, m->prof4 + 3 * c->L, m->prof + c->L};
   if ((r = set_sponge_prof(c, m, nullptr, &pfp))) return r;
   StagePairBufs BP;
   std::memset(&BP, 0, sizeof(BP));
@@ -1116,8 +1114,7 @@ int mixed_update(fedg_ctx* c, double* const q[5], int nsteps, const fedg_update_
   pc.s3e = split_host(o->dt * (1.0 - alp)); pc.s3i = split_host(o->dt * del);
   pc.q2e = split_host(o->dt * alp); pc.q2i = split_host(o->dt * del);
   pc.sf1 = pc.sf2 = split_host(o->dt * del); pc.sf3 = split_host(o->dt * gam);
-  ProfP pfp{m->prof5, m->prof5 + c->L, m->prof5 + 2 * c->L, m->prof5 + 3 * c->L, m->prof5 + 4 * c->L,
-            m->prof + c->L};
+  ProfP pfp{m->prof4, m->prof4 + c->L, m->prof4 + 2 * c->L, m->prof4 + 3 * c->L, m->prof + c->L};
   if ((r = set_sponge_prof(c, m, &pff, &pfp))) return r;
   StagePairBufs BP;
   std::memset(&BP, 0, sizeof(BP));

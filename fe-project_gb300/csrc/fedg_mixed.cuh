@@ -88,7 +88,7 @@ struct OpsP {
 };
 // base-state profiles for the pair stage kernels, [L] each
 struct ProfP {
-  const float2 *dh, *ph, *th, *rth, *ptr;  // DENS_hyd, PRES_hyd, THERM_hyd, 1/THERM_hyd, THERM_hyd/DENS_hyd
+  const float2 *dh, *ph, *rth, *ptr;        // DENS_hyd, PRES_hyd, 1/THERM_hyd, THERM_hyd/DENS_hyd
   const float* phf;                         // PRES_hyd in FP32 (wave speed)
   const float2* sl = nullptr;               // sponge-layer coefficient per level (NULL: no sponge)
   float sl_h = 0.f;                         // 1: the sponge also damps MOMX/MOMY
@@ -136,7 +136,8 @@ int launch_vi_cols(int N1, const Ops& op, const OpsX& ox, const ProfX& px, const
 
 // Float-pair column solve by a fixed-point series, a warp per two columns (fedg_viseries.cu): the first
 // pass of the solve from var0; columns it leaves get status VI_REDO and are solved by launch_vi_cols
-// with redo = true.  gsc: as for launch_vi_cols.  hyd: DENS_hyd and RHOT_hyd of the lowest level, smallest
+// with redo = true.  Their outputs may have been stored in part, and launch_vi_cols reads the inputs again: qsf and tout
+// must not overlap qin, z or a0.  gsc: as for launch_vi_cols.  hyd: DENS_hyd and RHOT_hyd of the lowest level, smallest
 // DENS_hyd.  Returns -1, nothing launched, if the columns are too tall for its shared memory or the base state's Courant
 // number is above vi_courant_max.
 int launch_vi_series(int N1, const Ops& op, const OpsX& ox, const ProfX& px, const X5& qin, const F5c& z, const A3& a0,

@@ -10,8 +10,8 @@
 //     compensated sums of exact products, divisions are pair reciprocals;
 //   - sums of two or three FP64 inputs (densities, mass flux and Rusanov coefficient) are taken in FP64, whose
 //     pipe is otherwise idle here, and split once.
-// Why: the FP64 kernels keep GB300's FP64 pipe ~86 % busy at ~80 FP64 instructions per node and
-// launch; the FP32 pipe has 64x its issue rate.  The pair path is FP64-class (relative rounding
+// Why: the FP64 kernels keep GB300's FP64 pipe 77 % (coefficient) and 90 % (stage) busy at 30 and 64 to 84 FP64
+// instructions per node and launch; the FP32 pipe has 64x its issue rate.  The pair path is FP64-class (relative rounding
 // ~1e-14), not bit-identical: the reciprocal replaces FP64 division, and the FCT face selection
 // 0.5 (R+ + R- - (R+ - R-) sign) is taken exactly as R- or R+.
 //

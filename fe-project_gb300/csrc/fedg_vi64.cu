@@ -9,11 +9,13 @@
 // delta += S (b - J delta), where S is a series of packed FP32 sweeps (fedg_sweep.cuh) that leaves about 1e-6
 // of its right-hand side, and b - J delta is formed in FP64 from the FP64 delta: two such residuals take the
 // linear system's error from 1e-6 over 1e-12 below 1e-16, where the next FP64 residual has nothing left
-// to see.  That costs about 250 FP64 operations per node with the nonlinear residual.  The pressure
+// to see; a system for which the residual does not say so is not taken as solved.  That costs 346 FP64 instructions per
+// node for a launch with one solve and its nonlinear residuals.  The pressure
 // deviation PRES_hyd ((1 + DRHOT/RHOT_hyd)^kappa - 1) is its binomial series up to 3 % (13 terms, to
 // roundoff, no cancellation of totals) and pow() beyond.  A pair of columns whose sweeps do not contract, whose Newton
 // does not converge in max_iter solves or whose residual is not finite stores nothing but a mark in
-// `status`; k_vi_fp64, launched after this kernel, solves the marked columns from the start.
+// `status`; k_vi_fp64, launched after this kernel, solves the marked columns from the start, and all of them where
+// block_lu_alone says so.
 //
 // MOMX/MOMY: Q - q* from the interface jumps, one Thomas sweep per component (see fedg_viseries.cu), in FP64.
 //
@@ -24,7 +26,8 @@
 // global slice of the warp, 16 bytes per lane and entry, which a persistent grid keeps in L2; the FP32
 // vectors and the exchange of level quantities are in shared memory.
 //
-// What bounds it: the FP64 pipe, 67 % busy (p = 7, 16x16x8 elements: 887 us per launch; block LU 4562 us).
+// What bounds it: the FP64 pipe, 69 % busy (p = 7, 16x16x8 elements: 968 us per launch, A(var0) alone 254 us; block LU
+// 4562 us); on small meshes the length of a warp's chain (93,000 instructions for 8 elements of p = 3).
 #include <algorithm>
 
 #include "fedg_kernels.cuh"

@@ -4,15 +4,16 @@
 // Same problem, residual and convergence test as k_vi_cols (fedg_vicol.cu; FElib's cal_vi,
 // scale_atm_dyn_dgm_nonhydro3d_rhot_hevi.F90:772-965, hevi_common_2.F90): Q - q* - impl_fac A(Q) = 0 for
 // the vertical operator A with the Rusanov speed frozen at var0, accepted only on the float-pair
-// residual.  What differs is how a correction J delta = b, J = I + K, is solved.  At the vertical
-// Courant numbers the explicit horizontal terms allow, ||K|| is well below one (about 0.26 on the
+// residual.  What differs is how a correction J delta = b, J = I + K, is solved: on elements about as tall as
+// wide, whose step the explicit horizontal terms set, ||K|| is well below one (about 0.26 on the
 // 128x128x16 p = 7 mesh at dt 0.005 s), and the fixed point x <- (1 - w) x + w (b - K x) reaches FP32
 // accuracy in about ten products K x, none of which needs the block-Thomas history, the element LU or
 // its shuffles.  w = 1 / (1 + d), d the face dissipation's diagonal entry: K's spectrum is the
-// dissipation's [0, 2 d] plus an almost imaginary acoustic part, and w centres it.  A warp whose
-// iteration does not contract, or whose Newton does not converge within the caller's limit, writes
-// nothing but a mark in `status`; k_vi_cols, launched after this kernel, solves the marked columns by
-// block LU from the start, so what it accepts or reports as failed is as before.
+// dissipation's [0, 2 d] plus an almost imaginary acoustic part, and w centres it.  On flat elements d grows; above
+// vi_courant_max the kernel is not launched.  A warp whose iteration does not contract, or whose Newton does not
+// converge within the caller's limit, leaves a mark in `status`; k_vi_cols, launched after this kernel, solves the
+// marked columns by block LU from the start.  From the second correction on such a warp has stored outputs already
+// (`emitted`); block LU overwrites them, and no output overlaps an input.
 //
 // MOMX/MOMY: E = Q - q* is a combination of the two interface jumps of each element,
 // E_ek = -beta_ek J_e + tau_ek J_{e+1}, and the jumps solve a scalar tridiagonal system with the jumps
@@ -29,7 +30,8 @@
 //
 // What bounds it (p = 7, 32x32x8 elements, 715 us per launch): the load/store path at 71 % -- half of its
 // wavefronts are the broadcast reads of the derivative, half the global accesses, where each lane's level is
-// on a line of its own -- with the issue slots at 50 % and the FMA pipe at 42 %.  A walk along the columns
+// on a line of its own -- with the issue slots at 50 % and the FMA pipe at 42 %.  With b and the Jacobian in global
+// scratch (32x32x16, 1381 us) 69, 41 and 39 %, and the load latency with three blocks per SM.  A walk along the columns
 // (one lane per node of an element, the element loop serial) took 760 us there and 100 instead of 24 us
 // for 8x8x8 elements of p = 3, where it is one warp's dependent chain.
 #include <algorithm>

@@ -148,7 +148,8 @@ int fedg_tint_advance(fedg_tint* t, int stage, double* const q[5]);           /*
  *   FEDG_PREC_MIXED: FP32 explicit arithmetic on deviations from the hydrostatic state and the
  *     reference wind; the Newton iterate, its certifying residual and the RK accumulation in
  *     float pairs (about 48 bits); FP32 Jacobian and LU.
- *   FEDG_PREC_PAIR: as FEDG_PREC_MIXED with the explicit operator also in float pairs.
+ *   FEDG_PREC_PAIR: as FEDG_PREC_MIXED with the explicit operator also in float pairs, and the FP32
+ *     corrections of the column solve by a fixed-point series where it contracts, else by that LU.
  *     It is FP64-class end to end; use it with a Newton tol near 1e-13, so the FP32
  *     corrections are refined to pair accuracy.  With eqs FEDG_HEVE: the three SSP-RK3 stages in
  *     float pairs (no implicit solve; use_guess must be 0, iters_out is 0).
