@@ -14,6 +14,10 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
+// the larger of |a| and |b|; NaN wins
+__device__ __forceinline__ float max_bits(float a, float b) {
+  return __uint_as_float(max(__float_as_uint(a) & 0x7fffffffu, __float_as_uint(b) & 0x7fffffffu));
+}
 // over the GL lanes of a pair; e >= 0 or NaN (which wins)
 template <int GL>
 __device__ __forceinline__ float pair_max_bits(float e) {

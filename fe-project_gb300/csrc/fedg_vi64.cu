@@ -301,13 +301,11 @@ __global__ void __launch_bounds__(64, 6)
     } else {
       // ---- DENS/MOMZ/RHOT Newton; the flags are the pair's, uniform over its lanes ----
       const SweepCoef<N1> sc(op, impl, c.A[0]);
-      const unsigned group = (GL == 32 ? FULL : ((1u << GL) - 1u)) << (lane & ~(GL - 1));
       bool run = p0 + grp < ncp, give_up = false;  // run: still iterating
       bool doneA = !run, doneB = doneA || colB == colA;
       int nsolve = 0;
       while (true) {
         float errA = 0.f, errB = 0.f, bmax = 0.f;
-        bool bad = false;
         pass64<N1, GL>(args, c, fill, [&](int e, const double2 (&own)[3], const double2 (&s)[3]) {
           const int l = e * N1 + k;
           const float dh = (float)__ldg(pf.dens + l), rh = (float)__ldg(pf.rhyd + l);
@@ -322,12 +320,11 @@ __global__ void __launch_bounds__(64, 6)
             const float2 f = unpk(bf);
             errA = fmaxf(errA, fabsf(f.x) * isc[v]);
             errB = fmaxf(errB, fabsf(f.y) * isc[v]);
-            bad = bad || !(fabsf(f.x) < 3.0e38f) || !(fabsf(f.y) < 3.0e38f);
-            bmax = fmaxf(bmax, wt[v] * fmaxf(fabsf(f.x), fabsf(f.y)));
+            bmax = max_bits(bmax, max_bits(wt[v] * f.x, wt[v] * f.y));
           }
         });
         bmax = pair_max_bits<GL>(bmax);
-        bad = (__ballot_sync(FULL, bad) & group) != 0;
+        bool bad = !(bmax < 3.0e38f);
         if (args.v.max_iter > 1) {
 #pragma unroll
           for (int o = GL / 2; o > 0; o >>= 1) {
@@ -379,7 +376,6 @@ __global__ void __launch_bounds__(64, 6)
           }
           if (!__any_sync(FULL, open)) break;
           float rm = 0.f;
-          bad = false;
           pass64<N1, GL>(
               args, c,
               [&](int e, double2 (&q)[5]) {  // linearised level quantities of delta
@@ -399,16 +395,14 @@ __global__ void __launch_bounds__(64, 6)
                   const u64x r = to_f((c.w(W_B, v, e) - own[v]) - s[v]);
                   if (c.act) c.B[v * L + l] = r;
                   const float2 f = unpk(r);
-                  bad = bad || !(fabsf(f.x) < 3.0e38f) || !(fabsf(f.y) < 3.0e38f);
-                  rm = fmaxf(rm, wt[v] * fmaxf(fabsf(f.x), fabsf(f.y)));
+                  rm = max_bits(rm, max_bits(wt[v] * f.x, wt[v] * f.y));
                 }
               });
           rmax = pair_max_bits<GL>(rm);
-          rho = bmax > 0.f ? rmax / bmax : 0.f;
-          bad = (__ballot_sync(FULL, bad) & group) != 0;
-          if (open) {
-            solved = !bad && rho < 1.0e-16f;
-            open = !bad && rho < 0.1f && !solved;
+          rho = bmax > 0.f ? rmax / bmax : rmax;
+          if (open) {  // NaN: neither
+            solved = rho < 1.0e-16f;
+            open = rho < 0.1f && !solved;
           }
           if (!__any_sync(FULL, open)) break;
         }
