@@ -14,14 +14,11 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-// the larger of |a| and |b|; NaN wins
-__device__ __forceinline__ float max_bits(float a, float b) {
-  return __uint_as_float(max(__float_as_uint(a) & 0x7fffffffu, __float_as_uint(b) & 0x7fffffffu));
-}
+// running maximum of w |a|, w > 0, as the bits of a non-negative float; NaN wins
+__device__ __forceinline__ void max_bits(unsigned& m, float w, float a) { m = max(m, __float_as_uint(w * fabsf(a))); }
 // over the GL lanes of a pair; e >= 0 or NaN (which wins)
 template <int GL>
-__device__ __forceinline__ float pair_max_bits(float e) {
-  unsigned v = __float_as_uint(e) & 0x7fffffffu;
+__device__ __forceinline__ float pair_max_bits(unsigned v) {
 #pragma unroll
   for (int o = GL / 2; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(FULL, v, o));
   return __uint_as_float(v);
@@ -42,11 +39,11 @@ struct SweepCtx {
   __device__ size_t pi(int v, int e) const { return (size_t)v * pn + pb + (size_t)e * ps; }
 };
 
-// One sweep x <- (1 - w) x + w (b - K x), from x = w b if first, stored if run; returns the lane's largest weighted
-// change.  (A NaN can drop out of the change; the FP64 residual that follows the sweeps looks at every node.)
+// One sweep x <- (1 - w) x + w (b - K x), from x = w b if first, stored for the columns in `run` (bit 0: A, 1: B); returns
+// the lane's largest weighted change in each column.  (A NaN can drop out of the change; the FP64 residual that follows the sweeps looks at every node.)
 template <int N1, int GL>
-__device__ __forceinline__ float sweep(const SweepCtx<N1, GL>& c, const u64x (&Dk)[N1], const u64x (&Tk)[N1],
-                                       u64x facB, u64x facT, u64x w, u64x w1, float c1, float c2, bool first, bool run) {
+__device__ __forceinline__ float2 sweep(const SweepCtx<N1, GL>& c, const u64x (&Dk)[N1], const u64x (&Tk)[N1],
+                                       u64x facB, u64x facT, u64x w, u64x w1, float c1, float c2, bool first, int run) {
   constexpr int N = N1 - 1;
   constexpr u64x SG = 0x8000000080000000ull;
   const int L = c.L, NeZ = c.NeZ;
@@ -73,8 +70,9 @@ __device__ __forceinline__ float sweep(const SweepCtx<N1, GL>& c, const u64x (&D
   load(0);
   put(0);
   if (NeZ > 1) load(1);
+  const u64x upd = (run & 1 ? 0xffffffffull : 0ull) | (run & 2 ? 0xffffffffull << 32 : 0ull);  // columns to store
   u64x pr = 0, pm = 0, pp = 0, pt = 0, ph = 0;  // node N of the element below
-  float dmax = 0.f;
+  float2 dmax = make_float2(0.f, 0.f);
   for (int e = 0; e < NeZ; ++e) {
     u64x xo[3], be[3];  // this element's x and b
 #pragma unroll
@@ -133,44 +131,55 @@ __device__ __forceinline__ float sweep(const SweepCtx<N1, GL>& c, const u64x (&D
     const u64x nr = xfma(w, xsub(be[0], y0), xmul(w1, xo[0]));
     const u64x nm = xfma(w, xsub(be[1], xadd(y1, z1)), xmul(w1, xo[1]));
     const u64x nh = xfma(w, xsub(be[2], y2), xmul(w1, xo[2]));
-    if (run && (GL == N1 || c.act)) {
-      c.X[l] = nr;
-      c.X[L + l] = nm;
-      c.X[2 * L + l] = nh;
+    if (GL == N1 || c.act) {  // a column that has stopped keeps its x
+      c.X[l] = (nr & upd) | (xo[0] & ~upd);
+      c.X[L + l] = (nm & upd) | (xo[1] & ~upd);
+      c.X[2 * L + l] = (nh & upd) | (xo[2] & ~upd);
     }
     const float2 a = unpk(xsub(nr, xo[0])), b = unpk(xsub(nm, xo[1])), d = unpk(xsub(nh, xo[2]));
-    const float ma = fmaxf(fmaxf(fabsf(a.x), c1 * fabsf(b.x)), c2 * fabsf(d.x));
-    const float mb = fmaxf(fmaxf(fabsf(a.y), c1 * fabsf(b.y)), c2 * fabsf(d.y));
-    dmax = fmaxf(dmax, fmaxf(ma, mb));
+    dmax.x = fmaxf(dmax.x, fmaxf(fmaxf(fabsf(a.x), c1 * fabsf(b.x)), c2 * fabsf(d.x)));
+    dmax.y = fmaxf(dmax.y, fmaxf(fmaxf(fabsf(a.y), c1 * fabsf(b.y)), c2 * fabsf(d.y)));
     __syncwarp();
   }
   return dmax;
 }
 
-// relaxation of a pair's sweeps: w from the wave speed of its lowest face
+// relaxation of the two columns' sweeps: w from the wave speed of each one's lowest face
 template <int N1>
 struct SweepCoef {
   u64x w, w1;
-  float wr;
+  float2 wr;
   __device__ __forceinline__ SweepCoef(const Ops& op, double impl_fac, u64x a0) {
     const float2 a = unpk(a0);
-    const float ds = 0.5f * (float)impl_fac * (float)op.Lb[0] * (float)op.FSz * fmaxf(a.x, a.y);
-    wr = 1.f / (1.f + ds);
-    w = pk1(wr);
-    w1 = pk1(1.f - wr);
+    const float f = 0.5f * (float)impl_fac * (float)op.Lb[0] * (float)op.FSz;
+    wr = make_float2(1.f / (1.f + f * a.x), 1.f / (1.f + f * a.y));
+    w = pk(wr.x, wr.y);
+    w1 = pk(1.f - wr.x, 1.f - wr.y);
   }
 };
 
 // Sweeps from x = w b until the change that the next one would make (the last change times the observed
-// contraction) is below rel times the first change.  bmax: the pair's largest weighted |b| (weights 1, c1, c2).  The
+// contraction) is below rel times the first change.  bmax: the columns' largest weighted |b| (weights 1, c1, c2).  The
 // change falls in beats (K's spectrum is complex), so it is held against a geometric envelope, not step to step: above
-// 4 SWEEP_RATE^n of the first change the sweeps end with false and the pair is left to block LU.  At FP32's floor (a
-// small change that falls no more) the result stands.  Each pair stops by itself (run: it takes part at all), so its x
-// does not depend on the warp's other pairs; the result is uniform over its lanes.
+// 4 SWEEP_RATE^n of the first change the column's sweeps end and it is left to block LU.  At FP32's floor (a
+// small change that falls no more) the result stands.  Each column in `run` (bit 0: A, 1: B) stops by itself, so its x
+// does not depend on the warp's other columns; returns those that came to the end, uniform over a pair's lanes.
 constexpr float SWEEP_RATE = 0.65f;
+struct SweepStop {
+  float d0, stop, prev, env;
+  __device__ __forceinline__ SweepStop(float wr, float bmax, float rel) : d0(wr * bmax), stop(rel * d0), prev(d0), env(4.f * d0) {}
+  // 0: go on, 1: done, 2: given up
+  __device__ __forceinline__ int step(float d) {
+    const float r = __fdividef(d, prev);
+    prev = d;
+    env *= SWEEP_RATE;
+    if (d * r <= stop || (!(r <= 0.8f) && d <= 1.0e-4f * d0)) return 1;
+    return d <= env ? 0 : 2;
+  }
+};
 template <int N1, int GL>
-__device__ __forceinline__ bool sweeps(const SweepCtx<N1, GL>& c, const SweepCoef<N1>& sc, const Ops& op, double impl_fac,
-                                       float bmax, float rel, float c1, float c2, bool run) {
+__device__ __forceinline__ int sweeps(const SweepCtx<N1, GL>& c, const SweepCoef<N1>& sc, const Ops& op, double impl_fac,
+                                      float2 bmax, float2 rel, float c1, float c2, int run) {
   const int k = c.k;
   const float fi = (float)impl_fac;
   const float fdzs = (float)op.E33 * fi;
@@ -182,19 +191,14 @@ __device__ __forceinline__ bool sweeps(const SweepCtx<N1, GL>& c, const SweepCoe
   }
   const u64x facB = pk1(0.5f * fi * (float)op.Lb[k] * (float)op.FSz);
   const u64x facT = pk1(0.5f * fi * (float)op.Lt[k] * (float)op.FSz);
-  const float d0 = sc.wr * bmax, stop = rel * d0;
-  float prev = d0, env = 4.f * d0;
-  bool ok = false;
+  SweepStop sa(sc.wr.x, bmax.x, rel.x), sb(sc.wr.y, bmax.y, rel.y);
+  int ok = 0;
   for (int n = 0; n < 32; ++n) {
-    const float d = pair_max_bits<GL>(sweep<N1, GL>(c, Dk, Tk, facB, facT, sc.w, sc.w1, c1, c2, n == 0, run));
-    const float r = __fdividef(d, prev);
-    if (run) {
-      env *= SWEEP_RATE;
-      ok = d * r <= stop || (!(r <= 0.8f) && d <= 1.0e-4f * d0);
-      run = !ok && d <= env;
-    }
+    const float2 d = sweep<N1, GL>(c, Dk, Tk, facB, facT, sc.w, sc.w1, c1, c2, n == 0, run);
+    const int a = sa.step(pair_max_bits<GL>(__float_as_uint(d.x))), b = sb.step(pair_max_bits<GL>(__float_as_uint(d.y)));
+    ok |= run & ((a == 1 ? 1 : 0) | (b == 1 ? 2 : 0));
+    run &= (a == 0 ? 1 : 0) | (b == 0 ? 2 : 0);
     if (!__any_sync(FULL, run)) break;
-    prev = d;
   }
   return ok;
 }

@@ -12,16 +12,16 @@
 // to see; a system for which the residual does not say so is not taken as solved.  That costs 346 FP64 instructions per
 // node for a launch with one solve and its nonlinear residuals.  The pressure
 // deviation PRES_hyd ((1 + DRHOT/RHOT_hyd)^kappa - 1) is its binomial series up to 3 % (13 terms, to
-// roundoff, no cancellation of totals) and pow() beyond.  A pair of columns whose sweeps do not contract, whose Newton
+// roundoff, no cancellation of totals) and pow() beyond.  A column whose sweeps do not contract, whose Newton
 // does not converge in max_iter solves or whose residual is not finite stores nothing but a mark in
 // `status`; k_vi_fp64, launched after this kernel, solves the marked columns from the start, and all of them where
 // block_lu_alone says so.
 //
 // MOMX/MOMY: Q - q* from the interface jumps, one Thomas sweep per component (see fedg_viseries.cu), in FP64.
 //
-// Layout: GL = 2, 4 or 8 lanes per pair of neighbouring columns of an element (the last of an odd number alone), lane
-// k < N1 owns node k of every element.  Relaxation, stopping rules and counts are the pair's own, so a column's result
-// does not depend on which columns share its warp: a decomposed mesh gives the bits of the whole one.
+// Layout: GL = 2, 4 or 8 lanes per pair of neighbouring columns, lane k < N1 owns node k of every element.  Relaxation,
+// stopping rules and counts are the column's own, so its result does not depend on which columns share its lanes or its
+// warp: a decomposed mesh gives the bits of the whole one.
 // FP64 fields of the columns in flight (the iterate, b, delta, the Jacobian's level quantities) sit in a
 // global slice of the warp, 16 bytes per lane and entry, which a persistent grid keeps in L2; the FP32
 // vectors and the exchange of level quantities are in shared memory.
@@ -195,13 +195,13 @@ __device__ __noinline__ double2 scaled_max(const Prof& pf, double cref, const do
 template <int N1, int GL>
 __global__ void __launch_bounds__(64, 6)
     k_vi64(const __grid_constant__ Ops op, const Prof pf, const F5c qin, const F5c z, const F5 tout, int* status,
-           const __grid_constant__ S64Args args, double* gsc) {
-  constexpr int N = N1 - 1, G = 32 / GL, NF = N1 * N1, Np = NF * N1, PE = (NF + 1) / 2;  // pairs per element
+           const __grid_constant__ S64Args args, int ncol, double* gsc) {
+  constexpr int N = N1 - 1, G = 32 / GL, NF = N1 * N1, Np = NF * N1;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const int slot = blockIdx.x * wpb + wib, nslot = gridDim.x * wpb;
   const int grp = lane / GL, kl = lane % GL;
-  const int NeZ = op.NeZ, L = op.L, ncp = op.NeX * op.NeY * PE;
+  const int NeZ = op.NeZ, L = op.L, ncp = (ncol + 1) / 2;
   const S64Layout lay(N1, GL, NeZ);
   unsigned char* base = smraw + (size_t)(wib * G + grp) * lay.stride;
   Ctx64<N1, GL> c;
@@ -219,10 +219,10 @@ __global__ void __launch_bounds__(64, 6)
   const int gv[3] = {VD, VMZ, VRT};
 
   for (int p0 = slot * G; p0 < ncp; p0 += nslot * G) {
-    const int cp = min(p0 + grp, ncp - 1), exy = cp / PE, ij = 2 * (cp - exy * PE), colA = exy * NF + ij, colB = ij + 1 < NF ? colA + 1 : colA;
+    const int cp = min(p0 + grp, ncp - 1), colA = 2 * cp, colB = min(colA + 1, ncol - 1);
     bool liveA = p0 + grp < ncp && c.act, liveB = liveA && colB != colA;
-    c.gA = (size_t)exy * Np + ij;
-    c.gB = c.gA + (colB - colA);
+    c.gA = (size_t)(colA / NF) * Np + colA % NF;
+    c.gB = (size_t)(colB / NF) * Np + colB % NF;
     c.gs = (size_t)op.NeX * op.NeY * Np;
     auto store = [&](int v, int e, double2 x) {
       const size_t o = (size_t)e * c.gs + (size_t)NF * k;
@@ -299,13 +299,13 @@ __global__ void __launch_bounds__(64, 6)
         for (int v = 0; v < 3; ++v) store(gv[v], e, neg2(s[v]));
       });
     } else {
-      // ---- DENS/MOMZ/RHOT Newton; the flags are the pair's, uniform over its lanes ----
+      // ---- DENS/MOMZ/RHOT Newton.  Sets of columns: bit 0 is A, bit 1 is B, uniform over the pair's lanes ----
       const SweepCoef<N1> sc(op, impl, c.A[0]);
-      bool run = p0 + grp < ncp, give_up = false;  // run: still iterating
-      bool doneA = !run, doneB = doneA || colB == colA;
+      int run = (p0 + grp < ncp ? 1 : 0) | (p0 + grp < ncp && colB != colA ? 2 : 0), give_up = 0;  // run: still iterating
       int nsolve = 0;
       while (true) {
-        float errA = 0.f, errB = 0.f, bmax = 0.f;
+        float errA = 0.f, errB = 0.f;
+        unsigned bm[2] = {0u, 0u};
         pass64<N1, GL>(args, c, fill, [&](int e, const double2 (&own)[3], const double2 (&s)[3]) {
           const int l = e * N1 + k;
           const float dh = (float)__ldg(pf.dens + l), rh = (float)__ldg(pf.rhyd + l);
@@ -320,11 +320,14 @@ __global__ void __launch_bounds__(64, 6)
             const float2 f = unpk(bf);
             errA = fmaxf(errA, fabsf(f.x) * isc[v]);
             errB = fmaxf(errB, fabsf(f.y) * isc[v]);
-            bmax = max_bits(bmax, max_bits(wt[v] * f.x, wt[v] * f.y));
+            max_bits(bm[0], wt[v], f.x);
+            max_bits(bm[1], wt[v], f.y);
           }
         });
-        bmax = pair_max_bits<GL>(bmax);
-        bool bad = !(bmax < 3.0e38f);
+        const float2 bmax = make_float2(pair_max_bits<GL>(bm[0]), pair_max_bits<GL>(bm[1]));
+        const int bad = run & ((bmax.x < 3.0e38f ? 0 : 1) | (bmax.y < 3.0e38f ? 0 : 2));
+        give_up |= bad;
+        run &= ~bad;
         if (args.v.max_iter > 1) {
 #pragma unroll
           for (int o = GL / 2; o > 0; o >>= 1) {
@@ -335,30 +338,28 @@ __global__ void __launch_bounds__(64, 6)
           // outside 1e-5 of tol; the rest takes the FP64 residual that the pass left
           auto above = [&](float x) { return x > 1.0e-30f && x > args.tol_hi; };
           auto sure = [&](float x) { return above(x) || (args.tol_lo > 1.0e-30f && x < args.tol_lo); };
-          bool convA = !above(errA), convB = !above(errB);
-          if (__any_sync(FULL, run && !bad && !((doneA || sure(errA)) && (doneB || sure(errB))))) {
+          int conv = (above(errA) ? 0 : 1) | (above(errB) ? 0 : 2);
+          if (__any_sync(FULL, run & ((sure(errA) ? 0 : 1) | (sure(errB) ? 0 : 2)))) {
             const double2 x = scaled_max<GL>(pf, args.v.cref, c.W + (size_t)3 * W_B * NeZ * 32 + lane, k, N1, NeZ);
-            convA = x.x <= args.v.tol;
-            convB = x.y <= args.v.tol;
+            conv = (x.x <= args.v.tol ? 1 : 0) | (x.y <= args.v.tol ? 2 : 0);
           }
-          if (run && !bad) {
-            if (!doneA && convA) { stA = nsolve; doneA = true; }
-            if (!doneB && convB) { stB = nsolve; doneB = true; }
-            bad = !(doneA && doneB) && nsolve >= args.v.max_iter;
+          conv &= run;
+          if (conv & 1) stA = nsolve;
+          if (conv & 2) stB = nsolve;
+          run &= ~conv;
+          if (nsolve >= args.v.max_iter) {
+            give_up |= run;
+            run = 0;
           }
-        }
-        if (run) {
-          give_up = bad;
-          run = !bad && !(doneA && doneB);
         }
         if (!__any_sync(FULL, run)) break;
         // ---- J delta = b by refinement: rho is the residual's size over b's.  Solved once what the last sweeps
         // left, or the residual itself, is below FP64's roundoff; anything else is left to block LU ----
-        float rho = 1.f, rmax = bmax;
-        bool open = run, solved = false;  // open: still refining
+        float2 rho = make_float2(1.f, 1.f), rmax = bmax;
+        int open = run, solved = 0;  // open: still refining
         for (int it = 0; it < 6; ++it) {
           // the sweeps leave rel of their right-hand side; the last ones need not go below FP64's roundoff
-          const float rel = fminf(1.0e-3f, fmaxf(1.0e-6f, 1.0e-17f / rho));
+          const float2 rel = make_float2(fminf(1.0e-3f, fmaxf(1.0e-6f, 1.0e-17f / rho.x)), fminf(1.0e-3f, fmaxf(1.0e-6f, 1.0e-17f / rho.y)));
           open = sweeps<N1, GL>(c, sc, op, impl, rmax, rel, args.c1, args.c2, open);
           if (open) {
             for (int e = 0; e < NeZ; ++e) {
@@ -366,16 +367,16 @@ __global__ void __launch_bounds__(64, 6)
               for (int v = 0; v < 3; ++v) {
                 const float2 x = unpk(c.X[v * L + e * N1 + k]);
                 double2& d = c.w(W_D, v, e);
-                d = it == 0 ? make_double2(x.x, x.y) : make_double2(d.x + x.x, d.y + x.y);
+                d = it == 0 ? make_double2(x.x, x.y) : make_double2(open & 1 ? d.x + x.x : d.x, open & 2 ? d.y + x.y : d.y);
               }
             }
-            if (rho <= 1.0e-11f) {  // what these sweeps left is below 1e-17 of b
-              solved = true;
-              open = false;
-            }
+            // what these sweeps left is below 1e-17 of b
+            const int last = open & ((rho.x <= 1.0e-11f ? 1 : 0) | (rho.y <= 1.0e-11f ? 2 : 0));
+            solved |= last;
+            open &= ~last;
           }
           if (!__any_sync(FULL, open)) break;
-          float rm = 0.f;
+          unsigned rm[2] = {0u, 0u};
           pass64<N1, GL>(
               args, c,
               [&](int e, double2 (&q)[5]) {  // linearised level quantities of delta
@@ -395,29 +396,27 @@ __global__ void __launch_bounds__(64, 6)
                   const u64x r = to_f((c.w(W_B, v, e) - own[v]) - s[v]);
                   if (c.act) c.B[v * L + l] = r;
                   const float2 f = unpk(r);
-                  rm = max_bits(rm, max_bits(wt[v] * f.x, wt[v] * f.y));
+                  max_bits(rm[0], wt[v], f.x);
+                  max_bits(rm[1], wt[v], f.y);
                 }
               });
-          rmax = pair_max_bits<GL>(rm);
-          rho = bmax > 0.f ? rmax / bmax : rmax;
-          if (open) {  // NaN: neither
-            solved = rho < 1.0e-16f;
-            open = rho < 0.1f && !solved;
-          }
+          rmax = make_float2(pair_max_bits<GL>(rm[0]), pair_max_bits<GL>(rm[1]));
+          rho = make_float2(bmax.x > 0.f ? rmax.x / bmax.x : rmax.x, bmax.y > 0.f ? rmax.y / bmax.y : rmax.y);
+          // NaN: neither solved nor open
+          solved |= open & ((rho.x < 1.0e-16f ? 1 : 0) | (rho.y < 1.0e-16f ? 2 : 0));
+          open &= ((rho.x < 0.1f ? 1 : 0) | (rho.y < 0.1f ? 2 : 0)) & ~solved;
           if (!__any_sync(FULL, open)) break;
         }
-        if (run) {
-          run = solved;
-          give_up = !solved;
-          ++nsolve;
-        }
+        give_up |= run & ~solved;
+        run &= solved;
+        ++nsolve;
         if (run) {
           for (int e = 0; e < NeZ; ++e) {
 #pragma unroll
             for (int v = 0; v < 3; ++v) {
               const double2 d = c.w(W_D, v, e);
               double2& P = c.w(W_P, v, e);
-              P = make_double2(doneA ? P.x : P.x + d.x, doneB ? P.y : P.y + d.y);
+              P = make_double2(run & 1 ? P.x + d.x : P.x, run & 2 ? P.y + d.y : P.y);
             }
           }
         }
@@ -427,13 +426,17 @@ __global__ void __launch_bounds__(64, 6)
           break;
         }
       }
-      if (give_up) {  // block LU for these columns, by the kernel that follows
-        if (k == 0 && liveA) status[colA] = VI_REDO;
-        if (k == 0 && liveB) status[colB] = VI_REDO;
-        liveA = liveB = false;
+      // block LU for these columns, by the kernel that follows
+      if ((give_up & 1) && liveA) {
+        if (k == 0) status[colA] = VI_REDO;
+        liveA = false;
+      }
+      if ((give_up & 2) && liveB) {
+        if (k == 0) status[colB] = VI_REDO;
+        liveB = false;
       }
       __syncwarp();
-      if (!__any_sync(FULL, liveA)) continue;
+      if (!__any_sync(FULL, liveA || liveB)) continue;
       for (int e = 0; e < NeZ; ++e) {
 #pragma unroll
         for (int v = 0; v < 3; ++v)
@@ -527,7 +530,7 @@ int plan_n(const Ops& op, Plan64& p) {
   }
   if (p.wpb == 0) return 0;  // the columns are too tall: block LU alone
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kfn, 32 * p.wpb, p.smem)) != cudaSuccess) return (int)e;
-  const int ncp = op.NeX * op.NeY * ((N1 * N1 + 1) / 2), per = G * p.wpb;
+  const int ncp = (op.NeX * op.NeY * N1 * N1 + 1) / 2, per = G * p.wpb;
   p.grid = std::max(1, std::min((ncp + per - 1) / per, nb * nsm));
   p.scratch = (size_t)p.grid * p.wpb * s64_slice(op.NeZ);
   return 0;
@@ -536,7 +539,7 @@ int plan_n(const Ops& op, Plan64& p) {
 template <int N1>
 int launch_n(const Plan64& p, const Ops& op, const Prof& pf, const F5c& qin, const F5c& z, const F5& tout, int* status,
              const S64Args& a, double* gsc, cudaStream_t s) {
-  k_vi64<N1, gl_of<N1>()><<<p.grid, 32 * p.wpb, p.smem, s>>>(op, pf, qin, z, tout, status, a, gsc);
+  k_vi64<N1, gl_of<N1>()><<<p.grid, 32 * p.wpb, p.smem, s>>>(op, pf, qin, z, tout, status, a, op.NeX * op.NeY * N1 * N1, gsc);
   return (int)cudaGetLastError();
 }
 
